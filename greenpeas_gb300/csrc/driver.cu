@@ -573,6 +573,7 @@ struct gpc_driver {
     tg_cap = 0;
     prepared = false;
     ran = false;
+    sizes.known = false;
     last_run_sig = 0;
   }
   // noise-rate gradients: record probabilities come from a device noise tensor
@@ -751,8 +752,9 @@ struct gpc_driver {
     L.slot = take(slots * sizeof(gpc::Slot));
     L.bagg = take((size_t)nb * 8);
     L.bout = take((size_t)nb * 8);
-    L.cout = take((size_t)N * 8);
     L.big_list = take((size_t)nb * 4);
+    // each circuit's first output slot, the flags and the totals side by side: one copy reads a run's result sizes
+    L.cout = take((size_t)N * 8);
     L.zero = o;
     L.err = take(4);
     L.totals = take(16);
@@ -1066,6 +1068,7 @@ struct gpc_driver {
     }
     prepared = false;
     ran = false;
+    sizes.known = false;
     if (texts) {
       if (n == 0) throw gpc::Error(GPC_ERR_INVALID, "empty batch");
       tcap = 32;
@@ -1159,6 +1162,7 @@ struct gpc_driver {
     if (!prepared) throw gpc::Error(GPC_ERR_INVALID, "no circuit prepared");
     CK(cudaSetDevice(device));
     used_global = false;
+    sizes.known = false;
     const bool single_global = ncirc() == 1 && (force_global || lists_off);
     // (a graph with the stage events is another graph)
     const uint64_t sig = cfg_sig ^ (stage_timing ? 0x9e3779b97f4a7c15ull : 0ull);
@@ -1620,16 +1624,29 @@ struct gpc_driver {
   // full 128-bit re-sorts, [4] target-buffer regrowths.
   std::atomic<uint64_t> fallbacks[5] = {};
 
+  // Result sizes of the last run, read once it has finished: device_dem answers every circuit of a
+  // batch from them without going back to the device (256 circuits: 55 us each before).  Forgotten by
+  // the next prepare or run.
+  struct RunSizes {
+    bool known = false;
+    uint32_t C = 0, NT = 0;
+    std::vector<uint2> first;  // each circuit's first output slot and target (written for batches)
+  } sizes;
+
   // Reads flags and totals; handles the rare fallbacks (bucket overflow,
   // long symptoms, short sort keys, target-buffer growth).
   Finish finish(uint32_t *groups, uint32_t *targets) {
-    pin_out.ensure(64);
-    uint32_t *h = static_cast<uint32_t *>(pin_out.p);
     bool did_full = false;
     for (int attempt = 0; attempt < 8; ++attempt) {
-      CK(cudaMemcpyAsync(h, dptr<char>(L.err), 4, cudaMemcpyDeviceToHost, stream));
-      CK(cudaMemcpyAsync(h + 1, dptr<char>(L.totals), 8, cudaMemcpyDeviceToHost, stream));
+      // one copy of [cout, flags, totals], which lie side by side (a rerun may have moved them)
+      const size_t bytes = L.totals + 8 - L.cout;
+      pin_out.ensure(bytes);
+      const char *hc = static_cast<const char *>(pin_out.p);
+      CK(cudaMemcpyAsync(pin_out.p, dptr<char>(L.cout), bytes, cudaMemcpyDeviceToHost, stream));
       wait();
+      uint32_t h[3];
+      memcpy(h, hc + (L.err - L.cout), 4);
+      memcpy(h + 1, hc + (L.totals - L.cout), 8);
       const uint32_t err = h[0];
       if (err & gpc::DEV_ERR_TIMEOUT) throw gpc::Error(GPC_ERR_TIMEOUT, "a bounded device wait timed out");
       if (err & gpc::DEV_ERR_COLLISION)
@@ -1689,6 +1706,11 @@ struct gpc_driver {
       if (h[1] > L.M || h[2] > tg_cap) throw gpc::Error(GPC_ERR_CUDA, "inconsistent merge totals");
       *groups = h[1];
       *targets = h[2];
+      sizes.C = h[1];
+      sizes.NT = h[2];
+      sizes.first.resize(ncirc());
+      memcpy(sizes.first.data(), hc, (size_t)ncirc() * 8);
+      sizes.known = true;
       return Finish::Ok;
     }
     throw gpc::Error(GPC_ERR_CUDA, "merge did not converge");
@@ -1701,22 +1723,14 @@ struct gpc_driver {
     if (i >= ncirc()) throw gpc::Error(GPC_ERR_INVALID, "circuit index out of range");
     CK(cudaSetDevice(device));
     uint32_t C = 0, NT = 0;
-    if (finish(&C, &NT) != Finish::Ok)
+    if (!sizes.known && finish(&C, &NT) != Finish::Ok)
       throw gpc::Error(GPC_ERR_UNSUPPORTED, "this batch was compiled circuit by circuit: no device arrays");
-    uint2 first = make_uint2(0, 0), next = make_uint2(C, NT);
-    pin_out.ensure(64);
-    uint32_t *h = static_cast<uint32_t *>(pin_out.p);
-    if (ncirc() > 1) {
-      CK(cudaMemcpyAsync(h, dptr<char>(L.cout) + (size_t)i * 8, i + 1 < ncirc() ? 16 : 8, cudaMemcpyDeviceToHost,
-                         stream));
+    const uint2 first = ncirc() > 1 ? sizes.first[i] : make_uint2(0, 0);
+    const uint2 next = i + 1 < ncirc() ? sizes.first[i + 1] : make_uint2(sizes.C, sizes.NT);
+    if (L.M == 0) {  // nothing was merged: the closing offset of the run was not written by a kernel
+      CK(cudaMemsetAsync(dptr<char>(L.out_off), 0, 4, stream));
       wait();
-      first = make_uint2(h[0], h[1]);
-      if (i + 1 < ncirc()) next = make_uint2(h[2], h[3]);
     }
-    // the closing offset of the whole run (offsets are positions in the run's target array)
-    h[8] = NT;
-    CK(cudaMemcpyAsync(dptr<char>(L.out_off) + (size_t)C * 4, h + 8, 4, cudaMemcpyHostToDevice, stream));
-    wait();
     *probs = dptr<double>(L.out_prob) + first.x;
     *offsets = dptr<uint32_t>(L.out_off) + first.x;
     *targets = static_cast<const uint32_t *>(tgbuf.p);

@@ -646,6 +646,7 @@ __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(MergeLaunch L) {
     if (tile == ntiles - 1) {
       L.totals[0] = pc + ac;
       L.totals[1] = pt + at;
+      if (pc + ac <= n) L.out_off[pc + ac] = pt + at;  // the closing offset (past n only after a timed-out look-back)
       if (pt + at > L.tg_cap) atomicOr(L.err, DEV_FLAG_TG_OVF);
     }
   }
@@ -1290,6 +1291,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) group_scan_kernel(GroupLaunch L)
   if (tile == gridDim.x - 1 && t == SCAN_THREADS - 1) {
     L.totals[0] = run.x;
     L.totals[1] = run.y;
+    L.out_off[run.x] = run.y;  // the closing offset
     if (run.y > L.tg_cap) atomicOr(L.err, DEV_FLAG_TG_OVF);
   }
 }

@@ -127,6 +127,16 @@ class _View:
         self.owner = owner
 
 
+class _DeviceView:
+    """CUDA-array-interface exporter of n elements at a device address."""
+
+    __slots__ = ("__cuda_array_interface__",)
+
+    def __init__(self, addr: int, n: int, typestr: str):
+        self.__cuda_array_interface__ = {"shape": (n,), "typestr": typestr, "data": (addr or 0, False), "version": 3,
+                                         "strides": None}
+
+
 def _owned(ptr, n: int, dtype, owner) -> np.ndarray:
     """Read-only numpy view of n elements at ptr whose base keeps ``owner`` (the gpc_dem) alive."""
     if n == 0:
@@ -149,6 +159,7 @@ class Driver:
         is lowered whole on all host threads."""
         L = _native.lib()
         self._h = ctypes.c_void_p()
+        self._views = None
         self.correlation_level = CorrelationLevel(correlation_level)
         self.device = device
         opts = _native.Options()
@@ -269,23 +280,41 @@ class Driver:
         write them): probs[E] float64, offsets[E + 1] int32 positions in
         targets (the run's whole target array, so offsets need not start at
         0)."""
-        import torch
         L = _native.lib()
         pp, po, pt = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p()
         n, end = ctypes.c_uint32(), ctypes.c_uint32()
         _native.check(L.gpc_device_dem(self._h, int(circuit), ctypes.byref(pp), ctypes.byref(po), ctypes.byref(pt),
                                        ctypes.byref(n), ctypes.byref(end)))
+        n, end = n.value, end.value
+        views = self._device_views(int(circuit), pp.value, po.value, pt.value, n, end)
+        return tuple(t[(addr - base) // size:(addr - base) // size + count] for (base, size, t), addr, count in
+                     zip(views, (pp.value, po.value, pt.value), (n, n + 1, end)))
 
-        class _View:
-            def __init__(self, ptr, count, typestr):
-                self.__cuda_array_interface__ = {"shape": (count,), "typestr": typestr,
-                                                 "data": (ptr or 0, False), "version": 3, "strides": None}
+    def _device_views(self, circuit, pp, po, pt, n, end):
+        """(address, item size, tensor) over the run's whole probability, offset and target buffers.
+
+        Wrapping a device address costs ~10 us in torch and a slice ~1 us, so the buffers are wrapped
+        once and a batch's circuits slice them; they are wrapped again when the wanted range is not inside
+        (the driver's buffers moved or grew)."""
+        want = ((pp, n * 8), (po, (n + 1) * 4), (pt, end * 4))
+        views = self._views
+        if views is not None and all(base <= a and a + b <= base + t.numel() * size
+                                     for (base, size, t), (a, b) in zip(views, want)):
+            return views
+        import torch
+        if circuit:  # the run's arrays start at its first circuit's
+            p0, o0, t0 = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p()
+            c = ctypes.c_uint32()
+            _native.check(_native.lib().gpc_device_dem(self._h, 0, ctypes.byref(p0), ctypes.byref(o0), ctypes.byref(t0),
+                                                       ctypes.byref(c), ctypes.byref(c)))
+            pp, po, pt = p0.value, o0.value, t0.value
+        raw = self.last_sizes()["raw"]  # capacity of the outputs; the target buffer holds 16 per mechanism at least
 
         dev = torch.device("cuda", self.device)
-        probs = torch.as_tensor(_View(pp.value, n.value, "<f8"), device=dev)
-        offsets = torch.as_tensor(_View(po.value, n.value + 1, "<i4"), device=dev)
-        targets = torch.as_tensor(_View(pt.value, end.value, "<i4"), device=dev)
-        return probs, offsets, targets
+        self._views = tuple((a, size, torch.as_tensor(_DeviceView(a, count, typestr), device=dev)) for a, count, size, typestr in
+                            ((pp, raw, 8, "<f8"), (po, raw + 1, 4, "<i4"),
+                             (pt, max(end, min(16 * raw, 0xFFFFFFF0)), 4, "<i4")))
+        return self._views
 
     # device-resident stages
     def prepare(self, circuit=None) -> None:
