@@ -325,7 +325,7 @@ cudaError_t launch_adjoint(const AdjointLaunch &L, cudaStream_t s);
 cudaError_t launch_scan_emit(const GroupLaunch &L, cudaStream_t s);
 
 // ---- global path (used when a bucket is too large for one CTA) -------------
-// Onesweep radix sort of (u64 key, u32 value) pairs on the low `bits` bits.
+// Onesweep radix sort of (u64 key, u32 value) pairs on the `bits` bits from bit `shift0` on.
 struct SortScratch {
   uint32_t *hist;      // [passes][RADIX]
   uint32_t *status;    // [passes][tiles][RADIX]
@@ -337,11 +337,11 @@ struct SortScratch {
   uint32_t hold_first;
 };
 size_t sort_scratch_words(uint32_t n, uint32_t bits);
-cudaError_t launch_sort(uint64_t *keys, uint64_t *keys_alt, uint32_t *vals, uint32_t *vals_alt, uint32_t n,
-                        uint32_t bits, const SortScratch &scr, cudaStream_t s, bool *result_in_alt);
-
-// sortkey[m] = key[m].x, perm[m] = m (inputs of the global sort).
-cudaError_t launch_sort_init(const ulonglong2 *key, uint64_t *sortkey, uint32_t *perm, uint32_t M, cudaStream_t s);
+// The first pass reads its keys from `first`, every `stride`-th u64, and its values from `vals` or (index_vals)
+// takes the keys' indices; the passes then alternate between (keys_alt, vals_alt) and (keys, vals).
+cudaError_t launch_sort(const uint64_t *first, uint32_t stride, bool index_vals, uint64_t *keys, uint64_t *keys_alt,
+                        uint32_t *vals, uint32_t *vals_alt, uint32_t n, uint32_t shift0, uint32_t bits,
+                        const SortScratch &scr, cudaStream_t s, bool *result_in_alt);
 
 // Gathers key128[perm[i]].y into out[i] (second pass of a 128-bit sort).
 cudaError_t launch_gather_hi(const ulonglong2 *key, const uint32_t *perm, uint64_t *out, uint32_t n, cudaStream_t s);

@@ -476,6 +476,7 @@ struct gpc_driver {
   int device = 0;
   int level = 2;
   uint32_t sort_bits = 64;
+  bool sort_auto = true;  // no sort_bits given: the global path sorts on as many top key bits as its size needs
   cudaStream_t stream = nullptr;
   static constexpr int kAux = 4;
   cudaStream_t aux[kAux] = {};
@@ -586,6 +587,10 @@ struct gpc_driver {
   bool use_graph = true;
   uint64_t cfg_sig = 0, graph_sig = 0, last_run_sig = 0;
   uint32_t tcap = 32;      // target-list stride (grows when a symptom is longer)
+  // A symptom of the prepared circuit overflowed its bucket: its later runs go to the global sort at
+  // once (the bucket pass, its wait and the second key pass cost 60 us of 250 on 118k mechanisms).
+  // Set by a run, forgotten with the circuit.
+  bool overflowed = false;
   bool lists_off = false;  // symptoms too long for target lists: merge from snapshots
   uint64_t last_d2h = 0;   // bytes copied device -> host by the last fetch
   uint64_t last_h2d = 0;   // bytes copied host -> device by the last prepare (a chunked batch: all of its chunks)
@@ -1053,7 +1058,7 @@ struct gpc_driver {
     if (T.empty()) throw gpc::Error(GPC_ERR_INVALID, "empty batch");
     param = false;
     tcap = 32;
-    lists_off = false;
+    lists_off = overflowed = false;
     if (ops_in_flight) wait();
     tapes.swap(T);
     have_tape = true;
@@ -1072,7 +1077,7 @@ struct gpc_driver {
     if (texts) {
       if (n == 0) throw gpc::Error(GPC_ERR_INVALID, "empty batch");
       tcap = 32;
-      lists_off = false;
+      lists_off = overflowed = false;
       const auto t0 = HostClock::now();
       lower_all(texts, lens, n);
       host_ms[0] = ms_since(t0);
@@ -1130,6 +1135,7 @@ struct gpc_driver {
     mix(tcap);
     mix((uint64_t)force_global);
     mix((uint64_t)lists_off);
+    mix((uint64_t)overflowed);
     mix(L.in_bytes);
     mix(L.zero_bytes);
     for (const auto &c : L.classes) {
@@ -1163,7 +1169,8 @@ struct gpc_driver {
     CK(cudaSetDevice(device));
     used_global = false;
     sizes.known = false;
-    const bool single_global = ncirc() == 1 && (force_global || lists_off);
+    const bool single_global = ncirc() == 1 && (force_global || lists_off || overflowed);
+    if (ncirc() == 1 && overflowed && !force_global && !lists_off) ++fallbacks[1];
     // (a graph with the stage events is another graph)
     const uint64_t sig = cfg_sig ^ (stage_timing ? 0x9e3779b97f4a7c15ull : 0ull);
     const bool graphable = use_graph && !single_global && ((graph_exec && graph_sig == sig) || last_run_sig == sig);
@@ -1430,7 +1437,7 @@ struct gpc_driver {
   // observables never vanish, so their walk covers every epoch, while the
   // detector words stop early; their keys are computed beside that walk.
   uint32_t split_word() const {
-    if (!key_split || seg_on || ncirc() != 1 || force_global || lists_off || tcap == 0 || L.classes.size() != 1)
+    if (!key_split || seg_on || ncirc() != 1 || force_global || lists_off || overflowed || tcap == 0 || L.classes.size() != 1)
       return gpc::kNoSplit;
     const Tape &T = tapes[0];
     if (T.nobs == 0 || T.n_epochs == 0) return gpc::kNoSplit;
@@ -1487,7 +1494,7 @@ struct gpc_driver {
     CK(cudaMemsetAsync(dptr<char>(L.zero), 0, L.zero_bytes, stream));
     for (uint32_t i = 0; i < ncirc(); ++i)
       if (tapes[i].n_epochs == 0) CK(cudaMemsetAsync(dptr<char>(L.c[i].band), 0, (size_t)tapes[i].w * 8, stream));
-    gpc::KeyLaunch kl = key_launch(param || (ncirc() == 1 && (force_global || lists_off)));
+    gpc::KeyLaunch kl = key_launch(param || (ncirc() == 1 && (force_global || lists_off || overflowed)));
     const uint32_t late = split_word();
     rec(0);
     if (seg_on) {
@@ -1506,8 +1513,8 @@ struct gpc_driver {
       CK(gpc::launch_keys_late(kl, stream));
     }
     rec(2);
-    if (ncirc() == 1 && (force_global || lists_off)) {
-      run_global(false);
+    if (ncirc() == 1 && (force_global || lists_off || overflowed)) {
+      run_global(SortKey::Auto);
     } else {
       CK(gpc::launch_group(group_launch(), stream));
       rec(3);
@@ -1543,15 +1550,29 @@ struct gpc_driver {
 
   // Global path (single circuit): sort every mechanism (on sort_bits, or all
   // 128 bits) and merge from the snapshots.
-  void run_global(bool full) {
+  enum class SortKey { Auto, Half, Full };  // sort_bits (or as many as the size needs) / 64 bits / 128 bits
+  void run_global(SortKey full) {
     used_global = true;
     CK(cudaMemsetAsync(dptr<char>(L.gzero), 0, L.gzero_bytes, stream));
     CK(cudaMemsetAsync(dptr<char>(L.totals), 0, 8, stream));
-    CK(gpc::launch_sort_init(dptr<ulonglong2>(L.key), dptr<uint64_t>(L.sk0), dptr<uint32_t>(L.pm0), L.M, stream));
     sort_and_merge(full);
   }
 
-  void sort_and_merge(bool full) {
+  // Key bits a sort of M mechanisms compares: from the top bit down, as many whole digits as keep the
+  // chance that two different keys agree on them under ~2^-10 (M^2 / 2 pairs), so that the order is the
+  // 64-bit order at 6 passes instead of 8 for ~100k mechanisms.  The merge reports such a pair
+  // (DEV_FLAG_MIXED) and the sort is done again on 64 bits.
+  static uint32_t auto_sort_bits(uint32_t M) {
+    uint32_t lg = 0;
+    while (lg < 32 && (1ull << lg) < M) ++lg;
+    const uint32_t bits = (2 * lg + 9 + gpc::RADIX_BITS - 1) / gpc::RADIX_BITS * gpc::RADIX_BITS;
+    return std::min(64u, bits);
+  }
+  SortKey sorted_on = SortKey::Auto;  // of the last global run
+  uint32_t sorted_bits = 64;
+
+  void sort_and_merge(SortKey key) {
+    const bool full = key == SortKey::Full;
     const uint32_t M = L.M;
     uint32_t *sw = dptr<uint32_t>(L.sort_scr);
     const uint32_t passes = 8;
@@ -1566,7 +1587,11 @@ struct gpc_driver {
     uint64_t *k0 = dptr<uint64_t>(L.sk0), *k1 = dptr<uint64_t>(L.sk1);
     uint32_t *p0 = dptr<uint32_t>(L.pm0), *p1 = dptr<uint32_t>(L.pm1);
     bool alt = false;
-    CK(gpc::launch_sort(k0, k1, p0, p1, M, full ? 64 : sort_bits, s1, stream, &alt));
+    const uint32_t bits = key != SortKey::Auto ? 64u : sort_auto ? auto_sort_bits(M) : sort_bits;
+    const uint32_t shift0 = key == SortKey::Auto && sort_auto ? 64u - bits : 0u;
+    sorted_on = key;
+    sorted_bits = bits;
+    CK(gpc::launch_sort(dptr<uint64_t>(L.key), 2, true, k0, k1, p0, p1, M, shift0, bits, s1, stream, &alt));
     uint64_t *ks = alt ? k1 : k0;
     uint32_t *ps = alt ? p1 : p0;
     if (full) {
@@ -1576,14 +1601,13 @@ struct gpc_driver {
       uint32_t *ps_alt = alt ? p0 : p1;
       CK(gpc::launch_gather_hi(dptr<ulonglong2>(L.key), ps, hk, M, stream));
       bool alt2 = false;
-      CK(gpc::launch_sort(hk, hk_alt, ps, ps_alt, M, 64, s2, stream, &alt2));
+      CK(gpc::launch_sort(hk, 1, false, hk, hk_alt, ps, ps_alt, M, 0, 64, s2, stream, &alt2));
       ks = alt2 ? hk_alt : hk;
       ps = alt2 ? ps_alt : ps;
     }
     perm_sorted = ps;
     sk_sorted = ks;
-    const uint32_t b = full ? 0 : sort_bits;
-    sort_mask = b == 0 ? 0ull : (b >= 64 ? ~0ull : ((1ull << b) - 1));
+    sort_mask = full ? 0ull : (bits >= 64 ? ~0ull : ((1ull << bits) - 1) << shift0);
     rec(3);
     launch_merge_now();
     rec(4);
@@ -1672,19 +1696,25 @@ struct gpc_driver {
       }
       if ((err & gpc::DEV_FLAG_BIG_BUCKET) && !used_global) {
         ++fallbacks[1];
+        overflowed = true;
         // a symptom repeated more often than a bucket holds: sort globally
         // (the bucket pass skipped the keys and descriptors this path reads)
         CK(cudaMemsetAsync(dptr<char>(L.err), 0, 4, stream));
         CK(gpc::launch_keys(key_launch(true), stream));
         CK(cudaMemsetAsync(dptr<char>(L.err), 0, 4, stream));
-        run_global(false);
+        run_global(SortKey::Auto);
+        continue;
+      }
+      if (used_global && (err & gpc::DEV_FLAG_MIXED) && sorted_on == SortKey::Auto && sort_auto && sorted_bits < 64) {
+        CK(cudaMemsetAsync(dptr<char>(L.err), 0, 4, stream));
+        run_global(SortKey::Half);
         continue;
       }
       if (used_global && (err & gpc::DEV_FLAG_MIXED) && !did_full) {
         ++fallbacks[3];
         // equal sort keys with different full keys: sort on all 128 bits
         CK(cudaMemsetAsync(dptr<char>(L.err), 0, 4, stream));
-        run_global(true);
+        run_global(SortKey::Full);
         did_full = true;
         continue;
       }
@@ -1887,7 +1917,7 @@ struct gpc_driver {
     const double per_list = M > 0 ? lists / M : 0.0;
     out[0] = walk;
     // records, snapshot words read, count (+ key, descriptor, probability when kept), lists, bucket slots
-    const bool all = param || (ncirc() == 1 && (force_global || lists_off));
+    const bool all = param || (ncirc() == 1 && (force_global || lists_off || overflowed));
     out[1] = R * 20 + 16.0 * pts + M * (all ? 36 : 4) + 4.0 * lists + (double)nonempty * 32;
     // slots read, lists compared for the non-head items, group records written, counts and aggregates
     out[2] = (double)nonempty * 32 + (double)(nonempty - std::min<double>(nonempty, groups)) * 8.0 * per_list +
@@ -2098,7 +2128,7 @@ struct gpc_driver {
         tapes.clear();
         tapes.push_back(std::move(T[i]));
         tcap = 32;
-        lists_off = false;
+        lists_off = overflowed = false;
         prepare(nullptr, nullptr, 0);
         run();
         std::vector<gpc_dem *> one;
@@ -2203,6 +2233,7 @@ struct gpc_driver {
       d->device = device;
       d->level = level;
       d->sort_bits = sort_bits;
+      d->sort_auto = sort_auto;
       d->force_global = force_global;
       d->walk_qpt = walk_qpt;
       d->bucket_mean = bucket_mean;
@@ -2583,7 +2614,10 @@ gpc_status gpc_get_driver(const char *stim_text, size_t len, int32_t correlation
   if (options) {
     d->device = options->device;
     if (options->sort_bits < 0 || options->sort_bits > 64) return fail(GPC_ERR_INVALID, "sort_bits must be in 0..64");
-    if (options->sort_bits) d->sort_bits = (uint32_t)options->sort_bits;
+    if (options->sort_bits) {
+      d->sort_bits = (uint32_t)options->sort_bits;
+      d->sort_auto = false;
+    }
     d->force_global = options->global_sort != 0;
     if (options->walk_qpt < 0 || (options->walk_qpt && !gpc::walk_max_threads((uint32_t)options->walk_qpt)))
       return fail(GPC_ERR_INVALID, "walk_qpt must be 0, 1, 2, 3, 4, 6, 8, 12 or 16");

@@ -354,23 +354,16 @@ __global__ void bucket_scatter_kernel(const ulonglong2 *__restrict__ key, uint32
   }
 }
 
-__global__ void sort_init_kernel(const ulonglong2 *__restrict__ key, uint64_t *__restrict__ sortkey,
-                                 uint32_t *__restrict__ perm, uint32_t M) {
-  for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
-    sortkey[m] = key[m].x;
-    perm[m] = m;
-  }
-}
-
 // ---- onesweep radix sort ----------------------------------------------------
 
-__global__ void sort_hist_kernel(const uint64_t *__restrict__ keys, uint32_t n, uint32_t passes,
-                                 uint32_t *__restrict__ hist) {
+// Key i of a sort: every `stride`-th u64 (2: the first halves of 128-bit keys).
+__global__ void sort_hist_kernel(const uint64_t *__restrict__ keys, uint32_t stride, uint32_t n, uint32_t shift0,
+                                 uint32_t passes, uint32_t *__restrict__ hist) {
   __shared__ uint32_t h[8][RADIX];
   for (uint32_t i = threadIdx.x; i < 8 * RADIX; i += blockDim.x) (&h[0][0])[i] = 0;
   __syncthreads();
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint64_t k = keys[i];
+    const uint64_t k = keys[(size_t)i * stride] >> shift0;
     for (uint32_t p = 0; p < passes; ++p) atomicAdd(&h[p][(k >> (p * RADIX_BITS)) & (RADIX - 1)], 1u);
   }
   __syncthreads();
@@ -400,8 +393,15 @@ constexpr uint32_t ST_AGG = 1u << 30;     // tile aggregate published
 constexpr uint32_t ST_PREFIX = 2u << 30;  // inclusive prefix published
 constexpr uint32_t ST_MASK = (1u << 30) - 1;
 
+// One digit of a sort.  vin null: the values are the keys' indices (a sort's first pass), and the
+// keys are every `stride`-th u64.
+// Bound by the look-back's latency (118k items are 58 tiles, all resident at once, and a pass moves
+// 2.8 MB): a thread loads the status of kLook predecessors before it uses any, so a chain of tiles
+// whose counts are published costs one round trip per kLook tiles (10.1 -> 8.9 us a pass; 32 at a time
+// and tiles of 512 or 1,024 items: 10-11 us).
+constexpr int kLook = 8;
 __global__ void __launch_bounds__(SORT_THREADS) sort_pass_kernel(
-    const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin, uint64_t *__restrict__ kout,
+    const uint64_t *__restrict__ kin, uint32_t stride, const uint32_t *__restrict__ vin, uint64_t *__restrict__ kout,
     uint32_t *__restrict__ vout, uint32_t n, uint32_t shift, const uint32_t *__restrict__ gofs,
     uint32_t *__restrict__ status, uint32_t *__restrict__ tile_ctr, uint32_t *__restrict__ err,
     unsigned long long spin_ns, uint32_t hold_tile0) {
@@ -424,8 +424,8 @@ __global__ void __launch_bounds__(SORT_THREADS) sort_pass_kernel(
   for (int k = 0; k < SORT_IPT; ++k) {
     const uint32_t idx = base + k * 32;
     if (idx < n) {
-      key[k] = kin[idx];
-      val[k] = vin[idx];
+      key[k] = kin[(size_t)idx * stride];
+      val[k] = vin ? vin[idx] : idx;
       dig[k] = (uint32_t)(key[k] >> shift) & (RADIX - 1);
     } else {
       key[k] = 0;
@@ -465,22 +465,31 @@ __global__ void __launch_bounds__(SORT_THREADS) sort_pass_kernel(
       uint32_t excl = 0;
       int32_t t = (int32_t)tile - 1;
       unsigned long long t0 = 0;
-      while (t >= 0) {
-        const uint32_t s = st[(size_t)t * RADIX + d];
-        if ((s & ~ST_MASK) == 0) {
-          if (t0 == 0) t0 = globaltimer();
-          else if (globaltimer() - t0 > spin_ns) {
-            atomicOr(err, DEV_ERR_TIMEOUT);
-            break;
+      bool found = false;
+      while (t >= 0 && !found) {
+        uint32_t s[kLook];
+#pragma unroll
+        for (int k = 0; k < kLook; ++k) s[k] = t >= k ? st[(size_t)(t - k) * RADIX + d] : 0u;
+        int used = 0;
+#pragma unroll
+        for (int k = 0; k < kLook; ++k) {
+          if (used == k && !found && (s[k] & ~ST_MASK) != 0) {
+            excl += s[k] & ST_MASK;
+            found = (s[k] & ST_PREFIX) != 0;
+            used = k + 1;
           }
-          continue;
         }
-        t0 = 0;
-        excl += s & ST_MASK;
-        if (s & ST_PREFIX) break;
-        --t;
+        t -= used;
+        if (used) {
+          t0 = 0;
+        } else if (t0 == 0) {
+          t0 = globaltimer();
+        } else if (globaltimer() - t0 > spin_ns) {
+          atomicOr(err, DEV_ERR_TIMEOUT);
+          break;
+        }
       }
-      __threadfence();
+      // (no fence: the status word is all that is passed on)
       st[(size_t)tile * RADIX + d] = ST_PREFIX | (excl + sum);
       dbase[d] = gofs[d] + excl;
     }
@@ -513,6 +522,61 @@ __device__ __forceinline__ unsigned long long ms_pack(uint32_t cnt, uint32_t tg)
   return ((unsigned long long)(cnt & 0x3FFFFFFFu) << 32) | tg;
 }
 
+// Warp 0 resolves the exclusive prefix of tile `tile` over tiles [0, tile)
+// by decoupled look-back: 32 predecessors per step.  `agg` is this tile's
+// (count, targets) aggregate.  Returns the prefix in every lane.
+__device__ __forceinline__ void warp_lookback(unsigned long long *status, uint32_t tile, uint32_t agg_c,
+                                              uint32_t agg_t, uint32_t *err, unsigned long long spin_ns,
+                                              uint32_t *pre_c, uint32_t *pre_t) {
+  const uint32_t lane = threadIdx.x & 31u;
+  volatile unsigned long long *st = status;
+  if (tile == 0) {
+    if (lane == 0) st[0] = MS_PREFIX | ms_pack(agg_c, agg_t);
+    *pre_c = 0;
+    *pre_t = 0;
+    return;
+  }
+  if (lane == 0) st[tile] = MS_AGG | ms_pack(agg_c, agg_t);
+  uint32_t ec = 0, et = 0;
+  int32_t base = (int32_t)tile - 1;
+  unsigned long long t0 = 0;
+  while (base >= 0) {
+    const int32_t idx = base - (int32_t)lane;
+    const unsigned long long s = idx >= 0 ? st[idx] : (MS_PREFIX | 0ull);
+    const uint32_t flag = (uint32_t)(s >> 62);
+    const uint32_t ready = __ballot_sync(0xFFFFFFFFu, flag != 0);
+    const uint32_t pref = __ballot_sync(0xFFFFFFFFu, flag == 2u);
+    // lanes up to (and including) the nearest prefix must all be ready
+    const uint32_t need = pref ? ((pref & (0u - pref)) << 1) - 1u : 0xFFFFFFFFu;
+    if ((ready & need) != need) {
+      if (t0 == 0) t0 = globaltimer();
+      else if (globaltimer() - t0 > spin_ns) {
+        if (lane == 0) atomicOr(err, DEV_ERR_TIMEOUT);
+        break;
+      }
+      continue;
+    }
+    t0 = 0;
+    uint32_t c = (need >> lane) & 1u ? (uint32_t)((s >> 32) & 0x3FFFFFFFu) : 0u;
+    uint32_t t = (need >> lane) & 1u ? (uint32_t)s : 0u;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
+      t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
+    }
+    ec += c;
+    et += t;
+    if (pref) break;
+    base -= 32;
+  }
+  if (lane == 0) st[tile] = MS_PREFIX | ms_pack(ec + agg_c, et + agg_t);  // (no fence: the word is all that is passed on)
+  *pre_c = ec;
+  *pre_t = et;
+}
+
+// a(1-b) + b(1-a), written as a + b(1-2a): two fused multiply-adds.
+__device__ __forceinline__ double xor_merge(double a, double b) { return fma(b, fma(-2.0, a, 1.0), a); }
+
 // Mask word i of the words where mechanism d's symptom can be non-zero: the
 // union of its points' non-zero masks (a word whose mask bit is clear has a
 // zero snapshot at that point, so it adds nothing to the symptom).
@@ -525,12 +589,24 @@ __device__ __forceinline__ uint64_t symptom_mask(const CircuitDev &C, uint64_t d
   return b;
 }
 
+// One thread per sorted position.  A run's probability is a segmented scan of the XOR-merge over its
+// positions: a tree inside a tile, and a run still open at its tile's end is followed by the whole
+// block, MERGE_THREADS positions at a time (one thread following its run alone waited for three
+// dependent loads per position: 503 us for the 118k mechanisms of a circuit whose runs are 300 long,
+// against 26 us).  The tree is deterministic and differs from a left-to-right fold by a few ulps.
 __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(MergeLaunch L) {
+  constexpr uint32_t NW = MERGE_THREADS / 32;
   const CircuitDev C = *L.c_dev;
   extern __shared__ uint2 sband[];  // [w]
   __shared__ uint32_t s_tile;
   __shared__ uint32_t wsum_c[MERGE_THREADS / 32], wsum_t[MERGE_THREADS / 32];
   __shared__ uint32_t s_pre_c, s_pre_t;
+  __shared__ double s_p[MERGE_THREADS];        // folded probability of the run that starts at a position
+  __shared__ double s_tail[NW], s_more[NW];    // each warp's open run; a chunk past the tile
+  __shared__ uint32_t s_last[NW];              // each warp's last run start (position in the tile + 1; 0: none)
+  __shared__ uint32_t s_first[NW];             // a run starts at the warp's first position
+  __shared__ ulonglong2 s_key;                 // the key of the run open at the tile's end
+  __shared__ uint32_t s_open;                  // its first position in the tile (MERGE_THREADS: none follows)
   const uint32_t w = L.w;
   for (uint32_t j = threadIdx.x; j < w; j += blockDim.x) sband[j] = C.band[j];
   if (threadIdx.x == 0) s_tile = atomicAdd(L.tile_ctr, 1u);
@@ -540,8 +616,9 @@ __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(MergeLaunch L) {
   const uint32_t n = L.n;
   const uint32_t ntiles = (n + MERGE_THREADS - 1) / MERGE_THREADS;
 
-  bool head = false;
+  bool head = false, newgroup = true;
   uint32_t ntg = 0, m = 0;
+  double q = 0.0;  // (0 leaves a run as it is)
   ulonglong2 k = make_ulonglong2(0, 0);
   // After a sort pass timed out (DEV_ERR_TIMEOUT, the compile fails) the
   // permutation may hold stale entries: an index past n is never followed.
@@ -551,8 +628,8 @@ __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(MergeLaunch L) {
     m = 0;
   } else if (i < n) {
     k = L.key[m];
+    q = __ldg(C.mp + m);
     const uint64_t d = __ldg(C.mdesc + m);
-    bool newgroup = true;
     const uint32_t mp = i > 0 ? L.perm[i - 1] : 0u;
     if (i > 0 && mp < n) {
       const ulonglong2 kp = L.key[mp];
@@ -604,67 +681,102 @@ __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(MergeLaunch L) {
     wsum_t[warp] = t_inc;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t ac = 0, at = 0;
-    for (int x = 0; x < MERGE_THREADS / 32; ++x) {
-      const uint32_t c = wsum_c[x], t = wsum_t[x];
-      wsum_c[x] = ac;
-      wsum_t[x] = at;
-      ac += c;
-      at += t;
+  // runs inside the warp: the segmented inclusive scan of q
+  const uint32_t hb = __ballot_sync(0xFFFFFFFFu, newgroup);
+  const uint32_t le = hb & (0xFFFFFFFFu >> (31u - lane));
+  const uint32_t seg0 = le ? 31u - __clz(le) : 0u;
+  double x = q;
+#pragma unroll
+  for (uint32_t o = 1; o < 32; o <<= 1) {
+    const double y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+    if (lane >= o && lane - o >= seg0) x = xor_merge(y, x);
+  }
+  if (lane == 31) {
+    s_tail[warp] = x;
+    s_last[warp] = hb ? warp * 32u + 32u - __clz(hb) : 0u;
+    s_first[warp] = hb & 1u;
+  }
+  __syncthreads();
+  {
+    // the run open at the warp's start: its value over the warps before, and where it starts (0: before the tile)
+    double carry = 0.0;
+    uint32_t open = 0;
+    for (uint32_t v = 0; v < warp; ++v) {
+      carry = s_last[v] ? s_tail[v] : xor_merge(carry, s_tail[v]);
+      open = s_last[v] ? s_last[v] : open;
     }
-    // decoupled look-back over preceding tiles
-    volatile unsigned long long *st = L.status;
-    uint32_t pc = 0, pt = 0;
-    if (tile == 0) {
-      st[0] = MS_PREFIX | ms_pack(ac, at);
-    } else {
-      st[tile] = MS_AGG | ms_pack(ac, at);
-      int32_t t = (int32_t)tile - 1;
-      unsigned long long t0 = 0;
-      while (t >= 0) {
-        const unsigned long long s = st[t];
-        if ((s >> 62) == 0) {
-          if (t0 == 0) t0 = globaltimer();
-          else if (globaltimer() - t0 > L.spin_ns) {
-            atomicOr(L.err, DEV_ERR_TIMEOUT);
-            break;
-          }
-          continue;
-        }
-        t0 = 0;
-        pc += (uint32_t)((s >> 32) & 0x3FFFFFFFu);
-        pt += (uint32_t)s;
-        if (s & MS_PREFIX) break;
-        --t;
+    if (le == 0) x = xor_merge(carry, x);
+    else open = warp * 32u + seg0 + 1u;
+    const bool last = lane == 31 ? threadIdx.x == MERGE_THREADS - 1 || s_first[warp + 1]
+                                 : ((hb >> (lane + 1u)) & 1u) != 0u;
+    // (the run's last position in the tile: positions past n start runs of their own)
+    if (last && open) s_p[open - 1] = x;
+    if (threadIdx.x == MERGE_THREADS - 1) {
+      s_open = open && i < n && (k.x | k.y) != 0 ? open - 1u : MERGE_THREADS;
+      s_key = k;
+    }
+  }
+  if (threadIdx.x < 32) {
+    const uint32_t wc = lane < NW ? wsum_c[lane] : 0u, wt = lane < NW ? wsum_t[lane] : 0u;
+    uint32_t ec = wc, et = wt;
+#pragma unroll
+    for (uint32_t o = 1; o < NW; o <<= 1) {
+      const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, ec, o), b = __shfl_up_sync(0xFFFFFFFFu, et, o);
+      if (lane >= o) {
+        ec += a;
+        et += b;
       }
-      __threadfence();
-      st[tile] = MS_PREFIX | ms_pack(pc + ac, pt + at);
     }
-    s_pre_c = pc;
-    s_pre_t = pt;
-    if (tile == ntiles - 1) {
-      L.totals[0] = pc + ac;
-      L.totals[1] = pt + at;
-      if (pc + ac <= n) L.out_off[pc + ac] = pt + at;  // the closing offset (past n only after a timed-out look-back)
-      if (pt + at > L.tg_cap) atomicOr(L.err, DEV_FLAG_TG_OVF);
+    const uint32_t ac = __shfl_sync(0xFFFFFFFFu, ec, NW - 1), at = __shfl_sync(0xFFFFFFFFu, et, NW - 1);
+    if (lane < NW) {
+      wsum_c[lane] = ec - wc;
+      wsum_t[lane] = et - wt;
+    }
+    uint32_t pc = 0, pt = 0;
+    warp_lookback(L.status, tile, ac, at, L.err, L.spin_ns, &pc, &pt);
+    if (lane == 0) {
+      s_pre_c = pc;
+      s_pre_t = pt;
+      if (tile == ntiles - 1) {
+        L.totals[0] = pc + ac;
+        L.totals[1] = pt + at;
+        if (pc + ac <= n) L.out_off[pc + ac] = pt + at;  // the closing offset (past n only after a timed-out look-back)
+        if (pt + at > L.tg_cap) atomicOr(L.err, DEV_FLAG_TG_OVF);
+      }
     }
   }
   __syncthreads();
+  // a run still open at the tile's end: the block folds its positions in the tiles after
+  if (s_open < MERGE_THREADS) {
+    const ulonglong2 ko = s_key;
+    for (uint32_t i2 = (tile + 1) * MERGE_THREADS + threadIdx.x;; i2 += MERGE_THREADS) {
+      double q2 = 0.0;
+      bool same = false;
+      const uint32_t m2 = i2 < n ? L.perm[i2] : n;
+      if (m2 < n) {  // (past n: the end, or a stale entry after a timed-out sort pass)
+        const ulonglong2 k2 = L.key[m2];
+        same = k2.x == ko.x && k2.y == ko.y;
+        if (same) q2 = __ldg(C.mp + m2);
+      }
+#pragma unroll
+      for (uint32_t o = 16; o > 0; o >>= 1) q2 = xor_merge(q2, __shfl_down_sync(0xFFFFFFFFu, q2, o));
+      if (lane == 0) s_more[warp] = q2;
+      const int all = __syncthreads_and(same ? 1 : 0);
+      if (threadIdx.x == 0) {
+        double p = s_p[s_open];
+#pragma unroll
+        for (uint32_t v = 0; v < NW; ++v) p = xor_merge(p, s_more[v]);
+        s_p[s_open] = p;
+      }
+      __syncthreads();
+      if (!all) break;
+    }
+  }
   if (!head) return;
   const uint32_t slot = s_pre_c + wsum_c[warp] + c_inc - c_in;
   if (slot >= n) return;  // only after a timed-out look-back
   const uint32_t toff = s_pre_t + wsum_t[warp] + t_inc - t_in;
-  // fold the run's probabilities left to right
-  double p = __ldg(C.mp + m);
-  for (uint32_t i2 = i + 1; i2 < n; ++i2) {
-    const uint32_t m2 = L.perm[i2];
-    if (m2 >= n) break;  // stale entry after a timed-out sort pass
-    const ulonglong2 k2 = L.key[m2];
-    if (k2.x != k.x || k2.y != k.y) break;
-    const double q = __ldg(C.mp + m2);
-    p = p * (1.0 - q) + q * (1.0 - p);
-  }
+  const double p = s_p[threadIdx.x];
   L.out_prob[slot] = p;
   L.out_off[slot] = toff;
   if ((uint64_t)toff + ntg <= L.tg_cap) {
@@ -689,60 +801,6 @@ __device__ __forceinline__ bool item_less(ulonglong2 a, uint32_t ma, ulonglong2 
   if (a.x != b.x) return a.x < b.x;
   if (a.y != b.y) return a.y < b.y;
   return ma < mb;
-}
-
-// Warp 0 resolves the exclusive prefix of tile `tile` over tiles [0, tile)
-// by decoupled look-back: 32 predecessors per step.  `agg` is this tile's
-// (count, targets) aggregate.  Returns the prefix in lane 0.
-__device__ __forceinline__ void warp_lookback(unsigned long long *status, uint32_t tile, uint32_t agg_c,
-                                              uint32_t agg_t, uint32_t *err, uint32_t *pre_c, uint32_t *pre_t) {
-  const uint32_t lane = threadIdx.x & 31u;
-  volatile unsigned long long *st = status;
-  if (tile == 0) {
-    if (lane == 0) st[0] = MS_PREFIX | ms_pack(agg_c, agg_t);
-    *pre_c = 0;
-    *pre_t = 0;
-    return;
-  }
-  if (lane == 0) st[tile] = MS_AGG | ms_pack(agg_c, agg_t);
-  uint32_t ec = 0, et = 0;
-  int32_t base = (int32_t)tile - 1;
-  unsigned long long t0 = 0;
-  while (base >= 0) {
-    const int32_t idx = base - (int32_t)lane;
-    const unsigned long long s = idx >= 0 ? st[idx] : (MS_PREFIX | 0ull);
-    const uint32_t flag = (uint32_t)(s >> 62);
-    const uint32_t ready = __ballot_sync(0xFFFFFFFFu, flag != 0);
-    const uint32_t pref = __ballot_sync(0xFFFFFFFFu, flag == 2u);
-    // lanes up to (and including) the nearest prefix must all be ready
-    const uint32_t need = pref ? ((pref & (0u - pref)) << 1) - 1u : 0xFFFFFFFFu;
-    if ((ready & need) != need) {
-      if (t0 == 0) t0 = globaltimer();
-      else if (globaltimer() - t0 > kSpinLimitNs) {
-        if (lane == 0) atomicOr(err, DEV_ERR_TIMEOUT);
-        break;
-      }
-      continue;
-    }
-    t0 = 0;
-    uint32_t c = (need >> lane) & 1u ? (uint32_t)((s >> 32) & 0x3FFFFFFFu) : 0u;
-    uint32_t t = (need >> lane) & 1u ? (uint32_t)s : 0u;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
-      t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
-    }
-    ec += c;
-    et += t;
-    if (pref) break;
-    base -= 32;
-  }
-  if (lane == 0) {
-    __threadfence();
-    st[tile] = MS_PREFIX | ms_pack(ec + agg_c, et + agg_t);
-  }
-  *pre_c = ec;
-  *pre_t = et;
 }
 
 // Loads a target list as 16-byte vectors (rows are 16-byte aligned).
@@ -851,7 +909,7 @@ __global__ void __launch_bounds__(BUCKET_THREADS) bucket_merge_kernel(BucketMerg
   }
   if (threadIdx.x < 32) {
     uint32_t pc = 0, pt = 0;
-    warp_lookback(L.status, b, carry_c, carry_t, L.err, &pc, &pt);
+    warp_lookback(L.status, b, carry_c, carry_t, L.err, kSpinLimitNs, &pc, &pt);
     if (threadIdx.x == 0) {
       s_pre_c = pc;
       s_pre_t = pt;
@@ -898,9 +956,6 @@ __global__ void __launch_bounds__(BUCKET_THREADS) bucket_merge_kernel(BucketMerg
 constexpr uint32_t GW_WARPS = 8;  // buckets per group/emit block (one warp each)
 
 __device__ __forceinline__ bool key_eq(ulonglong2 a, ulonglong2 b) { return a.x == b.x && a.y == b.y; }
-
-// a(1-b) + b(1-a), written as a + b(1-2a): two fused multiply-adds.
-__device__ __forceinline__ double xor_merge(double a, double b) { return fma(b, fma(-2.0, a, 1.0), a); }
 
 // One warp per bucket of at most WARP_CAP items; larger buckets are listed
 // for group_big_kernel.  Items are ordered by sub-bin (top 6 bits of the
@@ -1489,22 +1544,15 @@ cudaError_t launch_bucket_merge(const BucketMergeLaunch &L, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_sort_init(const ulonglong2 *key, uint64_t *sortkey, uint32_t *perm, uint32_t M, cudaStream_t s) {
-  if (M == 0) return cudaSuccess;
-  uint32_t blocks = (M + 255) / 256;
-  if (blocks > 152u * 16u) blocks = 152u * 16u;
-  sort_init_kernel<<<blocks, 256, 0, s>>>(key, sortkey, perm, M);
-  return cudaGetLastError();
-}
-
 size_t sort_scratch_words(uint32_t n, uint32_t bits) {
   const uint32_t passes = (bits + RADIX_BITS - 1) / RADIX_BITS;
   // hist + status + tile counters, for a 128-bit fallback as well (2 sorts)
   return 2 * ((size_t)passes * RADIX + (size_t)passes * sort_tiles(n) * RADIX + passes);
 }
 
-cudaError_t launch_sort(uint64_t *keys, uint64_t *keys_alt, uint32_t *vals, uint32_t *vals_alt, uint32_t n,
-                        uint32_t bits, const SortScratch &scr, cudaStream_t s, bool *result_in_alt) {
+cudaError_t launch_sort(const uint64_t *first, uint32_t stride, bool index_vals, uint64_t *keys, uint64_t *keys_alt,
+                        uint32_t *vals, uint32_t *vals_alt, uint32_t n, uint32_t shift0, uint32_t bits,
+                        const SortScratch &scr, cudaStream_t s, bool *result_in_alt) {
   *result_in_alt = false;
   if (n == 0) return cudaSuccess;
   const uint32_t passes = (bits + RADIX_BITS - 1) / RADIX_BITS;
@@ -1512,12 +1560,14 @@ cudaError_t launch_sort(uint64_t *keys, uint64_t *keys_alt, uint32_t *vals, uint
   const uint32_t tiles = sort_tiles(n);
   uint32_t hb = (n + 1023) / 1024;
   if (hb > 152u * 4u) hb = 152u * 4u;
-  sort_hist_kernel<<<hb, 1024, 0, s>>>(keys, n, passes, scr.hist);
+  sort_hist_kernel<<<hb, 1024, 0, s>>>(first, stride, n, shift0, passes, scr.hist);
   sort_scan_kernel<<<passes, RADIX, 0, s>>>(scr.hist);
   uint64_t *ki = keys, *ko = keys_alt;
   uint32_t *vi = vals, *vo = vals_alt;
   for (uint32_t p = 0; p < passes; ++p) {
-    sort_pass_kernel<<<tiles, SORT_THREADS, 0, s>>>(ki, vi, ko, vo, n, p * RADIX_BITS, scr.hist + p * RADIX,
+    sort_pass_kernel<<<tiles, SORT_THREADS, 0, s>>>(p == 0 ? first : ki, p == 0 ? stride : 1u,
+                                                    p == 0 && index_vals ? nullptr : vi, ko, vo, n,
+                                                    shift0 + p * RADIX_BITS, scr.hist + p * RADIX,
                                                     scr.status + (size_t)p * tiles * RADIX, scr.tile_ctr + p,
                                                     scr.err, scr.spin_ns, p == 0 ? scr.hold_first : 0u);
     uint64_t *tk = ki;
