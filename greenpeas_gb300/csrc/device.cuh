@@ -121,14 +121,12 @@ enum : uint32_t { SEG_FIRST = 0, SEG_AFF = 1, SEG_XFER = 2, SEG_REST = 3 };
 // from the dense transfer columns): measured on code circuits, rows hold 1-3
 // entries on average and up to 12 where a cut falls inside a round.
 constexpr uint32_t kSegRowCap = 16;
-// Entries of a row that the compose ring copies into shared memory (entries
-// kSegRingCap .. kSegRowCap - 1, rare, are read from global memory).
-constexpr uint32_t kSegRingCap = 8;
-// Most compose steps a REST item keeps in flight (shared-memory ring).
-constexpr uint32_t kSegRingMax = 4;
+// Entries of a row that the compose prefetches (one 16-byte load; entries
+// kSegNear .. kSegRowCap - 1, rare, are loaded when they are needed).
+constexpr uint32_t kSegNear = 8;
 struct SegItem {
   uint32_t kind;
-  uint32_t idx;             // word (SEG_XFER: transfer column)
+  uint32_t idx;             // word (SEG_XFER: first transfer column of the item's SegLaunch::cols)
   uint32_t e_begin, e_end;  // epochs walked
   uint32_t state;           // FIRST/AFF/XFER: state written at exit (0xFFFFFFFF: none); REST: entry state
   uint32_t s_from, s_to;    // REST: compose through segments [s_from, s_to) before walking; XFER: s_from
@@ -141,21 +139,21 @@ struct SegLaunch {
   const SegItem *items;
   uint32_t n_items;
   uint32_t threads, qpt, qpad;
-  uint32_t chunk_cap, max_epochs, max_chunks;
+  uint32_t max_epochs;
+  uint32_t cols;            // transfer columns a SEG_XFER item walks (ncol is a multiple of it)
   uint64_t *state;          // [states][2 qpad]
   uint32_t xfer0;           // state of segment s's transfer column c: xfer0 + s * ncol + c
-  uint32_t ncol;            // 64-row columns of a transfer matrix: ceil(2 qpad / 64)
+  uint32_t ncol;            // 64-row columns of a transfer matrix: ceil(2 qpad / 64), rounded up to cols
   const uint32_t *aff;      // [w][S] state of word j's SEG_AFF walk of segment s (0xFFFFFFFF: no measurements)
   uint32_t S;
   uint32_t *xcnt;           // [S][2 qpad] (zeroed) entries of each transfer row
-  uint16_t *xlst;           // entries 0..7 [S][2 qpad][kSegRingCap], then entries 8..15 [S][2 qpad][8]
-  uint32_t ring_nb;         // compose step buffers of a REST CTA (launch B; 0 in launch A)
-  uint32_t *err;
+  uint16_t *xlst;           // entries 0..7 [S][2 qpad][kSegNear], then entries 8..15 [S][2 qpad][8]
 };
 // Dynamic shared memory of a segment launch (0: it does not fit a CTA).
 size_t walk_seg_smem_bytes(const SegLaunch &L);
-cudaError_t launch_walk_seg(const SegLaunch &L, cudaStream_t s);
-bool walk_seg_supported(uint32_t qpt);
+cudaError_t launch_walk_seg(const SegLaunch &L, bool rest, cudaStream_t s);  // launch A, or (rest) launch B
+bool walk_seg_supported(uint32_t qpad, uint32_t qpt);
+uint32_t walk_seg_cols(uint32_t qpad, uint32_t qpt);  // transfer columns per SEG_XFER item
 // Staged epoch/chunk table bytes for a launch (0: the tables are read from global memory).
 uint32_t walk_table_bytes(uint32_t max_epochs, uint32_t max_chunks);
 size_t walk_smem_bytes(uint32_t qpad, uint32_t chunk_cap, uint32_t table_bytes, uint32_t words);

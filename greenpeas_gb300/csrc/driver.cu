@@ -541,7 +541,7 @@ struct gpc_driver {
   std::vector<gpc::SegItem> seg_items;
   uint32_t seg_na = 0, seg_nb = 0;
   std::vector<uint32_t> seg_aff;  // [w][S]
-  uint32_t seg_states = 0, seg_xfer0 = 0, seg_ncol = 0, seg_qpt = 1, seg_ring = 1;
+  uint32_t seg_states = 0, seg_xfer0 = 0, seg_ncol = 0, seg_qpt = 1, seg_cols = 1;
   bool seg_band_reset = false;    // a word without measurements: its band is zeroed before the walk
   // host phases of the last prepare / fetch (ms): lower, layout, staging,
   // wait for the pipeline + result sizes, D2H copies, DEM split
@@ -1155,7 +1155,7 @@ struct gpc_driver {
       mix(seg_nb);
       mix(seg_states);
       mix(seg_qpt);
-      mix(seg_ring);
+      mix(seg_cols);
       for (uint32_t b : seg_bounds) mix(b);
     }
     cfg_sig = h;
@@ -1244,52 +1244,22 @@ struct gpc_driver {
   }
 
   // ---- segmented walk (one circuit) ----------------------------------------
-  // Auto policy: segments of about kSegTarget cost units (an epoch costs its
+  // Auto policy: segments of about seg_target() cost units (an epoch costs its
   // slots + 2), taken when the longest word walk is at least kSegMinSpan
-  // segments long.  Measured on GB300 (walk stage, L2 flushed between runs):
-  // [[144,12,12]] r12 77 -> 41 us at 32 (16: 53, 48: 42), surface d = 7 61 ->
-  // 34, d = 11 86 -> 41, [[72,12,6]] 42 -> 30, [[288,12,18]] 129 -> 77 (48:
-  // 69); surface d = 3 walks 17 epochs and stays whole (segmenting it costs
-  // 2-5 us; its longest walk costs 123 units, under kSegMinSpan segments).
-  // A compose step costs about 1 us (instruction latency of one CTA
-  // over a sparse transfer matrix), a segment epoch about 0.8 us.  Segment
-  // walks copy the tape in chunks of at most kSegChunk bytes that never cross
-  // a cut, so several segment CTAs share an SM and a segment's first copy is
-  // short.
-  static constexpr uint32_t kSegTarget = 32;
+  // segments long.  A short segment means short walks and more compose steps
+  // (about 0.5 us each); a large circuit's segment CTAs fill the GPU (one per
+  // SM from ~600 slots on), so it is bound by their number and wants fewer.
+  // Measured on GB300 (walk stage with its event, whole / 32 / 64 / 96 units,
+  // us): [[144,12,12]] r12 77 / 28.5 / 30.8 / 39, surface d = 11 77 / 26 / 33 /
+  // 45, [[288,12,18]] 129 / 59 / 65 / 57, d = 17 - / 57 / 53 / 59, d = 21 192 /
+  // 104 / 98 / 100, d = 25 291 / 166 / 143 / 133; surface d = 3 walks 17 epochs
+  // and stays whole (its longest walk costs 123 units).
+  static uint32_t seg_target(uint32_t qpad) { return 32u * (1u + qpad / 512u); }
   static constexpr uint32_t kSegMinSpan = 4;
-  static constexpr uint32_t kSegChunk = 24 * 1024;
   // A detector word's rows vanish some epochs after its last measurement
   // (the walk reaches the resets of the qubits they sit on); its segments
   // reach this many epochs past that measurement, the last one walking on.
   static constexpr uint32_t kSegTail = 12;
-
-  // Chunks of whole epochs of at most the chunk capacity, cut at every bound.
-  static void rechunk_at(Tape &T, const std::vector<uint32_t> &bounds, uint32_t cap_want) {
-    const uint32_t nE = T.n_epochs;
-    uint64_t big = 0;
-    for (uint32_t e = 0; e < nE; ++e) big = std::max<uint64_t>(big, (uint64_t)T.ep_k[e] * T.qpad * 8);
-    const uint64_t want = std::max<uint64_t>((big + 255) & ~(uint64_t)255, cap_want);
-    T.chunk_cap = (uint32_t)std::min<uint64_t>(gpc::walk_chunk_cap(T.qpad), want);
-    T.ep_chunk.assign(nE, 0);
-    T.ch_off.clear();
-    T.ch_bytes.clear();
-    for (size_t s = 0; s + 1 < bounds.size(); ++s) {
-      for (uint32_t e = bounds[s]; e < bounds[s + 1];) {
-        const uint32_t c = (uint32_t)T.ch_off.size();
-        uint64_t bytes = 0;
-        uint32_t f = e;
-        while (f < bounds[s + 1] && bytes + (uint64_t)T.ep_k[f] * T.qpad * 8 <= T.chunk_cap) {
-          bytes += (uint64_t)T.ep_k[f] * T.qpad * 8;
-          T.ep_chunk[f] = c;
-          ++f;
-        }
-        T.ch_off.push_back(T.ep_opoff[e]);
-        T.ch_bytes.push_back((uint32_t)bytes);
-        e = f;
-      }
-    }
-  }
 
   // Decides whether the single circuit's walk runs in segments and builds
   // the items of the two launches (device.cuh, SEG_*).
@@ -1301,7 +1271,7 @@ struct gpc_driver {
     const uint32_t nE = T.n_epochs;
     if (nE < 2 || T.w == 0) return;
     const uint32_t q = walk_qpt_for(T.qpad, walk_qpt);
-    if (!gpc::walk_seg_supported(q) || !walk_qpt_fits(T.qpad, q)) return;
+    if (!walk_qpt_fits(T.qpad, q) || !gpc::walk_seg_supported(T.qpad, q)) return;
     std::vector<uint64_t> cum(nE + 1, 0);  // cost of epochs [0, e)
     for (uint32_t e = 0; e < nE; ++e) cum[e + 1] = cum[e] + gpc::walk_epoch_cost(T.ep_k[e]);
     auto holds_obs = [&](uint32_t j) { return (uint64_t)(j + 1) * 64 > T.ndet; };
@@ -1312,7 +1282,7 @@ struct gpc_driver {
       const uint32_t hi = holds_obs(j) ? nE : std::min(nE, T.inj_hi[j] + 1);
       longest = std::max<uint64_t>(longest, cum[hi] - cum[lo]);
     }
-    const uint32_t target = walk_segment > 0 ? (uint32_t)walk_segment : kSegTarget;
+    const uint32_t target = walk_segment > 0 ? (uint32_t)walk_segment : seg_target(T.qpad);
     if (walk_segment == 0 && longest < (uint64_t)kSegMinSpan * target) return;
     gpc::walk_segment_bounds(T, target, seg_bounds);
     const uint32_t S = (uint32_t)seg_bounds.size() - 1;
@@ -1322,7 +1292,8 @@ struct gpc_driver {
       return (uint32_t)(std::upper_bound(b.begin(), b.end(), e) - b.begin()) - 1;
     };
     seg_qpt = q;
-    seg_ncol = (2 * T.qpad + 63) / 64;
+    seg_cols = gpc::walk_seg_cols(T.qpad, q);
+    seg_ncol = ((2 * T.qpad + 63) / 64 + seg_cols - 1) / seg_cols * seg_cols;
     seg_aff.assign((size_t)T.w * S, gpc::kNone);
     std::vector<gpc::SegItem> A, B;
     std::vector<char> need_xfer(S, 0);
@@ -1355,32 +1326,15 @@ struct gpc_driver {
     seg_xfer0 = states;
     for (uint32_t s = 0; s < S; ++s)
       if (need_xfer[s])
-        for (uint32_t c = 0; c < seg_ncol; ++c)
+        for (uint32_t c = 0; c < seg_ncol; c += seg_cols)
           A.push_back(gpc::SegItem{gpc::SEG_XFER, c, b[s], b[s + 1], seg_xfer0 + s * seg_ncol + c, s, 0, 0});
     seg_states = seg_xfer0 + S * seg_ncol;
-    rechunk_at(T, seg_bounds, kSegChunk);
-    // compose ring: as many step buffers (2 to kSegRingMax: step k + 1 is copied while step k is
-    // composed) as the REST CTA's shared memory holds
-    uint32_t max_steps = 0;
-    for (const auto &it : B) max_steps = std::max(max_steps, it.s_to - it.s_from);
-    seg_ring = 0;
-    for (uint32_t nb = std::min(gpc::kSegRingMax, std::max(2u, max_steps)); nb >= 2; --nb) {
-      gpc::SegLaunch probe{};
-      probe.qpad = T.qpad;
-      probe.chunk_cap = T.chunk_cap;
-      probe.max_epochs = nE;
-      probe.max_chunks = (uint32_t)T.ch_off.size();
-      probe.S = S;
-      probe.ring_nb = nb;
-      if (gpc::walk_seg_smem_bytes(probe)) {
-        seg_ring = nb;
-        break;
-      }
-    }
-    if (seg_ring == 0) {  // no room for a compose step: the plain walk, with the tape's usual chunks
-      rechunk_at(T, {0u, nE}, 0xFFFFFFFFu);
-      return;
-    }
+    gpc::SegLaunch probe{};
+    probe.qpad = T.qpad;
+    probe.cols = seg_cols;
+    probe.max_epochs = nE;
+    probe.S = S;
+    if (!gpc::walk_seg_smem_bytes(probe)) return;  // (the plain walk)
     // longest items first (launch order is the order CTAs start in)
     auto span = [&](const gpc::SegItem &it) {
       return cum[it.e_end] - cum[it.e_begin] + (it.kind == gpc::SEG_REST ? 8ull * (it.s_to - it.s_from) : 0ull);
@@ -1412,9 +1366,8 @@ struct gpc_driver {
     sl.qpt = seg_qpt;
     sl.qpad = T.qpad;
     sl.threads = T.qpad / seg_qpt;
-    sl.chunk_cap = T.chunk_cap;
     sl.max_epochs = T.n_epochs;
-    sl.max_chunks = (uint32_t)T.ch_off.size();
+    sl.cols = seg_cols;
     sl.state = dptr<uint64_t>(L.seg_state);
     sl.xfer0 = seg_xfer0;
     sl.ncol = seg_ncol;
@@ -1422,13 +1375,10 @@ struct gpc_driver {
     sl.S = (uint32_t)seg_bounds.size() - 1;
     sl.xcnt = dptr<uint32_t>(L.seg_xcnt);
     sl.xlst = dptr<uint16_t>(L.seg_xlst);
-    sl.err = dptr<uint32_t>(L.err);
-    sl.ring_nb = 0;
-    CK(gpc::launch_walk_seg(sl, stream));
+    CK(gpc::launch_walk_seg(sl, false, stream));
     sl.items += seg_na;
     sl.n_items = seg_nb;
-    sl.ring_nb = seg_ring;
-    CK(gpc::launch_walk_seg(sl, stream));
+    CK(gpc::launch_walk_seg(sl, true, stream));
     CK(cudaStreamWaitEvent(stream, join_ev[0], 0));
   }
 

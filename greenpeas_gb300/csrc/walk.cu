@@ -134,219 +134,6 @@ __device__ __forceinline__ void mbar_inval(uint64_t *bar) {
 
 enum : uint32_t { ITEM_DONE = 0, ITEM_EMPTY = 1, ITEM_ABORTED = 2 };
 
-// What walk_item runs: the plain walk of words j0 .. j0+W-1, or one item of
-// the segmented walk (device.cuh: SEG_*; one word per CTA).
-enum : int { MODE_PLAIN = 0, MODE_FIRST = 1, MODE_AFF = 2, MODE_XFER = 3, MODE_REST = 4 };
-
-// One segment item as walk_item sees it.
-struct SegCtx {
-  uint32_t e_begin, e_end;  // epochs walked
-  uint64_t *out;            // FIRST / AFF / XFER: exit rows ([2 qpad]; null: none)
-  const uint64_t *in;       // REST: entry rows of segment s_from
-  const uint64_t *state;    // all states (transfer columns, AFF exits)
-  const uint32_t *aff_row;  // REST: [S] AFF state of this word in each segment (kNoState: none)
-  uint32_t *xcnt;           // [S][2 qpad] entries of each transfer row (XFER adds, REST reads)
-  uint16_t *xlst;           // entries (the rows at the segment's start, as word offsets in a published
-                            // buffer: 2 slot for X, 2 slot + 1 for Z): [S][2 qpad][kSegRingCap] entries
-                            // 0..7, then [S][2 qpad][kSegRowCap - kSegRingCap] entries 8..15
-  uint32_t xfer0, ncol, s_from, s_to;
-  uint32_t col, seg;        // XFER: the unit column walked, its segment
-  uint32_t ring_nb;         // REST: step buffers of the compose ring
-  uint32_t S;               // segments of the plan (sizes the staged AFF table)
-};
-constexpr uint32_t kNoState = 0xFFFFFFFFu;
-
-// Bytes of one compose step in shared memory: entry counts (u32), entries
-// 0..7 (kSegRingCap u16) and the segment's AFF rows (u64) of every row.
-__host__ __device__ constexpr size_t seg_step_bytes(uint32_t qpad) {
-  return (size_t)2 * qpad * (4 + 2 * kSegRingCap + 8);
-}
-
-// XFER exit: the set bits of row r's word of column col, as entries of the
-// row's sparse list (order is free: the compose XORs them).  An entry is the
-// row's word offset in a published buffer, so the compose adds it to the
-// buffer's address as it is.
-__device__ __forceinline__ void seg_list_add(const SegCtx &sc, uint32_t n2, uint32_t r, uint64_t w) {
-  const size_t row = (size_t)sc.seg * n2 + r;
-  const uint32_t qpad = n2 / 2u;
-  uint16_t *const hi = sc.xlst + (size_t)sc.S * n2 * kSegRingCap;
-  for (; w; w &= w - 1) {
-    const uint32_t j = sc.col * 64u + (uint32_t)(__ffsll((long long)w) - 1);
-    const uint16_t wj = (uint16_t)(j < qpad ? 2u * j : 2u * (j - qpad) + 1u);
-    const uint32_t pos = atomicAdd(sc.xcnt + row, 1u);
-    if (pos < kSegRingCap)
-      sc.xlst[row * kSegRingCap + pos] = wj;
-    else if (pos < kSegRowCap)
-      hi[row * (kSegRowCap - kSegRingCap) + pos - kSegRingCap] = wj;
-  }
-}
-
-// One transfer row of one compose step, held in registers: its entry count,
-// its first eight entries (u16 pairs) and its AFF row.
-struct SegRow {
-  uint32_t n;
-  uint32_t e[4];
-  uint64_t c;
-};
-
-// REST: composes the entry rows of segment s_to from those of s_from, one
-// segment at a time: rows <- A_s rows ^ c_s.  Row r of A_s is the sparse list
-// of the rows at the segment's start that feed it (XFER built it; a row
-// with more than kSegRowCap entries is read from the dense transfer columns
-// instead: bit r' mod 64 of word r of column r' / 64).  The current rows sit
-// in the published buffer, so a thread reads the rows its entries name from
-// shared memory.  Each step's lists and AFF rows are copied into a ring of
-// ring_nb shared-memory buffers by cp.async.bulk, issued ring_nb - 1 steps
-// ahead by lane 0 of the last warp on one mbarrier per buffer (mbar[2 + b]);
-// thread 0 issues the walk's first tape copies (issue_walk_copies).  A thread keeps the
-// next step's row lists in registers (loaded while the current step runs: they
-// do not depend on its result), so a step's chain is: publish the rows, one
-// barrier, the entries' loads from the published rows, XOR.  Waits are
-// bounded and a timeout aborts the item.  CTA-wide (barriers); one word per
-// CTA.  Returns false after a wait gave up (in-flight ring copies have been
-// waited for).
-template <int QPT, typename F>
-__device__ __forceinline__ bool seg_compose(uint64_t (&X)[QPT][1], uint64_t (&Z)[QPT][1], const SegCtx &sc,
-                                            ulonglong2 *pub, const uint32_t qpad, uint64_t *mbar,
-                                            unsigned char *ring, const uint32_t *s_aff, uint32_t *err,
-                                            F &&issue_walk_copies) {
-  const uint32_t T = blockDim.x, tid = threadIdx.x;
-  const uint32_t n2 = 2 * qpad;
-  const uint32_t steps = sc.s_to - sc.s_from, NB = sc.ring_nb;
-  const size_t step_bytes = seg_step_bytes(qpad);
-  const uint32_t cnt_b = n2 * 4u, lst_b = n2 * 2u * kSegRingCap, c_b = n2 * 8u;
-  const uint16_t *const xhi = sc.xlst + (size_t)sc.S * n2 * kSegRingCap;  // entries 8..15
-  // the ring's copies are issued by lane 0 of the last warp (whose slots are
-  // the packing's padding when there is any), so the first warp is not held up
-  const uint32_t issuer = T - 32u;
-  uint32_t issued = 0, waited = 0;  // steps issued (issuer) / seen complete (this thread)
-  auto issue = [&]() {  // issuer: the next step into its ring buffer
-    const uint32_t k = issued++;
-    const uint32_t s = sc.s_from + k;
-    unsigned char *dst = ring + (size_t)(k % NB) * step_bytes;
-    uint64_t *bar = &mbar[2 + k % NB];
-    const uint32_t ai = s_aff[s];
-    mbar_expect_tx(bar, cnt_b + lst_b + (ai == kNoState ? 0u : c_b));
-    bulk_g2s(dst, sc.xcnt + (size_t)s * n2, cnt_b, bar);
-    bulk_g2s(dst + cnt_b, sc.xlst + (size_t)s * n2 * kSegRingCap, lst_b, bar);
-    if (ai != kNoState) bulk_g2s(dst + cnt_b + lst_b, sc.state + (size_t)ai * n2, c_b, bar);
-  };
-  if (tid == issuer) {
-    while (issued < min(NB, steps)) issue();
-  }
-  if (tid == 0) issue_walk_copies();  // the walk's first tape chunks (thread 0 owns them), needed after the compose
-  bool bad = false;
-  auto wait_step = [&](uint32_t k) {
-    if (!mbar_wait_bounded(&mbar[2 + k % NB], (k / NB) & 1u)) bad = true;
-    else waited = k + 1;
-  };
-  const unsigned char *const ring_c = ring;
-  auto load_row = [&](uint32_t k, uint32_t r, SegRow &m) {
-    const unsigned char *buf = ring_c + (size_t)(k % NB) * step_bytes;
-    m.n = reinterpret_cast<const uint32_t *>(buf)[r];
-    const uint4 e = reinterpret_cast<const uint4 *>(buf + cnt_b)[r];  // entries 0..7
-    m.e[0] = e.x;
-    m.e[1] = e.y;
-    m.e[2] = e.z;
-    m.e[3] = e.w;
-    m.c = s_aff[sc.s_from + k] != kNoState ? reinterpret_cast<const uint64_t *>(buf + cnt_b + lst_b)[r] : 0ull;
-  };
-  // the published rows as words: word 2 j of a buffer is X of slot j, word 2 j + 1 its Z
-  const uint32_t pub_s0 = smem_u32(pub);
-  auto word_addr = [&](uint32_t pbuf, uint32_t j) -> uint32_t {
-    return pbuf + (j < qpad ? j * 16u : (j - qpad) * 16u + 8u);
-  };
-  // row r of step k: its AFF row XOR the published rows its entries name.
-  // The loads of a row issue together, without branches: entries past the
-  // row's count read a shared word that is always zero (four loads always,
-  // four more for a row of five to eight entries: rows of one role share a
-  // warp).  A step takes as long as its slowest row's chain, since a barrier
-  // follows.
-  __shared__ uint64_t s_zero;
-  if (tid == 0) s_zero = 0;  // read after the first step's barrier
-  const uint32_t zaddr = smem_u32(&s_zero);
-  auto apply = [&](uint32_t k, uint32_t r, const SegRow &m, uint64_t self, uint32_t pbuf) -> uint64_t {
-    uint64_t v = m.c;
-    if (m.n <= kSegRowCap) {
-#pragma unroll
-      for (uint32_t i = 0; i < 4; ++i) {
-        const uint32_t wj = (m.e[i >> 1] >> ((i & 1u) * 16u)) & 0xFFFFu;
-        v ^= lds64(i < m.n ? pbuf + wj * 8u : zaddr);
-      }
-      if (m.n > 4) {
-#pragma unroll
-        for (uint32_t i = 4; i < kSegRingCap; ++i) {
-          const uint32_t wj = (m.e[i >> 1] >> ((i & 1u) * 16u)) & 0xFFFFu;
-          v ^= lds64(i < m.n ? pbuf + wj * 8u : zaddr);
-        }
-      }
-      if (m.n > kSegRingCap) {  // entries 8..15 (rare): from global memory
-        const uint4 t = __ldg(reinterpret_cast<const uint4 *>(
-            xhi + ((size_t)(sc.s_from + k) * n2 + r) * (kSegRowCap - kSegRingCap)));
-        const uint32_t e2[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-        for (uint32_t i = 0; i < kSegRowCap - kSegRingCap; ++i) {
-          const uint32_t wj = (e2[i >> 1] >> ((i & 1u) * 16u)) & 0xFFFFu;
-          v ^= lds64(i + kSegRingCap < m.n ? pbuf + wj * 8u : zaddr);
-        }
-      }
-    } else {  // a long row: its words from the dense transfer columns
-      const uint64_t *tm = sc.state + (size_t)(sc.xfer0 + (sc.s_from + k) * sc.ncol) * n2;
-      for (uint32_t c = 0; c < sc.ncol; ++c)
-        for (uint64_t w = __ldg(tm + (size_t)c * n2 + r); w; w &= w - 1) {
-          const uint32_t j = c * 64u + (uint32_t)(__ffsll((long long)w) - 1);
-          v ^= j == r ? self : j < n2 ? lds64(word_addr(pbuf, j)) : 0ull;
-        }
-    }
-    return v;
-  };
-  SegRow mx[QPT], mz[QPT];
-  if (steps) {
-    wait_step(0);
-#pragma unroll
-    for (int u = 0; u < QPT; ++u) {
-      load_row(0, tid + (uint32_t)u * T, mx[u]);
-      load_row(0, qpad + tid + (uint32_t)u * T, mz[u]);
-    }
-  }
-  for (uint32_t k = 0; k < steps; ++k) {
-    ulonglong2 *pb = pub + (size_t)(k & 1u) * qpad;
-#pragma unroll
-    for (int u = 0; u < QPT; ++u) pb[tid + u * T] = make_ulonglong2(X[u][0], Z[u][0]);
-    if (__syncthreads_or(bad ? 1 : 0)) {
-      bad = true;
-      break;
-    }
-    // every thread is done with step k - 1's buffer
-    if (tid == issuer && k >= 1 && issued < steps) issue();
-    const uint32_t pbuf = pub_s0 + (k & 1u) * qpad * 16u;
-#pragma unroll
-    for (int u = 0; u < QPT; ++u) {
-      const uint32_t slot = tid + (uint32_t)u * T;
-      const uint64_t nx = apply(k, slot, mx[u], X[u][0], pbuf);
-      const uint64_t nz = apply(k, qpad + slot, mz[u], Z[u][0], pbuf);
-      X[u][0] = nx;
-      Z[u][0] = nz;
-    }
-    if (k + 1 < steps) {
-      wait_step(k + 1);
-#pragma unroll
-      for (int u = 0; u < QPT; ++u) {
-        load_row(k + 1, tid + (uint32_t)u * T, mx[u]);
-        load_row(k + 1, qpad + tid + (uint32_t)u * T, mz[u]);
-      }
-    }
-  }
-  if (bad && tid == issuer) {
-    atomicOr(err, DEV_ERR_TIMEOUT);
-    // copies still in flight target this CTA's shared memory
-    for (uint32_t k = waited; k < issued; ++k)
-      if (!mbar_wait_bounded(&mbar[2 + k % NB], (k / NB) & 1u)) break;
-  }
-  __syncthreads();  // the walk publishes into buffer 0 next, which may have been read last
-  return !bad;
-}
-
 // One walk item: the words j0 .. j0+W-1 of circuit C (rows W x 64 bits per
 // qubit; a batch halves its CTAs with W = 2 while each epoch's latency chain
 // stays about the same), walked by the whole CTA.  `pub_slots` lays out the
@@ -357,21 +144,12 @@ __device__ __forceinline__ bool seg_compose(uint64_t (&X)[QPT][1], uint64_t (&Z)
 // multiple of 32, so whole warps idle).  Returns ITEM_EMPTY when the words
 // inject nothing (the mbarriers were not initialised), ITEM_ABORTED after a
 // bounded wait gave up, else ITEM_DONE.  CTA-uniform.
-//
-// Segment items (MODE != MODE_PLAIN, W = 1, `sc` given) walk [e_begin, e_end)
-// only: FIRST from zero rows with snapshots (and the word's band), AFF from
-// zero rows without snapshots, XFER from unit rows without measurement bits
-// or snapshots (stopping once the rows vanish), REST from composed entry rows
-// with snapshots (a REST that stops early lowers the band's end).
-template <int QPT, int W, bool QUEUE, int MODE = MODE_PLAIN>
+template <int QPT, int W, bool QUEUE>
 __device__ __forceinline__ uint32_t walk_item(const CircuitDev &C, const uint32_t j0, unsigned char *smem,
                                               const uint32_t pub_slots, const uint32_t chunk_cap,
                                               const uint32_t table_bytes, uint32_t *__restrict__ err,
-                                              uint32_t &s_abort, const SegCtx *sc = nullptr) {
-  constexpr bool SEG = MODE != MODE_PLAIN;
-  constexpr bool SNAPS = MODE == MODE_PLAIN || MODE == MODE_FIRST || MODE == MODE_REST;
-  static_assert(!SEG || (W == 1 && !QUEUE), "segment items walk one word per CTA");
-  const uint32_t nw = SEG ? 1u : min((uint32_t)W, C.w - j0);  // words of this CTA (the circuit's last group may be short)
+                                              uint32_t &s_abort) {
+  const uint32_t nw = min((uint32_t)W, C.w - j0);  // words of this CTA (the circuit's last group may be short)
   const uint32_t T = blockDim.x;
   const uint32_t tid = threadIdx.x;
   const uint32_t qpad = C.qpad;
@@ -382,24 +160,18 @@ __device__ __forceinline__ uint32_t walk_item(const CircuitDev &C, const uint32_
 
   // the CTA walks from the earliest first injection of its words to the
   // latest last injection (and on until every row is zero)
-  uint32_t e0 = 0xFFFFFFFFu, elast = 0, e_end = nE;
-  if constexpr (SEG) {
-    e0 = sc->e_begin;
-    e_end = sc->e_end;
-    if constexpr (MODE != MODE_XFER) elast = C.inj_hi[j0];
-  } else {
+  uint32_t e0 = 0xFFFFFFFFu, elast = 0;
 #pragma unroll
-    for (int wi = 0; wi < W; ++wi) {
-      if ((uint32_t)wi >= nw) break;
-      const uint32_t lo = C.inj_lo[j0 + wi];
-      if (lo == 0xFFFFFFFFu || lo >= nE) continue;
-      e0 = min(e0, lo);
-      elast = max(elast, C.inj_hi[j0 + wi]);
-    }
-    if (e0 == 0xFFFFFFFFu) {
-      if (tid < nw) C.band[j0 + tid] = make_uint2(0u, 0u);
-      return ITEM_EMPTY;
-    }
+  for (int wi = 0; wi < W; ++wi) {
+    if ((uint32_t)wi >= nw) break;
+    const uint32_t lo = C.inj_lo[j0 + wi];
+    if (lo == 0xFFFFFFFFu || lo >= nE) continue;
+    e0 = min(e0, lo);
+    elast = max(elast, C.inj_hi[j0 + wi]);
+  }
+  if (e0 == 0xFFFFFFFFu) {
+    if (tid < nw) C.band[j0 + tid] = make_uint2(0u, 0u);
+    return ITEM_EMPTY;
   }
 
   // shared memory: [published rows x2][mbarriers][tables][chunk buffer x2]
@@ -409,23 +181,11 @@ __device__ __forceinline__ uint32_t walk_item(const CircuitDev &C, const uint32_
   off += 128;
   uint2 *etab = reinterpret_cast<uint2 *>(smem + off);  // epoch e0+i: (op offset, slots | chunk << 8)
   const uint32_t c0 = C.ep_chunk[e0];
-  const uint32_t c_end = SEG ? C.ep_chunk[e_end - 1] + 1 : C.n_chunks;  // chunks past the last one walked
-  const uint32_t ne = e_end - e0, nc = c_end - c0;
+  const uint32_t ne = nE - e0, nc = C.n_chunks - c0;
   const bool staged = ((size_t)ne + nc) * sizeof(uint2) <= table_bytes;
   uint2 *ctab = etab + ne;  // chunk c0+i: (op offset, bytes)
   off += table_bytes;
   unsigned char *buf = smem + off;  // two buffers of chunk_cap bytes
-  // REST: [S aff states (u32, 16-byte rounded)][ring_nb compose step buffers]
-  uint32_t *s_aff = nullptr;
-  unsigned char *ring = nullptr;
-  if constexpr (MODE == MODE_REST) {
-    off += (size_t)2 * chunk_cap;
-    s_aff = reinterpret_cast<uint32_t *>(smem + off);
-    off += ((size_t)sc->S * 4 + 15) & ~(size_t)15;
-    ring = smem + ((off + 127) & ~(size_t)127);
-    for (uint32_t i = tid; i < sc->s_to; i += T) s_aff[i] = sc->aff_row[i];
-  }
-
   if (staged) {
     for (uint32_t i = tid; i < ne; i += T)
       etab[i] = make_uint2(C.ep_opoff[e0 + i], C.ep_k[e0 + i] | (C.ep_chunk[e0 + i] << 8));
@@ -435,8 +195,6 @@ __device__ __forceinline__ uint32_t walk_item(const CircuitDev &C, const uint32_
     s_abort = 0;
     mbar_init(&mbar[0], 1);
     mbar_init(&mbar[1], 1);
-    if constexpr (MODE == MODE_REST)
-      for (uint32_t b = 0; b < sc->ring_nb; ++b) mbar_init(&mbar[2 + b], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -457,42 +215,16 @@ __device__ __forceinline__ uint32_t walk_item(const CircuitDev &C, const uint32_
     bulk_g2s(buf + (size_t)(issued & 1u) * chunk_cap, C.ops + ck.x, ck.y, bar);
     ++issued;
   };
-  auto issue_first_chunks = [&]() {
+  if (tid == 0) {
     issue();
     if (nc > 1) issue();
-  };
-  // (REST: after the compose ring's first copies, which are needed first)
-  if (MODE != MODE_REST && tid == 0) issue_first_chunks();
+  }
 
   uint64_t X[QPT][W], Z[QPT][W], acc[QPT][W], last_inj[QPT][W];
-  bool compose_bad = false;
 #pragma unroll
   for (int u = 0; u < QPT; ++u)
 #pragma unroll
     for (int wi = 0; wi < W; ++wi) X[u][wi] = Z[u][wi] = acc[u][wi] = last_inj[u][wi] = 0;
-  if constexpr (MODE == MODE_XFER) {
-    // unit rows of column col: row r (X of slot r, or Z of slot r - qpad) holds bit r - 64 col
-#pragma unroll
-    for (int u = 0; u < QPT; ++u) {
-      const uint32_t xr = tid + (uint32_t)u * T, zr = qpad + xr;
-      if constexpr (W == 1) {
-        X[u][0] = (xr >> 6) == sc->col ? 1ull << (xr & 63u) : 0ull;
-        Z[u][0] = (zr >> 6) == sc->col ? 1ull << (zr & 63u) : 0ull;
-      }
-    }
-  } else if constexpr (MODE == MODE_REST) {
-    if constexpr (W == 1) {
-#pragma unroll
-      for (int u = 0; u < QPT; ++u) {
-        const uint32_t slot = tid + (uint32_t)u * T;
-        X[u][0] = __ldg(sc->in + slot);
-        Z[u][0] = __ldg(sc->in + qpad + slot);
-      }
-      compose_bad = !seg_compose<QPT>(X, Z, *sc, reinterpret_cast<ulonglong2 *>(smem), qpad, mbar, ring, s_aff,
-                                      err, issue_first_chunks);
-    }
-  }
-
   const uint32_t np = C.npoints;
   ulonglong2 *snap0 = C.snap + (size_t)j0 * np;  // word j0 + wi at + wi * np
   const uint32_t jlo = j0 * 64u;
@@ -501,7 +233,7 @@ __device__ __forceinline__ uint32_t walk_item(const CircuitDev &C, const uint32_
   unsigned long long *nzm0 = C.nzm + (j0 >> 6);
   const uint32_t mw = C.mw;
   const uint32_t jsh = j0 & 63u;
-  bool timed_out = compose_bad, aborted = false;  // (the walk's first barrier aborts after a failed compose)
+  bool timed_out = false, aborted = false;
   uint32_t e = e0;
   uint32_t seq = 0;
   uint32_t cur = 0xFFFFFFFFu;  // chunk whose data this thread has waited for
@@ -548,16 +280,15 @@ __device__ __forceinline__ uint32_t walk_item(const CircuitDev &C, const uint32_
       aborted = true;
       break;
     }
-    // (XFER has no measurement bits: its rows stay zero once they vanish)
-    if ((!any && (MODE == MODE_XFER || e > elast)) || e >= e_end) break;
+    if ((!any && e > elast) || e >= nE) break;
     const uint2 ek = ek_next;
-    if (e + 1 < e_end) ek_next = epoch(e + 1);  // used next epoch: its latency hides behind this one
+    if (e + 1 < nE) ek_next = epoch(e + 1);  // used next epoch: its latency hides behind this one
     const uint32_t K = ek.y & 0xFFu;
     const uint32_t ch = ek.y >> 8;
     if (ch != cur) {
       // (3) first epoch of a chunk: every thread has finished the previous
       //     chunk (barrier above), so its buffer can take the chunk after this one
-      if (tid == 0 && ch + 1 < c_end && c0 + issued == ch + 1) issue();
+      if (tid == 0 && ch + 1 < C.n_chunks && c0 + issued == ch + 1) issue();
       const uint32_t i = ch - c0;
       if (!mbar_wait_bounded(&mbar[i & 1u], (i >> 1) & 1u)) {
         timed_out = true;
@@ -588,7 +319,7 @@ __device__ __forceinline__ uint32_t walk_item(const CircuitDev &C, const uint32_
 #pragma unroll
           for (int wi = 0; wi < W; ++wi) Z[u][wi] ^= lds64(pa + wi * 16u + 8u);
         } else if (opc == OP_SNAP) {
-          if constexpr (SNAPS) snapshot(arg, X[u], Z[u]);
+          snapshot(arg, X[u], Z[u]);
         } else if (opc == OP_XPZ) {
 #pragma unroll
           for (int wi = 0; wi < W; ++wi) X[u][wi] ^= lds64(pa + wi * 16u + 8u);
@@ -613,7 +344,6 @@ __device__ __forceinline__ uint32_t walk_item(const CircuitDev &C, const uint32_
 #pragma unroll
             for (int wi = 0; wi < W; ++wi) X[u][wi] = Z[u][wi] = 0;
           } else if (opc == OP_INJ) {
-            if constexpr (MODE == MODE_XFER) continue;  // the linear part only
             // measurement bits (one or two) that fall in this CTA's words
             const uint32_t b2 = ((uint32_t)op >> 8) & 0xFFFFFFu;
             const uint32_t d1 = arg - jlo, d2 = b2 - jlo;
@@ -629,7 +359,6 @@ __device__ __forceinline__ uint32_t walk_item(const CircuitDev &C, const uint32_
             for (int wi = 0; wi < W; ++wi) {
               uint64_t inj = acc[u][wi];
               if (d1 - wi * 64u < 64u) inj |= 1ull << (d1 & 63u);
-              if constexpr (MODE == MODE_XFER) inj = 0;
               acc[u][wi] = 0;
               if (sub & 4u) X[u][wi] = Z[u][wi] = 0;
               if (basis != 1u) X[u][wi] ^= inj;
@@ -637,7 +366,6 @@ __device__ __forceinline__ uint32_t walk_item(const CircuitDev &C, const uint32_
               last_inj[u][wi] = inj;
             }
           } else if (opc == OP_SNAPD) {
-            if constexpr (!SNAPS) continue;
             if constexpr (W == 1) {
               snap0[arg] = make_ulonglong2(last_inj[u][0], 0ull);
               if (last_inj[u][0]) red_or(nzm0 + arg * mw, 1ull << jsh);
@@ -652,32 +380,7 @@ __device__ __forceinline__ uint32_t walk_item(const CircuitDev &C, const uint32_
       }
     }
   }
-  if constexpr (MODE == MODE_PLAIN) {
-    if (tid < nw) C.band[j0 + tid] = make_uint2(C.ep_ptoff[e0], C.ep_ptoff[e < nE ? e : nE]);
-  } else if constexpr (MODE == MODE_FIRST) {
-    // later segments (if any) cover up to the end unless they stop early
-    if (tid == 0) C.band[j0] = make_uint2(C.ep_ptoff[e0], C.ep_ptoff[e < e_end ? e : nE]);
-  } else if constexpr (MODE == MODE_REST) {
-    if (tid == 0 && e < e_end) atomicMin(&C.band[j0].y, C.ep_ptoff[e]);
-  }
-  if constexpr (MODE == MODE_XFER) {
-#pragma unroll
-    for (int u = 0; u < QPT; ++u) {
-      const uint32_t slot = tid + (uint32_t)u * T;
-      seg_list_add(*sc, 2 * qpad, slot, X[u][0]);
-      seg_list_add(*sc, 2 * qpad, qpad + slot, Z[u][0]);
-    }
-  }
-  if constexpr (MODE == MODE_FIRST || MODE == MODE_AFF || MODE == MODE_XFER) {
-    if (sc->out) {
-#pragma unroll
-      for (int u = 0; u < QPT; ++u) {
-        const uint32_t slot = tid + (uint32_t)u * T;
-        sc->out[slot] = X[u][0];
-        sc->out[qpad + slot] = Z[u][0];
-      }
-    }
-  }
+  if (tid < nw) C.band[j0 + tid] = make_uint2(C.ep_ptoff[e0], C.ep_ptoff[e < nE ? e : nE]);
   if (tid == 0) {
     // Copies still in flight target this CTA's shared memory: wait for them
     // (bounded) before the CTA exits or takes another item.
@@ -738,49 +441,404 @@ __global__ void __launch_bounds__(WalkBound<QPT>::value) walk_queue_kernel(const
   }
 }
 
-// Segmented walk of one circuit: one CTA per segment item (SEG_*).
+// ---- segmented walk of one circuit (device.cuh: SEG_*) ------------------------
+//
+// Bound by the latency of one CTA's epochs and compose steps (and, from ~600
+// slots on, by how many CTAs there are: one fits an SM), so both read global
+// memory ahead into registers and share only the published rows:
+//  * the tape is a stream of [slot][qubit] op rows, whatever their epochs, so a
+//    thread keeps its ops of the next kAhead rows in registers (an L2 load of
+//    ~700 cycles hides behind two or three rows of ~300);
+//  * a compose step's row lists are loaded while the step before it runs.
+// Chunks of whole epochs and a ring of step buffers in shared memory, filled
+// by bulk copies, needed 243 KB for the 896 slots of a d = 21 surface memory,
+// which therefore walked whole.  Walk stage before -> now: surface d = 25 (1,280
+// slots) 291 -> 133 us, d = 21 192 -> 98, [[144,12,12]] 34.7 -> 28.5.
+constexpr int kAhead = 4;
+constexpr uint32_t kNoState = 0xFFFFFFFFu;
+enum : int { MODE_FIRST = 0, MODE_AFF = 1, MODE_XFER = 2, MODE_REST = 3 };
+
+// Largest block of a segment kernel (registers: 64 and 72 a thread).
 template <int QPT>
-__global__ void __launch_bounds__(WalkBound<QPT>::value) walk_seg_kernel(const SegLaunch L, uint32_t table_bytes) {
+struct SegBound {
+  static constexpr uint32_t value = QPT == 1 ? 1024 : 896;
+};
+
+template <int W>
+__device__ __forceinline__ void lds_words(uint64_t (&v)[W], uint32_t a) {
+  if constexpr (W == 1) {
+    v[0] = lds64(a);
+  } else {
+#pragma unroll
+    for (int i = 0; i < W; i += 2) {
+      const ulonglong2 p = lds128(a + i * 8u);
+      v[i] = p.x;
+      v[i + 1] = p.y;
+    }
+  }
+}
+
+template <int W>
+__device__ __forceinline__ void sts_words(uint32_t a, const uint64_t (&v)[W]) {
+  if constexpr (W == 1) {
+    asm volatile("st.shared.u64 [%0], %1;" ::"r"(a), "l"(v[0]) : "memory");
+  } else {
+#pragma unroll
+    for (int i = 0; i < W; i += 2)
+      asm volatile("st.shared.v2.u64 [%0], {%1, %2};" ::"r"(a + i * 8u), "l"(v[i]), "l"(v[i + 1]) : "memory");
+  }
+}
+
+// Walks epochs [e0, e_end) from rows X, Z (W words per slot): FIRST and REST
+// store snapshots of word j, AFF does not, XFER leaves measurement bits out
+// too and stops once its rows vanish.  Published row r (X of slot r, or Z of
+// slot r - qpad) of buffer b is words [r * W, r * W + W) at pub + b * 2 qpad W
+// words; the first epoch publishes into buffer `seq` & 1.  Returns the epoch
+// the walk stopped at.
+template <int QPT, int W, int MODE>
+__device__ __forceinline__ uint32_t stream_walk(const CircuitDev &C, const uint32_t j, const uint32_t e0,
+                                                const uint32_t e_end, uint64_t (&X)[QPT][W], uint64_t (&Z)[QPT][W],
+                                                const uint32_t pub, const uint32_t *ks, uint32_t seq) {
+  constexpr bool SNAPS = MODE == MODE_FIRST || MODE == MODE_REST;
+  static_assert(W == 1 || MODE == MODE_XFER, "only transfer columns are walked several at a time");
+  const uint32_t T = blockDim.x, tid = threadIdx.x, qpad = C.qpad, nE = C.n_epochs;
+  const uint32_t op0 = C.ep_opoff[e0];
+  const uint32_t op1 = e_end < nE ? C.ep_opoff[e_end] : C.ep_opoff[nE - 1] + C.ep_k[nE - 1] * qpad;
+  uint32_t left = (op1 - op0) / qpad;  // op rows not loaded yet
+  const uint64_t *next = C.ops + op0 + tid;
+  uint64_t f[QPT][kAhead];
+#pragma unroll
+  for (int a = 0; a < kAhead; ++a) {
+#pragma unroll
+    for (int u = 0; u < QPT; ++u) f[u][a] = left ? __ldg(next + (uint32_t)u * T) : 0ull;
+    next += qpad;
+    left -= left ? 1u : 0u;
+  }
+  const uint32_t elast = MODE == MODE_XFER ? 0u : C.inj_hi[j];
+  ulonglong2 *const snap = C.snap + (size_t)j * C.npoints;
+  unsigned long long *const nzm = C.nzm + (j >> 6);
+  const uint32_t mw = C.mw;
+  const unsigned long long jbit = 1ull << (j & 63u);
+  const uint32_t jlo = j * 64u;
+  uint64_t acc[QPT], last_inj[QPT];
+#pragma unroll
+  for (int u = 0; u < QPT; ++u) acc[u] = last_inj[u] = 0;
+  uint32_t k_next = ks ? ks[0] : __ldg(C.ep_k + e0);
+  uint32_t e = e0;
+  for (;; ++e, ++seq) {
+    const uint32_t pb = pub + (seq & 1u) * qpad * (16u * W);
+#pragma unroll
+    for (int u = 0; u < QPT; ++u) {
+      const uint32_t slot = tid + (uint32_t)u * T;
+      sts_words<W>(pb + slot * (8u * W), X[u]);
+      sts_words<W>(pb + (qpad + slot) * (8u * W), Z[u]);
+    }
+    // the epoch barrier; past the word's last measurement it also tells whether any row is left
+    if (MODE == MODE_XFER || e <= elast) {
+      __syncthreads();
+    } else {
+      bool nz = false;
+#pragma unroll
+      for (int u = 0; u < QPT; ++u) nz |= (X[u][0] | Z[u][0]) != 0;
+      if (!__syncthreads_or(nz ? 1 : 0)) break;
+    }
+    if (e >= e_end) break;
+    const uint32_t K = k_next;
+    if (e + 1 < e_end) k_next = ks ? ks[e + 1 - e0] : __ldg(C.ep_k + e + 1);
+    for (uint32_t k = 0; k < K; ++k) {
+      uint64_t ops[QPT];
+#pragma unroll
+      for (int u = 0; u < QPT; ++u) {
+        ops[u] = f[u][0];
+#pragma unroll
+        for (int a = 0; a + 1 < kAhead; ++a) f[u][a] = f[u][a + 1];
+        f[u][kAhead - 1] = left ? __ldg(next + (uint32_t)u * T) : 0ull;
+      }
+      next += qpad;
+      left -= left ? 1u : 0u;
+#pragma unroll
+      for (int u = 0; u < QPT; ++u) {
+        const uint64_t op = ops[u];
+        const uint32_t opc = (uint32_t)op & 0xFFu;
+        if (opc == OP_NOP) continue;
+        const uint32_t arg = (uint32_t)(op >> 32);
+        if (opc >= OP_XPX) {  // one XOR with a partner row: X with X, Z with Z, X with Z
+          uint64_t v[W];
+          lds_words<W>(v, pb + (arg + (opc == OP_XPX ? 0u : qpad)) * (8u * W));
+#pragma unroll
+          for (int w = 0; w < W; ++w) {
+            X[u][w] ^= opc == OP_ZPZ ? 0ull : v[w];
+            Z[u][w] ^= opc == OP_ZPZ ? v[w] : 0ull;
+          }
+        } else if (opc == OP_SNAP) {
+          if constexpr (SNAPS) {
+            snap[arg] = make_ulonglong2(X[u][0], Z[u][0]);
+            if (X[u][0] | Z[u][0]) red_or(nzm + arg * mw, jbit);
+          }
+        } else {
+          const uint32_t sub = ((uint32_t)op >> 8) & 0xFFu;
+          if (opc == OP_C1) {
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+              const uint64_t x = X[u][w], z = Z[u][w];
+              X[u][w] = sel2(sub & 3u, x, z);
+              Z[u][w] = sel2(sub >> 2, x, z);
+            }
+          } else if (opc == OP_C2) {
+            uint64_t px[W], pz[W];
+            lds_words<W>(px, pb + arg * (8u * W));
+            lds_words<W>(pz, pb + (qpad + arg) * (8u * W));
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+              const uint64_t x = X[u][w], z = Z[u][w];
+              X[u][w] = sel4(sub & 15u, x, z, px[w], pz[w]);
+              Z[u][w] = sel4(sub >> 4, x, z, px[w], pz[w]);
+            }
+          } else if (opc == OP_R) {
+#pragma unroll
+            for (int w = 0; w < W; ++w) X[u][w] = Z[u][w] = 0;
+          } else if (opc == OP_M) {
+            if (sub & 4u) {
+#pragma unroll
+              for (int w = 0; w < W; ++w) X[u][w] = Z[u][w] = 0;
+            }
+            if constexpr (MODE != MODE_XFER) {
+              const uint32_t d1 = arg - jlo, basis = sub & 3u;
+              uint64_t inj = acc[u];
+              if (d1 < 64u) inj |= 1ull << d1;
+              acc[u] = 0;
+              if (basis != 1u) X[u][0] ^= inj;
+              if (basis != 0u) Z[u][0] ^= inj;
+              last_inj[u] = inj;
+            }
+          } else if (opc == OP_INJ) {
+            if constexpr (MODE != MODE_XFER) {
+              // measurement bits (one or two) that fall in this word
+              const uint32_t b2 = ((uint32_t)op >> 8) & 0xFFFFFFu;
+              const uint32_t d1 = arg - jlo, d2 = b2 - jlo;
+              if (d1 < 64u) acc[u] |= 1ull << d1;
+              if (b2 != 0xFFFFFFu && d2 < 64u) acc[u] |= 1ull << d2;
+            }
+          } else if (opc == OP_SNAPD) {
+            if constexpr (SNAPS) {
+              snap[arg] = make_ulonglong2(last_inj[u], 0ull);
+              if (last_inj[u]) red_or(nzm + arg * mw, jbit);
+            }
+          }
+        }
+      }
+    }
+  }
+  return e;
+}
+
+// The epochs' slot counts of [e0, e_end) in shared memory (null: they do not fit `bytes`).
+__device__ __forceinline__ const uint32_t *stage_epochs(const CircuitDev &C, uint32_t e0, uint32_t e_end, uint32_t *tab,
+                                                        uint32_t bytes) {
+  if ((e_end - e0) * 4u > bytes) return nullptr;
+  for (uint32_t i = threadIdx.x; i < e_end - e0; i += blockDim.x) tab[i] = C.ep_k[e0 + i];
+  return tab;
+}
+
+// XFER exit: the set bits of row r's word of column col, as entries (row
+// numbers at the segment's start) of the row's sparse list; their order is
+// free, the compose XORs them.
+__device__ __forceinline__ void seg_list_add(const SegLaunch &L, uint32_t seg, uint32_t col, uint32_t r, uint64_t w) {
+  const uint32_t n2 = 2 * L.qpad;
+  const size_t row = (size_t)seg * n2 + r;
+  uint16_t *const far = L.xlst + (size_t)L.S * n2 * kSegNear;
+  for (; w; w &= w - 1) {
+    const uint16_t j = (uint16_t)(col * 64u + (uint32_t)(__ffsll((long long)w) - 1));
+    const uint32_t pos = atomicAdd(L.xcnt + row, 1u);
+    if (pos < kSegNear)
+      L.xlst[row * kSegNear + pos] = j;
+    else if (pos < kSegRowCap)
+      far[row * (kSegRowCap - kSegNear) + pos - kSegNear] = j;
+  }
+}
+
+// Launch A: first parts, walks of later segments from zero rows, and transfer
+// columns (XW of them per CTA: a column's walk is the same chain of epochs,
+// so several at once cost little more than one).
+template <int QPT, int XW>
+__global__ void __launch_bounds__(SegBound<QPT>::value) seg_first_kernel(const SegLaunch L, uint32_t table_bytes) {
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ uint32_t s_abort;
   const SegItem it = L.items[blockIdx.x];
-  if (it.kind == SEG_REST && L.ring_nb < 2) {  // no compose ring in this launch
-    if (threadIdx.x == 0) atomicOr(L.err, DEV_ERR_TIMEOUT);
+  const CircuitDev &C = *L.circ;
+  const uint32_t T = blockDim.x, tid = threadIdx.x, qpad = L.qpad;
+  const size_t n2 = (size_t)2 * qpad;
+  const uint32_t pub = smem_u32(smem);
+  const uint32_t *ks = stage_epochs(C, it.e_begin, it.e_end, reinterpret_cast<uint32_t *>(smem + 2 * n2 * 8 * XW), table_bytes);
+  __syncthreads();
+  if (it.kind == SEG_XFER) {
+    // unit rows: row r (X of slot r, or Z of slot r - qpad) holds bit r - 64 col of column col
+    uint64_t X[QPT][XW], Z[QPT][XW];
+#pragma unroll
+    for (int u = 0; u < QPT; ++u) {
+      const uint32_t xr = tid + (uint32_t)u * T, zr = qpad + xr;
+#pragma unroll
+      for (int w = 0; w < XW; ++w) {
+        X[u][w] = (xr >> 6) == it.idx + w ? 1ull << (xr & 63u) : 0ull;
+        Z[u][w] = (zr >> 6) == it.idx + w ? 1ull << (zr & 63u) : 0ull;
+      }
+    }
+    stream_walk<QPT, XW, MODE_XFER>(C, 0, it.e_begin, it.e_end, X, Z, pub, ks, 0);
+#pragma unroll
+    for (int u = 0; u < QPT; ++u) {
+      const uint32_t slot = tid + (uint32_t)u * T;
+#pragma unroll
+      for (int w = 0; w < XW; ++w) {
+        uint64_t *out = L.state + (it.state + w) * n2;
+        out[slot] = X[u][w];
+        out[qpad + slot] = Z[u][w];
+        seg_list_add(L, it.s_from, it.idx + w, slot, X[u][w]);
+        seg_list_add(L, it.s_from, it.idx + w, qpad + slot, Z[u][w]);
+      }
+    }
     return;
   }
-  const CircuitDev C = *L.circ;
-  const size_t n2 = (size_t)2 * C.qpad;
-  SegCtx sc;
-  sc.e_begin = it.e_begin;
-  sc.e_end = it.e_end;
-  sc.out = it.kind != SEG_REST && it.state != kNoState ? L.state + (size_t)it.state * n2 : nullptr;
-  sc.in = it.kind == SEG_REST ? L.state + (size_t)it.state * n2 : nullptr;
-  sc.state = L.state;
-  sc.aff_row = L.aff + (size_t)(it.kind == SEG_XFER ? 0u : it.idx) * L.S;
-  sc.xfer0 = L.xfer0;
-  sc.ncol = L.ncol;
-  sc.s_from = it.s_from;
-  sc.s_to = it.s_to;
-  sc.col = it.idx;
-  sc.seg = it.s_from;
-  sc.xcnt = L.xcnt;
-  sc.xlst = L.xlst;
-  sc.ring_nb = L.ring_nb;
-  sc.S = L.S;
-  switch (it.kind) {
-    case SEG_FIRST:
-      walk_item<QPT, 1, false, MODE_FIRST>(C, it.idx, smem, C.qpad, L.chunk_cap, table_bytes, L.err, s_abort, &sc);
-      break;
-    case SEG_AFF:
-      walk_item<QPT, 1, false, MODE_AFF>(C, it.idx, smem, C.qpad, L.chunk_cap, table_bytes, L.err, s_abort, &sc);
-      break;
-    case SEG_XFER:
-      walk_item<QPT, 1, false, MODE_XFER>(C, 0, smem, C.qpad, L.chunk_cap, table_bytes, L.err, s_abort, &sc);
-      break;
-    default:
-      walk_item<QPT, 1, false, MODE_REST>(C, it.idx, smem, C.qpad, L.chunk_cap, table_bytes, L.err, s_abort, &sc);
-      break;
+  uint64_t X[QPT][1], Z[QPT][1];
+#pragma unroll
+  for (int u = 0; u < QPT; ++u) X[u][0] = Z[u][0] = 0;
+  if (it.kind == SEG_FIRST) {
+    const uint32_t e = stream_walk<QPT, 1, MODE_FIRST>(C, it.idx, it.e_begin, it.e_end, X, Z, pub, ks, 0);
+    // later segments (if any) cover up to the end unless they stop early
+    if (tid == 0) C.band[it.idx] = make_uint2(C.ep_ptoff[it.e_begin], C.ep_ptoff[e < it.e_end ? e : C.n_epochs]);
+  } else {
+    stream_walk<QPT, 1, MODE_AFF>(C, it.idx, it.e_begin, it.e_end, X, Z, pub, ks, 0);
   }
+  if (it.state != kNoState) {
+    uint64_t *out = L.state + (size_t)it.state * n2;
+#pragma unroll
+    for (int u = 0; u < QPT; ++u) {
+      const uint32_t slot = tid + (uint32_t)u * T;
+      out[slot] = X[u][0];
+      out[qpad + slot] = Z[u][0];
+    }
+  }
+}
+
+// One transfer row of one compose step: its entry count and first eight
+// entries (u16 pairs).
+struct SegRow {
+  uint32_t n;
+  uint4 e;
+};
+
+// Launch B: a later segment of a word.  Its entry rows are composed from the
+// first part's exit rows, one segment at a time: rows <- A_s rows ^ c_s, where
+// row r of A_s is the sparse list of the rows at the segment's start that feed
+// it (a row of more than kSegRowCap entries is read from the dense transfer
+// columns: bit r' mod 64 of word r of column r' / 64).  A step: publish the
+// rows, one barrier, the entries' loads from the published rows, XOR.  A
+// row's loads issue together, without branches: entries past its count read a
+// shared word that is always zero (four loads always, four more for a row of
+// five to eight entries: rows of one role share a warp).
+template <int QPT>
+__global__ void __launch_bounds__(SegBound<QPT>::value) seg_rest_kernel(const SegLaunch L, uint32_t table_bytes) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ uint64_t s_zero;
+  const SegItem it = L.items[blockIdx.x];
+  const CircuitDev &C = *L.circ;
+  const uint32_t T = blockDim.x, tid = threadIdx.x, qpad = L.qpad, n2 = 2 * qpad;
+  const uint32_t pub = smem_u32(smem);
+  unsigned char *const tab = smem + (size_t)2 * n2 * 8 * L.cols;
+  const uint32_t *ks = stage_epochs(C, it.e_begin, it.e_end, reinterpret_cast<uint32_t *>(tab), table_bytes);
+  uint32_t *s_aff = reinterpret_cast<uint32_t *>(tab + table_bytes);
+  const uint32_t steps = it.s_to - it.s_from;
+  for (uint32_t i = tid; i < steps; i += T) s_aff[i] = L.aff[(size_t)it.idx * L.S + it.s_from + i];
+  if (tid == 0) s_zero = 0;
+  uint64_t X[QPT][1], Z[QPT][1];
+  const uint64_t *const in = L.state + (size_t)it.state * n2;
+#pragma unroll
+  for (int u = 0; u < QPT; ++u) {
+    const uint32_t slot = tid + (uint32_t)u * T;
+    X[u][0] = __ldg(in + slot);
+    Z[u][0] = __ldg(in + qpad + slot);
+  }
+  const uint16_t *const far = L.xlst + (size_t)L.S * n2 * kSegNear;
+  const uint32_t zaddr = smem_u32(&s_zero);
+  auto load_row = [&](uint32_t k, uint32_t r, SegRow &m) {
+    const size_t row = (size_t)(it.s_from + k) * n2 + r;
+    m.n = __ldg(L.xcnt + row);
+    m.e = __ldg(reinterpret_cast<const uint4 *>(L.xlst + row * kSegNear));
+  };
+  auto apply = [&](uint32_t k, uint32_t r, const SegRow &m, uint32_t pb) -> uint64_t {
+    uint64_t v = 0;
+    const uint32_t e[4] = {m.e.x, m.e.y, m.e.z, m.e.w};
+    if (m.n <= kSegRowCap) {
+#pragma unroll
+      for (uint32_t i = 0; i < 4; ++i)
+        v ^= lds64(i < m.n ? pb + ((e[i >> 1] >> ((i & 1u) * 16u)) & 0xFFFFu) * 8u : zaddr);
+      if (m.n > 4) {
+#pragma unroll
+        for (uint32_t i = 4; i < kSegNear; ++i)
+          v ^= lds64(i < m.n ? pb + ((e[i >> 1] >> ((i & 1u) * 16u)) & 0xFFFFu) * 8u : zaddr);
+      }
+      if (m.n > kSegNear) {  // entries 8..15 (rare)
+        const uint4 t = __ldg(reinterpret_cast<const uint4 *>(
+            far + ((size_t)(it.s_from + k) * n2 + r) * (kSegRowCap - kSegNear)));
+        const uint32_t e2[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+        for (uint32_t i = 0; i < kSegRowCap - kSegNear; ++i)
+          v ^= lds64(i + kSegNear < m.n ? pb + ((e2[i >> 1] >> ((i & 1u) * 16u)) & 0xFFFFu) * 8u : zaddr);
+      }
+    } else {  // a long row: its words from the dense transfer columns
+      const uint64_t *tm = L.state + (size_t)(L.xfer0 + (it.s_from + k) * L.ncol) * n2;
+      for (uint32_t c = 0; c < L.ncol; ++c)
+        for (uint64_t w = __ldg(tm + (size_t)c * n2 + r); w; w &= w - 1) {
+          const uint32_t j = c * 64u + (uint32_t)(__ffsll((long long)w) - 1);
+          if (j < n2) v ^= lds64(pb + j * 8u);
+        }
+    }
+    return v;
+  };
+  SegRow mx[QPT], mz[QPT];
+  if (steps) {
+#pragma unroll
+    for (int u = 0; u < QPT; ++u) {
+      load_row(0, tid + (uint32_t)u * T, mx[u]);
+      load_row(0, qpad + tid + (uint32_t)u * T, mz[u]);
+    }
+  }
+  __syncthreads();  // the staged tables
+  for (uint32_t k = 0; k < steps; ++k) {
+    SegRow nx[QPT], nz[QPT];
+    uint64_t cx[QPT], cz[QPT];
+    const uint32_t ai = s_aff[k];
+#pragma unroll
+    for (int u = 0; u < QPT; ++u) {  // the next step's lists and this step's c, ahead of the barrier
+      const uint32_t slot = tid + (uint32_t)u * T;
+      if (k + 1 < steps) {
+        load_row(k + 1, slot, nx[u]);
+        load_row(k + 1, qpad + slot, nz[u]);
+      }
+      cx[u] = cz[u] = 0;
+      if (ai != kNoState) {
+        cx[u] = __ldg(L.state + (size_t)ai * n2 + slot);
+        cz[u] = __ldg(L.state + (size_t)ai * n2 + qpad + slot);
+      }
+    }
+    const uint32_t pb = pub + (k & 1u) * qpad * 16u;
+#pragma unroll
+    for (int u = 0; u < QPT; ++u) {
+      const uint32_t slot = tid + (uint32_t)u * T;
+      sts_words<1>(pb + slot * 8u, X[u]);
+      sts_words<1>(pb + (qpad + slot) * 8u, Z[u]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < QPT; ++u) {
+      const uint32_t slot = tid + (uint32_t)u * T;
+      X[u][0] = apply(k, slot, mx[u], pb) ^ cx[u];
+      Z[u][0] = apply(k, qpad + slot, mz[u], pb) ^ cz[u];
+      mx[u] = nx[u];
+      mz[u] = nz[u];
+    }
+  }
+  // (the walk goes on alternating the published buffers)
+  const uint32_t e = stream_walk<QPT, 1, MODE_REST>(C, it.idx, it.e_begin, it.e_end, X, Z, pub, ks, steps);
+  if (tid == 0 && e < it.e_end) atomicMin(&C.band[it.idx].y, C.ep_ptoff[e]);
 }
 
 }  // namespace
@@ -814,13 +872,12 @@ cudaError_t walk_queue_set_limit_one(int optin) {
                               optin - (int)a.sharedSizeBytes);
 }
 
-template <int QPT>
-cudaError_t walk_seg_set_limit_one(int optin) {
+template <typename K>
+cudaError_t walk_seg_set_limit_one(K kernel, int optin) {
   cudaFuncAttributes a{};
-  cudaError_t e = cudaFuncGetAttributes(&a, walk_seg_kernel<QPT>);
+  cudaError_t e = cudaFuncGetAttributes(&a, kernel);
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(walk_seg_kernel<QPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              optin - (int)a.sharedSizeBytes);
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)a.sharedSizeBytes);
 }
 
 cudaError_t walk_set_smem_limit() {
@@ -841,8 +898,11 @@ cudaError_t walk_set_smem_limit() {
   if (e == cudaSuccess) e = walk_queue_set_limit_one<2, 1>(optin);
   if (e == cudaSuccess) e = walk_queue_set_limit_one<1, 2>(optin);
   if (e == cudaSuccess) e = walk_queue_set_limit_one<2, 2>(optin);
-  if (e == cudaSuccess) e = walk_seg_set_limit_one<1>(optin);
-  if (e == cudaSuccess) e = walk_seg_set_limit_one<2>(optin);
+  if (e == cudaSuccess) e = walk_seg_set_limit_one(seg_first_kernel<1, 1>, optin);
+  if (e == cudaSuccess) e = walk_seg_set_limit_one(seg_first_kernel<1, 2>, optin);
+  if (e == cudaSuccess) e = walk_seg_set_limit_one(seg_first_kernel<2, 4>, optin);
+  if (e == cudaSuccess) e = walk_seg_set_limit_one(seg_rest_kernel<1>, optin);
+  if (e == cudaSuccess) e = walk_seg_set_limit_one(seg_rest_kernel<2>, optin);
   return e;
 }
 
@@ -936,26 +996,43 @@ cudaError_t launch_walk(const WalkLaunch &L, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-bool walk_seg_supported(uint32_t qpt) { return qpt == 1 || qpt == 2; }
+bool walk_seg_supported(uint32_t qpad, uint32_t qpt) {
+  return (qpt == 1 && qpad <= SegBound<1>::value) || (qpt == 2 && qpad / 2 <= SegBound<2>::value);
+}
 
+// A large circuit's transfer columns are walked several per CTA: its CTAs fill the GPU, and a walk of two
+// columns costs little more than one of one (d = 21: walk stage 113 -> 98 us with two, d = 25: 153 -> 151 with
+// four for two); a small circuit has SMs to spare and wants the shorter walk.
+uint32_t walk_seg_cols(uint32_t qpad, uint32_t qpt) { return qpt == 2 ? 4u : qpad > 512 ? 2u : 1u; }
+
+// Epoch table bytes a segment CTA stages (0: read from global memory).
+static uint32_t seg_table_bytes(uint32_t max_epochs) {
+  return (uint64_t)max_epochs * 4 <= kWalkTableBudget ? (max_epochs * 4 + 15) / 16 * 16 : 0u;
+}
+
+// Both launches: the published rows twice (cols words each), the epoch table, the AFF states.
 size_t walk_seg_smem_bytes(const SegLaunch &L) {
-  const uint32_t tb = walk_table_bytes(L.max_epochs, L.max_chunks);
-  size_t b = walk_smem_bytes(L.qpad, L.chunk_cap, tb, 1);
-  if (L.ring_nb) b = ((b + ((size_t)L.S * 4 + 15) / 16 * 16 + 127) & ~(size_t)127) + L.ring_nb * seg_step_bytes(L.qpad);
+  const size_t b = (size_t)2 * 2 * L.qpad * 8 * L.cols + seg_table_bytes(L.max_epochs) + ((size_t)L.S * 4 + 15) / 16 * 16;
   return b <= 227 * 1024 - 1024 ? b : 0;
 }
 
-cudaError_t launch_walk_seg(const SegLaunch &L, cudaStream_t s) {
+cudaError_t launch_walk_seg(const SegLaunch &L, bool rest, cudaStream_t s) {
   if (L.n_items == 0) return cudaSuccess;
-  const uint32_t tb = walk_table_bytes(L.max_epochs, L.max_chunks);
+  const uint32_t tb = seg_table_bytes(L.max_epochs);
   const size_t smem = walk_seg_smem_bytes(L);
-  // a compose ring needs two buffers at least: step k + 1's copy is issued
-  // only once every thread is done with step k - 1's buffer
-  if (smem == 0 || L.ring_nb > kSegRingMax || L.ring_nb == 1) return cudaErrorInvalidValue;
-  if (!walk_seg_supported(L.qpt) || L.threads * L.qpt != L.qpad || L.threads > walk_max_threads(L.qpt))
-    return cudaErrorInvalidValue;
-  if (L.qpt == 1) walk_seg_kernel<1><<<L.n_items, L.threads, smem, s>>>(L, tb);
-  else walk_seg_kernel<2><<<L.n_items, L.threads, smem, s>>>(L, tb);
+  if (smem == 0) return cudaErrorInvalidValue;
+  if (!walk_seg_supported(L.qpad, L.qpt) || L.threads * L.qpt != L.qpad || L.ncol % L.cols) return cudaErrorInvalidValue;
+  if (rest) {
+    if (L.qpt == 1) seg_rest_kernel<1><<<L.n_items, L.threads, smem, s>>>(L, tb);
+    else seg_rest_kernel<2><<<L.n_items, L.threads, smem, s>>>(L, tb);
+  } else if (L.qpt == 1) {
+    if (L.cols == 1) seg_first_kernel<1, 1><<<L.n_items, L.threads, smem, s>>>(L, tb);
+    else if (L.cols == 2) seg_first_kernel<1, 2><<<L.n_items, L.threads, smem, s>>>(L, tb);
+    else return cudaErrorInvalidValue;
+  } else {
+    if (L.cols != 4) return cudaErrorInvalidValue;
+    seg_first_kernel<2, 4><<<L.n_items, L.threads, smem, s>>>(L, tb);
+  }
   return cudaGetLastError();
 }
 
