@@ -34,13 +34,13 @@ struct CircuitDev {
   const uint64_t *rec;        // [R] noise records
   const double *rec_p;        // [R]
   const uint32_t *rec_moff;   // [R + 1]
-  uint64_t *mdesc;            // [M] mechanism descriptors (written by the key kernel)
-  double *mp;                 // [M] mechanism probabilities (written by the key kernel)
-  uint32_t *tl;               // [M][tcap] targets of each mechanism, ascending (written by the key kernel)
-  uint32_t *tn;               // [M] number of targets of each mechanism
+  uint64_t *mdesc;            // [M] mechanism descriptors (global path)
+  double *mp;                 // [M] mechanism probabilities (global path)
+  uint32_t *tl;               // allocation-free merge: [M][tcap] targets of each mechanism, ascending
+  uint32_t *tn;               // allocation-free merge: [M] number of targets of each mechanism
   uint32_t nq, qpad, n_epochs, w;
   uint32_t npoints, M, R;
-  uint32_t tcap;              // stride of tl (0: no target lists, merge from snapshots)
+  uint32_t tcap;              // most targets of a listed symptom (0: no target lists, merge from snapshots)
   uint32_t n_chunks, chunk_cap;
   uint32_t mbase;             // first mechanism of this circuit in the batch-wide arrays
   uint32_t bbase, bbits;      // first bucket of this circuit, log2 of its bucket count
@@ -160,59 +160,65 @@ size_t walk_smem_bytes(uint32_t qpad, uint32_t chunk_cap, uint32_t table_bytes, 
 uint32_t walk_max_threads(uint32_t qpt);  // 0: no walk instance for this many qubits per thread
 bool walk_queue_supported(uint32_t qpt, uint32_t words);  // a persistent walk instance exists
 
-// Key kernel: one thread per noise record; expands the record into its
-// mechanisms (mdesc, mp), computes each mechanism's 128-bit key, and counts
-// non-empty keys per bucket (top `bucket_bits` bits of key.x).
-// One bucket slot (32 bytes, one sector): the mechanism's 128-bit key, then
-// (mechanism, target count, probability).  The group stage overwrites the
-// second half of a bucket's first slots with one record per group:
-// (head mechanism, targets before the group inside the bucket, probability).
+// One bucket slot (64 bytes): an item is one symptom of one noise record, with
+// the record's mechanisms that have it merged.  Its 128-bit key, then (first
+// mechanism, targets | mechanisms merged << 24, probability), then its first
+// targets: 16 16-bit ones when every circuit of the run has at most 65,536
+// detectors and observables (narrow), else 8 32-bit ones; unused ones are zero.
+// Later targets sit in the first mechanism's row of the target lists.  With
+// the targets in a row of their own, the grouping and the emission read one
+// scattered sector per item for them (32 mixed surface codes: emission 42 -> 37
+// us with them here).
+// The group stage overwrites the tail of a bucket's first slots with one record
+// per group: (head mechanism, targets before the group inside the bucket,
+// probability), and the keys with four 32-bit words: of slot s, [0] the first
+// mechanism and [3] the mechanisms merged of the item at sorted position s;
+// for s < groups, [1] the first sorted position of group s and [2] the slot of
+// its head.
 struct SlotTail {
   uint32_t m, t;
   double p;
 };
 static_assert(sizeof(SlotTail) == 16, "slot tail is 16 bytes");
-// A slot: key and tail side by side, so a mechanism's item is one 32-byte
-// sector written once and read once.  After grouping, the key half of slot s
-// holds the saved permutation as two 32-bit words: [0] the mechanism at
-// sorted position s, [1] (for s < groups) the first sorted position of group s.
-struct Slot {
+constexpr uint32_t kSlotCount = 0xFFFFFFu;  // target count in SlotTail::t (saturated)
+struct alignas(64) Slot {
   ulonglong2 key;
   SlotTail tail;
+  uint32_t list[8];
 };
-static_assert(sizeof(Slot) == 32, "a slot is one 32-byte sector");
+static_assert(sizeof(Slot) == 64, "a slot is two 32-byte sectors");
 __host__ __device__ __forceinline__ uint32_t *slot_perm(Slot *bucket, uint32_t s) {
   return reinterpret_cast<uint32_t *>(&bucket[s].key);
 }
 __host__ __device__ __forceinline__ const uint32_t *slot_perm(const Slot *bucket, uint32_t s) {
   return reinterpret_cast<const uint32_t *>(&bucket[s].key);
 }
+// Items of a bucket counter (its high half counts mechanisms; past 2^16 of
+// either the counter wraps, but the run was flagged long before).
+__device__ __forceinline__ uint32_t bucket_items(uint32_t count) { return count & 0xFFFFu; }
 
 struct KeyLaunch {
   const CircuitDev *circs;  // [n_circ]
-  const uint32_t *mbase;    // [n_circ + 1] first mechanism of each circuit (+ total)
+  const uint32_t *kbase;    // [n_circ] first key warp of each circuit
   uint32_t n_circ, M;       // circuits, mechanisms of the whole batch
-  uint2 *blk_info;          // [key blocks] (record of the block's first mechanism, its circuit | spans << 31)
-  ulonglong2 *key;          // [M]
-  uint32_t *bucket_count;   // [buckets of the batch] (zeroed)
+  uint32_t n_warps, chunk;  // key warps, of `chunk` mechanisms each: ceil(mechanisms / chunk) of each circuit
+  uint32_t *first;          // [n_warps] first record of each warp (launch_key_prep); of a circuit's first warp 0
+  uint32_t *bucket_count;   // [buckets of the batch] (zeroed) items | mechanisms << 16
   Slot *slot;               // [buckets * SLOT_CAP] bucket slots
+  uint32_t *tl;             // [M][tstride] targets past a slot's
+  uint32_t tstride, narrow;
   uint32_t *list_total;     // += targets written to the lists (for traffic accounting)
   uint32_t *err;
-  uint32_t write_all;       // also write key[], and descriptors/probabilities (global path, gradients)
-  // One circuit whose key pass is split (kNoSplit: one pass over every word):
-  // key_kernel covers the words below late_word and leaves each mechanism's
-  // descriptor, probability, targets and partial key; key_late_kernel adds
-  // the words from late_word on (the observables', whose walk is the longest)
-  // and files the mechanism in its bucket.
-  uint32_t late_word;
+  ulonglong2 *key;          // [M] global path (one circuit)
 };
-constexpr uint32_t kNoSplit = 0xFFFFFFFFu;
 constexpr uint32_t KEY_THREADS = 256;
-inline uint32_t key_blocks(uint32_t M) { return (M + KEY_THREADS - 1) / KEY_THREADS; }
-// Finds each key block's first record (one thread per block).
+uint32_t key_chunk(uint64_t mechanisms);  // mechanisms per key warp for a run of this many
+// Finds each key warp's first record (one thread per warp).
 cudaError_t launch_key_prep(const KeyLaunch &L, cudaStream_t s);
+// Bucket path: the records' symptoms keyed, listed and filed in their buckets.
 cudaError_t launch_keys(const KeyLaunch &L, cudaStream_t s);
-cudaError_t launch_keys_late(const KeyLaunch &L, cudaStream_t s);  // second pass of a split key pass
+// Global path: every mechanism's key, descriptor and probability.
+cudaError_t launch_keys_all(const KeyLaunch &L, cudaStream_t s);
 
 // Exclusive scan of the bucket counts into bucket offsets (+ total at [nb]).
 cudaError_t launch_bucket_scan(const uint32_t *count, uint32_t *offset, uint32_t nb, cudaStream_t s);
@@ -242,8 +248,8 @@ struct BucketMergeLaunch {
 cudaError_t launch_bucket_merge(const BucketMergeLaunch &L, cudaStream_t s);
 
 // Merge of the compile pipeline (no inter-CTA waits).  The key kernel has put
-// every non-empty mechanism into a slot of its bucket (SLOT_CAP slots per
-// bucket; more raises DEV_FLAG_BIG_BUCKET).
+// every item into a slot of its bucket (SLOT_CAP slots per bucket; more than
+// SLOT_CAP mechanisms raise DEV_FLAG_BIG_BUCKET).
 //  group: one warp per bucket of <= WARP_CAP items (one CTA per larger bucket)
 //         orders its items (by 64 sub-bins on the top bits of the key's second
 //         half, then by (key, m) inside a sub-bin), checks collisions, folds each group's
@@ -255,12 +261,11 @@ cudaError_t launch_bucket_merge(const BucketMergeLaunch &L, cudaStream_t s);
 //  emit:  one warp per bucket writes its groups' probabilities, offsets and
 //         target lists to the DEM arrays.
 struct GroupLaunch {
-  const uint32_t *tl;       // [M][tcap] batch-wide target lists
-  const uint32_t *tn;       // [M]
-  uint32_t tcap;
+  const uint32_t *tl;       // [M][tstride] targets past a slot's
+  uint32_t tcap, tstride, narrow;
   Slot *slot;               // [nb * SLOT_CAP] items; afterwards the saved permutation in the
-                            // key halves (slot_perm) and one group record per group in the tails
-  const uint32_t *count;    // [nb]
+                            // keys (slot_perm) and one group record per group in the tails
+  const uint32_t *count;    // [nb] (bucket_items)
   uint32_t nb;
   uint2 *bagg;              // [nb] (groups, targets) of each bucket
   uint2 *bout;              // [nb] exclusive prefix of bagg
@@ -306,10 +311,11 @@ struct AdjointLaunch {
   const uint32_t *count;
   const uint2 *bagg, *bout;
   uint32_t nb;
-  const uint2 *blk_info;   // [key blocks] record of each key block's first mechanism (the forward's key pass)
+  const uint32_t *first;   // [key warps] first record of each key warp (launch_key_prep)
+  uint32_t chunk;
   const double *rec_p;     // [R] each record's component probability of the forward (from the noise tensor)
   const double *grad_out;  // [groups] dL/dp of each merged mechanism
-  double *gq;              // [M] (zeroed) dL/dq of each mechanism
+  double *gq;              // [M] (zeroed) dL/dq summed over each item's mechanisms, at its first mechanism
   const uint64_t *rec;
   const uint32_t *rec_src, *rec_moff;
   uint32_t R;

@@ -155,10 +155,10 @@ struct WalkClass {
 // one copy each).
 struct Layout {
   std::vector<CircLayout> c;
-  size_t cdev, items, mbase, cbbase;
+  size_t cdev, items, kbase, cbbase;
   size_t in_bytes;
   size_t ext_ops;  // bytes of page-locked tape ops
-  size_t mdesc, mp, tl, tn, key, blk_r0, slot, bagg, bout, cout, big_list;
+  size_t mdesc, mp, tl, key, key_first, slot, bagg, bout, cout, big_list;
   size_t zero, err, totals, bcount, tsum, big_n, wq, zero_bytes;
   size_t sk0, sk1, pm0, pm1, hik;  // global path (single circuit)
   size_t src_off, src_rec, gq, grad_rec, ptab;  // noise-rate gradients (single circuit)
@@ -166,7 +166,7 @@ struct Layout {
   size_t out_prob, out_off;
   size_t seg_items, seg_aff, seg_state, seg_xcnt, seg_xlst;  // segmented walk (single circuit)
   size_t total;
-  uint32_t M, nb, n_items;
+  uint32_t M, nb, n_items, key_warps, key_chunk;
   uint32_t sort_tiles, merge_tiles;
   size_t sort_words;
   std::vector<WalkClass> classes;
@@ -529,7 +529,6 @@ struct gpc_driver {
   uint32_t batch_words = 0, batch_qpt = 0;  // walk configuration of batches chosen by autotune (0: defaults)
   uint32_t batch_queue = 0;                  // 1: batches walk in one persistent launch (autotune's choice)
   int walk_queue = 0;                        // option walk_queue: 1 always, -1 never, 0 batch_queue
-  bool key_split = true;                     // split key pass for one circuit when it pays (option key_split)
   int walk_segment = 0;                      // option walk_segment: 0 when it pays, -1 never, > 0 target cost
   unsigned long long spin_ns = 200ull * 1000 * 1000;  // option wait_limit_us: global-path look-back waits
   uint32_t hold_runs = 0;  // option test_hold_tile: global-path runs left whose first sort tile stays unpublished
@@ -586,7 +585,9 @@ struct gpc_driver {
   cudaGraphExec_t graph_exec = nullptr;
   bool use_graph = true;
   uint64_t cfg_sig = 0, graph_sig = 0, last_run_sig = 0;
-  uint32_t tcap = 32;      // target-list stride (grows when a symptom is longer)
+  uint32_t tcap = 32;      // most targets of a listed symptom (grows when a symptom is longer)
+  bool narrow = true;      // 16-bit targets in the bucket slots
+  uint32_t tstride = 16;   // targets per row past the slots'
   // A symptom of the prepared circuit overflowed its bucket: its later runs go to the global sort at
   // once (the bucket pass, its wait and the second key pass cost 60 us of 250 on 118k mechanisms).
   // Set by a run, forgotten with the circuit.
@@ -685,7 +686,7 @@ struct gpc_driver {
       return r;
     };
     L.c.assign(N, CircLayout{});
-    uint64_t M = 0, nb = 0, items = 0;
+    uint64_t M = 0, nb = 0, items = 0, kw = 0;
     // Bucket size, from each circuit's own mechanism count (so a circuit gets
     // the same buckets, and bit for bit the same DEM, alone and in a batch):
     // small circuits are latency-bound and want more buckets (more warps in
@@ -721,13 +722,16 @@ struct gpc_driver {
       nb += 1ull << bb;
       items += T.w;
     }
+    L.key_chunk = gpc::key_chunk(M);
+    for (const Tape &T : tapes) kw += (T.M + L.key_chunk - 1) / L.key_chunk;
+    L.key_warps = (uint32_t)kw;
     if (M >= 0xFFFFFFF0ull || nb >= 0x7FFFFFFFull) throw gpc::Error(GPC_ERR_CAPACITY, "batch too large");
     L.M = (uint32_t)M;
     L.nb = (uint32_t)nb;
     L.n_items = (uint32_t)items;
     L.cdev = take((size_t)N * sizeof(CircuitDev));
     L.items = take((size_t)items * sizeof(uint2));
-    L.mbase = take((size_t)(N + 1) * 4);
+    L.kbase = take((size_t)N * 4);
     L.cbbase = take((size_t)N * 4);
     L.seg_items = take(seg_on ? seg_items.size() * sizeof(gpc::SegItem) : 0);
     L.seg_aff = take(seg_on ? seg_aff.size() * 4 : 0);
@@ -747,12 +751,16 @@ struct gpc_driver {
       L.c[i].snap = take((size_t)tapes[i].w * tapes[i].npoints * 16);
       L.c[i].band = take((size_t)tapes[i].w * 8);
     }
-    L.mdesc = take((size_t)M * 8);
-    L.mp = take((size_t)M * 8);
-    L.tl = take((size_t)M * tcap * 4);
-    L.tn = take((size_t)M * 4);
-    L.key = take((size_t)M * 16);
-    L.blk_r0 = take((size_t)gpc::key_blocks((uint32_t)M) * 8);
+    // targets past a slot's: 16 fit one when every circuit's fit 16 bits, else 8
+    narrow = true;
+    for (const Tape &T : tapes) narrow &= T.nbits <= 65536u;
+    tstride = tcap ? tcap - (narrow ? 16u : 8u) : 0u;
+    L.tl = take((size_t)M * tstride * 4);
+    const size_t Ms = N == 1 ? M : 0;  // the global path and gradients take one circuit
+    L.mdesc = take(Ms * 8);
+    L.mp = take(Ms * 8);
+    L.key = take(Ms * 16);
+    L.key_first = take((size_t)L.key_warps * 4);
     const size_t slots = (size_t)nb * gpc::SLOT_CAP;
     L.slot = take(slots * sizeof(gpc::Slot));
     L.bagg = take((size_t)nb * 8);
@@ -897,7 +905,11 @@ struct gpc_driver {
       if (bytes) memcpy(h + off, src, bytes);
     };
     std::vector<CircuitDev> cd(N);
-    std::vector<uint32_t> mb(N + 1), cb(N);
+    std::vector<uint32_t> kb(N), cb(N);
+    for (uint32_t i = 0, kw = 0; i < N; ++i) {
+      kb[i] = kw;
+      kw += (tapes[i].M + L.key_chunk - 1) / L.key_chunk;
+    }
     // circuits fill disjoint regions of the staging buffer: a batch copies in parallel
     order_by_size(N, [&](uint32_t i) { return (uint64_t)tapes[i].ops.size() + tapes[i].rec.size(); });
     for_each(N, N >= 8, [&](uint32_t x, uint32_t) {
@@ -954,10 +966,8 @@ struct gpc_driver {
       c.rec = dptr<uint64_t>(l.rec);
       c.rec_p = dptr<double>(l.rec_p);
       c.rec_moff = dptr<uint32_t>(l.rec_moff);
-      c.mdesc = dptr<uint64_t>(L.mdesc) + l.mbase;
-      c.mp = dptr<double>(L.mp) + l.mbase;
-      c.tl = dptr<uint32_t>(L.tl) + (size_t)l.mbase * tcap;
-      c.tn = dptr<uint32_t>(L.tn) + l.mbase;
+      c.mdesc = dptr<uint64_t>(L.mdesc);
+      c.mp = dptr<double>(L.mp);
       c.tcap = tcap;
       c.nq = T.nq;
       c.qpad = T.qpad;
@@ -971,12 +981,10 @@ struct gpc_driver {
       c.mbase = l.mbase;
       c.bbase = l.bbase;
       c.bbits = l.bbits;
-      mb[i] = l.mbase;
       cb[i] = l.bbase;
     });
-    mb[N] = L.M;
     put(L.cdev, cd.data(), cd.size() * sizeof(CircuitDev));
-    put(L.mbase, mb.data(), mb.size() * 4);
+    put(L.kbase, kb.data(), kb.size() * 4);
     put(L.cbbase, cb.data(), cb.size() * 4);
     put(L.items, walk_items.data(), walk_items.size() * sizeof(uint2));
     if (seg_on) {
@@ -1133,6 +1141,9 @@ struct gpc_driver {
     mix(L.nb);
     mix(L.M);
     mix(tcap);
+    mix(narrow);
+    mix(L.key_warps);
+    mix(L.key_chunk);
     mix((uint64_t)force_global);
     mix((uint64_t)lists_off);
     mix((uint64_t)overflowed);
@@ -1148,7 +1159,6 @@ struct gpc_driver {
       mix(c.qpt);
       mix(c.queue);
     }
-    mix(split_word());
     mix((uint64_t)seg_on);
     if (seg_on) {
       mix(seg_na);
@@ -1169,7 +1179,7 @@ struct gpc_driver {
     CK(cudaSetDevice(device));
     used_global = false;
     sizes.known = false;
-    const bool single_global = ncirc() == 1 && (force_global || lists_off || overflowed);
+    const bool single_global = global_plan();
     if (ncirc() == 1 && overflowed && !force_global && !lists_off) ++fallbacks[1];
     // (a graph with the stage events is another graph)
     const uint64_t sig = cfg_sig ^ (stage_timing ? 0x9e3779b97f4a7c15ull : 0ull);
@@ -1218,24 +1228,14 @@ struct gpc_driver {
     CK(gpc::launch_walk(wl, s));
   }
 
+  // Several walk classes: each on an auxiliary stream, the key warps' first records beside them.
   void launch_walks(const gpc::KeyLaunch &kl) {
     const uint32_t nc = (uint32_t)L.classes.size();
-    auto one = [&](const WalkClass &wc, cudaStream_t s) { walk_one(wc, s); };
-    if (nc <= 1) {
-      // the key-block table on an auxiliary stream beside the walk
-      CK(cudaEventRecord(fork_ev, stream));
-      CK(cudaStreamWaitEvent(aux[0], fork_ev, 0));
-      CK(gpc::launch_key_prep(kl, aux[0]));
-      if (nc == 1) one(L.classes[0], stream);
-      CK(cudaEventRecord(join_ev[0], aux[0]));
-      CK(cudaStreamWaitEvent(stream, join_ev[0], 0));
-      return;
-    }
     // fork: each class on an auxiliary stream, joined back into the main stream
     CK(cudaEventRecord(fork_ev, stream));
     const uint32_t used = std::min<uint32_t>(nc, kAux);
     for (uint32_t a = 0; a < used; ++a) CK(cudaStreamWaitEvent(aux[a], fork_ev, 0));
-    for (uint32_t k = 0; k < nc; ++k) one(L.classes[k], aux[k % kAux]);
+    for (uint32_t k = 0; k < nc; ++k) walk_one(L.classes[k], aux[k % kAux]);
     CK(gpc::launch_key_prep(kl, stream));
     for (uint32_t a = 0; a < used; ++a) {
       CK(cudaEventRecord(join_ev[a], aux[a]));
@@ -1350,14 +1350,9 @@ struct gpc_driver {
   }
 
   // Launch A (first parts, AFF and transfer walks) then launch B (the rest
-  // of every segmented word) on the main stream; the key-block table beside
-  // them on an auxiliary stream.
-  void launch_walks_seg(const gpc::KeyLaunch &kl) {
+  // of every segmented word) on the main stream.
+  void launch_walks_seg() {
     const Tape &T = tapes[0];
-    CK(cudaEventRecord(fork_ev, stream));
-    CK(cudaStreamWaitEvent(aux[0], fork_ev, 0));
-    CK(gpc::launch_key_prep(kl, aux[0]));
-    CK(cudaEventRecord(join_ev[0], aux[0]));
     if (seg_band_reset) CK(cudaMemsetAsync(dptr<char>(L.c[0].band), 0, (size_t)T.w * 8, stream));
     gpc::SegLaunch sl{};
     sl.circ = dptr<CircuitDev>(L.cdev);
@@ -1379,93 +1374,56 @@ struct gpc_driver {
     sl.items += seg_na;
     sl.n_items = seg_nb;
     CK(gpc::launch_walk_seg(sl, true, stream));
-    CK(cudaStreamWaitEvent(stream, join_ev[0], 0));
   }
 
-  // First word of a split key pass, or kNoSplit.  One circuit with target
-  // lists whose observables sit in words after some detector-only words: the
-  // observables never vanish, so their walk covers every epoch, while the
-  // detector words stop early; their keys are computed beside that walk.
-  uint32_t split_word() const {
-    if (!key_split || seg_on || ncirc() != 1 || force_global || lists_off || overflowed || tcap == 0 || L.classes.size() != 1)
-      return gpc::kNoSplit;
-    const Tape &T = tapes[0];
-    if (T.nobs == 0 || T.n_epochs == 0) return gpc::kNoSplit;
-    const uint32_t W = std::max(1u, L.classes[0].words);
-    const uint32_t late = T.ndet / 64u / W * W;  // whole walk items before the first observable's word
-    // worth a second launch only when the detector words' keys are a real
-    // kernel and the observables' walk is long (measured: a loss for d = 5-9
-    // surface circuits, a gain for [[144,12,12]] with 27 detector words)
-    return late >= 8 && late < T.w && T.n_epochs >= 64 ? late : gpc::kNoSplit;
-  }
-
-  // The walks of a split key pass: the detector words on the main stream, the
-  // late words (from `late`) and the key-block table on auxiliary streams; the
-  // end of the late walk is timing event 1 and join_ev[1].
-  void launch_walks_split(const gpc::KeyLaunch &kl, uint32_t late) {
-    const WalkClass &wc = L.classes[0];
-    WalkClass a = wc, b = wc;
-    a.n_items = late / std::max(1u, wc.words);
-    b.item0 = wc.item0 + a.n_items;
-    b.n_items = wc.n_items - a.n_items;
-    CK(cudaEventRecord(fork_ev, stream));
-    CK(cudaStreamWaitEvent(aux[0], fork_ev, 0));
-    CK(cudaStreamWaitEvent(aux[1], fork_ev, 0));
-    CK(gpc::launch_key_prep(kl, aux[0]));
-    CK(cudaEventRecord(join_ev[0], aux[0]));
-    walk_one(b, aux[1]);
-    if (stage_timing) {
-      if (capturing) CK(cudaEventRecordWithFlags(ev[1], aux[1], cudaEventRecordExternal));
-      else CK(cudaEventRecord(ev[1], aux[1]));
-    }
-    CK(cudaEventRecord(join_ev[1], aux[1]));
-    walk_one(a, stream);
-    CK(cudaStreamWaitEvent(stream, join_ev[0], 0));
-  }
-
-  gpc::KeyLaunch key_launch(bool write_all) {
+  gpc::KeyLaunch key_launch() {
     gpc::KeyLaunch kl{};
     kl.circs = dptr<CircuitDev>(L.cdev);
-    kl.mbase = dptr<uint32_t>(L.mbase);
+    kl.kbase = dptr<uint32_t>(L.kbase);
     kl.n_circ = ncirc();
     kl.M = L.M;
-    kl.key = dptr<ulonglong2>(L.key);
+    kl.n_warps = L.key_warps;
+    kl.chunk = L.key_chunk;
+    kl.first = dptr<uint32_t>(L.key_first);
     kl.bucket_count = dptr<uint32_t>(L.bcount);
-    kl.blk_info = dptr<uint2>(L.blk_r0);
     kl.slot = dptr<gpc::Slot>(L.slot);
+    kl.tl = dptr<uint32_t>(L.tl);
+    kl.tstride = tstride;
+    kl.narrow = narrow ? 1u : 0u;
     kl.list_total = dptr<uint32_t>(L.totals) + 2;
     kl.err = dptr<uint32_t>(L.err);
-    kl.write_all = write_all ? 1u : 0u;
-    kl.late_word = gpc::kNoSplit;
+    kl.key = dptr<ulonglong2>(L.key);
     return kl;
   }
+
+  // The circuit merges through the global sort (one circuit).
+  bool global_plan() const { return ncirc() == 1 && (force_global || lists_off || overflowed); }
 
   void enqueue() {
     CK(cudaMemsetAsync(dptr<char>(L.zero), 0, L.zero_bytes, stream));
     for (uint32_t i = 0; i < ncirc(); ++i)
       if (tapes[i].n_epochs == 0) CK(cudaMemsetAsync(dptr<char>(L.c[i].band), 0, (size_t)tapes[i].w * 8, stream));
-    gpc::KeyLaunch kl = key_launch(param || (ncirc() == 1 && (force_global || lists_off || overflowed)));
-    const uint32_t late = split_word();
+    const gpc::KeyLaunch kl = key_launch();
     rec(0);
-    if (seg_on) {
-      launch_walks_seg(kl);
-      rec(1);
-      CK(gpc::launch_keys(kl, stream));
-    } else if (late == gpc::kNoSplit) {
-      launch_walks(kl);
-      rec(1);
-      CK(gpc::launch_keys(kl, stream));
+    if (L.classes.size() <= 1) {  // the key warps' first records, found beside the walk
+      CK(cudaEventRecord(fork_ev, stream));
+      CK(cudaStreamWaitEvent(aux[0], fork_ev, 0));
+      CK(gpc::launch_key_prep(kl, aux[0]));
+      CK(cudaEventRecord(join_ev[0], aux[0]));
+      if (seg_on) launch_walks_seg();
+      else if (L.classes.size() == 1) walk_one(L.classes[0], stream);
+      CK(cudaStreamWaitEvent(stream, join_ev[0], 0));
     } else {
-      launch_walks_split(kl, late);
-      kl.late_word = late;
-      CK(gpc::launch_keys(kl, stream));  // the detector words, beside the late walk
-      CK(cudaStreamWaitEvent(stream, join_ev[1], 0));
-      CK(gpc::launch_keys_late(kl, stream));
+      launch_walks(kl);
     }
-    rec(2);
-    if (ncirc() == 1 && (force_global || lists_off || overflowed)) {
+    rec(1);
+    if (global_plan()) {
+      CK(gpc::launch_keys_all(kl, stream));
+      rec(2);
       run_global(SortKey::Auto);
     } else {
+      CK(gpc::launch_keys(kl, stream));
+      rec(2);
       CK(gpc::launch_group(group_launch(), stream));
       rec(3);
       CK(gpc::launch_scan_emit(group_launch(), stream));
@@ -1476,8 +1434,9 @@ struct gpc_driver {
   gpc::GroupLaunch group_launch() {
     gpc::GroupLaunch gl{};
     gl.tl = dptr<uint32_t>(L.tl);
-    gl.tn = dptr<uint32_t>(L.tn);
     gl.tcap = tcap;
+    gl.tstride = tstride;
+    gl.narrow = narrow ? 1u : 0u;
     gl.slot = dptr<gpc::Slot>(L.slot);
     gl.count = dptr<uint32_t>(L.bcount);
     gl.nb = L.nb;
@@ -1650,8 +1609,7 @@ struct gpc_driver {
         // a symptom repeated more often than a bucket holds: sort globally
         // (the bucket pass skipped the keys and descriptors this path reads)
         CK(cudaMemsetAsync(dptr<char>(L.err), 0, 4, stream));
-        CK(gpc::launch_keys(key_launch(true), stream));
-        CK(cudaMemsetAsync(dptr<char>(L.err), 0, 4, stream));
+        CK(gpc::launch_keys_all(key_launch(), stream));
         run_global(SortKey::Auto);
         continue;
       }
@@ -1812,7 +1770,8 @@ struct gpc_driver {
     A.bagg = dptr<uint2>(L.bagg);
     A.bout = dptr<uint2>(L.bout);
     A.nb = L.nb;
-    A.blk_info = dptr<uint2>(L.blk_r0);
+    A.first = dptr<uint32_t>(L.key_first);
+    A.chunk = L.key_chunk;
     A.rec_p = dptr<double>(L.c[0].rec_p);
     A.grad_out = grad_out;
     A.gq = dptr<double>(L.gq);
@@ -1863,17 +1822,19 @@ struct gpc_driver {
       }
       R += (double)T.rec.size();
     }
-    const double M = L.M, lists = tot[2], groups = tot[0], targets = tot[1], nb = L.nb;
-    const double per_list = M > 0 ? lists / M : 0.0;
+    const double M = L.M, groups = tot[0], targets = tot[1], nb = L.nb;
     out[0] = walk;
-    // records, snapshot words read, count (+ key, descriptor, probability when kept), lists, bucket slots
-    const bool all = param || (ncirc() == 1 && (force_global || lists_off || overflowed));
-    out[1] = R * 20 + 16.0 * pts + M * (all ? 36 : 4) + 4.0 * lists + (double)nonempty * 32;
-    // slots read, lists compared for the non-head items, group records written, counts and aggregates
-    out[2] = (double)nonempty * 32 + (double)(nonempty - std::min<double>(nonempty, groups)) * 8.0 * per_list +
-             groups * 16 + nb * 12;
-    // aggregates and prefixes, group records, head lists gathered and written, DEM probabilities and offsets
-    out[3] = nb * 24 + groups * (16 + 4) + 8.0 * targets + groups * 12;
+    if (global_plan()) {
+      // records, snapshot words read, key, descriptor and probability written
+      out[1] = R * 20 + 16.0 * pts + M * 32;
+    } else {
+      // records, snapshot words read, bucket slots written, targets past the slots' (at most all)
+      out[1] = R * 20 + 16.0 * pts + (double)nonempty * 64;
+    }
+    // slots read, group records and the permutation written, counts and aggregates
+    out[2] = (double)nonempty * (64 + 16) + groups * 16 + nb * 12;
+    // aggregates and prefixes, group records and head lists read, targets, DEM probabilities and offsets
+    out[3] = nb * 24 + groups * (32 + 32) + 4.0 * targets + groups * 12;
   }
 
   // A fetch whose copies are issued and whose DEMs are not built yet, with
@@ -2188,7 +2149,6 @@ struct gpc_driver {
       d->walk_qpt = walk_qpt;
       d->bucket_mean = bucket_mean;
       d->walk_words = walk_words;
-      d->key_split = key_split;
       d->batch_words = batch_words;
       d->batch_qpt = batch_qpt;
       d->batch_queue = batch_queue;
@@ -2578,7 +2538,6 @@ gpc_status gpc_get_driver(const char *stim_text, size_t len, int32_t correlation
     if (options->walk_words < 0 || options->walk_words > 2) return fail(GPC_ERR_INVALID, "walk_words must be 0, 1 or 2");
     d->walk_words = (uint32_t)options->walk_words;
     if (options->key_split != 0 && options->key_split != -1) return fail(GPC_ERR_INVALID, "key_split must be 0 or -1");
-    d->key_split = options->key_split == 0;
     if (options->walk_queue < -1 || options->walk_queue > 1) return fail(GPC_ERR_INVALID, "walk_queue must be -1, 0 or 1");
     d->walk_queue = options->walk_queue;
     if (options->walk_segment < -1) return fail(GPC_ERR_INVALID, "walk_segment must be -1, 0 or positive");

@@ -5,26 +5,27 @@
 // + a 64-bit FNV hash with no collision check, CUB radix sort, a gather of
 // probabilities, CUB reduce-by-key and a gather of the full class matrix.
 //
-//  * key_kernel: one thread per noise record.  It expands the record into
-//    its mechanisms (the Pauli components of the channel), computes each
-//    mechanism's symptom words from the walk's snapshots -- word j is the
-//    XOR of the selected rows of its one or two points, zero outside word
-//    j's band -- and folds them into a 128-bit key K = XOR_j H(j, word_j)
-//    with H(j, 0) = 0, so the empty symptom has key 0.  Non-empty keys are
-//    counted per bucket (the top bits of K: one MSD radix digit).
-//  * bucket scan + scatter: the radix partition pass.
-//  * bucket_merge_kernel: one CTA per bucket sorts its items in shared memory
-//    by (K, mechanism), so a group (run of equal K) keeps ascending mechanism
-//    order; every item checks its full symptom against its predecessor
-//    (collision check); group heads fold their run's probabilities left to
-//    right with p <- p(1-q) + q(1-p) (CUDAHandlers.hpp:124-139) in FP64,
-//    extract their targets and get an output slot from a block scan plus a
-//    warp-wide decoupled look-back over the preceding buckets.  The empty
-//    symptom is dropped (Driver.hpp:185).
-//  * global path, used when a bucket exceeds one CTA (a symptom repeated
-//    more than BUCKET_CAP times): LSD onesweep radix sort of all keys (one
+//  * key_items_kernel: a warp takes a run of noise records.  Each record's
+//    mechanisms (the Pauli components of its channel) are the XORs of the
+//    snapshot rows of its one or two points; the components of one symptom
+//    become one item, with a 128-bit key K = XOR_j H(j, word_j) over the
+//    symptom's words (H(j, 0) = 0, so the empty symptom has key 0) and its
+//    target list, filed in a slot of its bucket (the top bits of K).
+//  * group_warp_kernel, group_big_kernel: order a bucket's items by key, check
+//    every item's full target list against its run's (collision check) and
+//    fold the run's probabilities with p <- p(1-q) + q(1-p)
+//    (CUDAHandlers.hpp:124-139) in FP64; group_scan_kernel and emit_kernel
+//    write the groups to the DEM arrays.  The empty symptom is dropped
+//    (Driver.hpp:185).
+//  * bucket scan + scatter, bucket_merge_kernel: the allocation-free merge of
+//    raw mechanisms (static_merge.cu): one CTA per bucket sorts its items in
+//    shared memory and gets its output slot from a warp-wide decoupled
+//    look-back over the preceding buckets.
+//  * global path, used when a bucket overflows (more than SLOT_CAP mechanisms):
+//    key_all_kernel keys every mechanism on its own; LSD onesweep radix sort of all keys (one
 //    kernel per 8-bit digit, tile ranks by warp match/popc, decoupled
 //    look-back for digit offsets) and a merge kernel over the sorted run.
+#include <algorithm>
 #include <cstdint>
 
 #include "device.cuh"
@@ -93,75 +94,504 @@ __constant__ uint8_t kComp[6][15] = {
 };
 #undef PP
 
-// Thread per key block: the record holding the block's first mechanism, the
-// block's circuit, and whether the block spans more than one circuit.
-__global__ void key_prep_kernel(KeyLaunch L) {
-  const uint32_t blk = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t m0 = blk * KEY_THREADS;
-  if (m0 >= L.M) return;
-  const uint32_t c = find_circuit(L.mbase, L.n_circ, m0);
-  const uint32_t c1 = find_circuit(L.mbase, L.n_circ, min(L.M - 1, m0 + KEY_THREADS - 1));
-  const CircuitDev &C = L.circs[c];
-  const uint32_t m = m0 - L.mbase[c];
-  uint32_t lo = 0, hi = C.R;
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (__ldg(C.rec_moff + mid) <= m) lo = mid;
-    else hi = mid;
+// a(1-b) + b(1-a), written as a + b(1-2a): two fused multiply-adds.
+__device__ __forceinline__ double xor_merge(double a, double b) { return fma(b, fma(-2.0, a, 1.0), a); }
+
+// find_circuit by a warp: 32 places per round of loads.
+__device__ __forceinline__ uint32_t find_circuit_warp(const uint32_t *base, uint32_t n, uint32_t x) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t lo = 0, len = n;
+  while (len > 1) {
+    const uint32_t step = (len + 31u) / 32u, at = lane * step;
+    const uint32_t le = __ballot_sync(0xFFFFFFFFu, at < len && __ldg(base + lo + at) <= x);
+    const uint32_t k = (31u - __clz(le)) * step;
+    lo += k;
+    len = min(step, len - k);
   }
-  L.blk_info[blk] = make_uint2(lo, c | (c1 != c ? 0x80000000u : 0u));
+  return lo;
 }
 
-// One thread per mechanism (global numbering over the batch).  Writes the
-// mechanism's descriptor, probability, 128-bit key, target list, and its item
-// into a slot of its bucket.  The symptom's words are the words set in the
-// non-zero masks of the mechanism's points (ascending); a block inside one
-// circuit finds its mechanisms' records in shared memory.
-__global__ void __launch_bounds__(KEY_THREADS, 5) key_kernel(KeyLaunch L) {
-  __shared__ uint32_t srm[KEY_THREADS + 1];  // rec_moff of the block's records
-  __shared__ uint8_t sown[KEY_THREADS];      // record (from r0) of each of the block's mechanisms
-  __shared__ uint32_t stg[8][KEY_THREADS];   // each thread's first eight targets ([slot][thread]: no bank conflicts)
-  const uint32_t tid = threadIdx.x, lane = tid & 31u;
-  const uint32_t m0 = blockIdx.x * KEY_THREADS;
-  const uint32_t mg = m0 + tid;
-  const uint2 info = L.blk_info[blockIdx.x];
-  const uint32_t r0 = info.x, c0 = info.y & 0x7FFFFFFFu;
-  const bool one = (info.y >> 31) == 0;
-  // every record holds at least one mechanism, so the block's records are r0 .. r0 + KEY_THREADS - 1
-  const uint32_t nr = one ? min(KEY_THREADS, L.circs[c0].R - r0) : 0;
-  if (one) {
-    for (uint32_t k = tid; k <= nr; k += KEY_THREADS) srm[k] = __ldg(L.circs[c0].rec_moff + r0 + k);
-    __syncthreads();
-    // each record marks its mechanisms inside the block (at most 15), so a
-    // mechanism finds its record with one shared load instead of a search
-    const uint32_t mb0 = m0 - __ldg(L.mbase + c0);  // the block's first mechanism within its circuit
-    for (uint32_t k = tid; k < nr; k += KEY_THREADS) {
-      const uint32_t a = max(srm[k], mb0), b = min(srm[k + 1], mb0 + KEY_THREADS);
-      for (uint32_t j = a; j < b; ++j) sown[j - mb0] = (uint8_t)k;
-    }
-  }
-  __syncthreads();
-  if (mg >= L.M) return;
+// ---- keys of the bucket path ---------------------------------------------------
+//
+// Bound by instructions (863 a warp of 32 mechanisms when a thread followed
+// one mechanism: its words, two 64-bit mixes per word, its targets), so the
+// work is done once per distinct thing instead of once per mechanism.  A
+// record's mechanisms are the XORs of the (X, Z) rows of its one or two points,
+// selected by s = Pauli a | Pauli b << 2, so over the words a record touches
+// (entries) each entry holds the span of four rows: 1 or 3 distinct non-zero
+// values for 97% of the entries of the code circuits, 3, 7 or 15 distinct
+// symptoms for a two-qubit channel's 15 components.  A warp takes the records
+// that start among L.chunk mechanisms:
+//   records  (a lane each)  masks of the non-zero words, one entry per set word;
+//   entries  (a lane each)  rows, their coordinates in a basis of their span
+//                           (lut: nibble s is the coordinate of value s; equal
+//                           coordinates, equal values), the distinct values, the
+//                           targets of the union and each row as a bit mask of them;
+//   values   (a lane each)  the 128-bit hash of (word, value);
+//   records                 the selections whose symptom vanishes (a subgroup: the
+//                           nibbles that are zero in every entry), one item per
+//                           coset, with as many of the channel's components
+//                           as lie in it (a coset's components share the symptom
+//                           and the probability, so they are merged here);
+//   items    (a lane each)  key = XOR of the values' hashes, targets, a slot.
+// Warps never wait for one another.  Measured on 32 mixed surface codes (4.0M
+// mechanisms): 863 -> ~590 instructions per 32 mechanisms, 212 -> 126 us, and
+// a third fewer items for the grouping (203 -> 153 us, 10 -> 2 for the buckets
+// of more than a warp's items); surface d = 25 60 -> 46 us, [[144,12,12]] (one
+// wave of warps, bound by a warp's latency) 15.8 -> 17.5 and its grouping 18.7
+// -> 13.2.  Kept out: 48 registers for a fifth block an SM (spills: 152 us), and
+// a copy of the launch's parameters on the stack (151 us).
+constexpr uint32_t kKeyWarps = 8;
+constexpr uint32_t kKeyEntries = 64;   // entries a warp holds at once
+constexpr uint32_t kKeyValues = 128;   // distinct values
+constexpr uint32_t kKeyTargets = 160;  // targets of the records' unions (up to 32 a record)
+constexpr uint32_t kKeyItems = 256;
 
-  const uint32_t c = one ? c0 : find_circuit(L.mbase, L.n_circ, mg);
-  const CircuitDev &C = L.circs[c];
-  const uint32_t m = mg - __ldg(L.mbase + c);
-  uint32_t r;
-  if (one) {
-    r = r0 + sown[tid];
-  } else {
-    uint32_t lo = 0, hi = C.R;
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (__ldg(C.rec_moff + mid) <= m) lo = mid;
-      else hi = mid;
-    }
-    r = lo;
+// Components present (bit s) and their place in the component list, by record type (kComp).
+__constant__ uint16_t kPresent[6] = {0, 0x0006, 0x000E, 0x0536, 0x177E, 0xFFFE};
+// (nibble s is the place of component s)
+__constant__ uint64_t kPlace[6] = {0, 0x100, 0x1200, 0x50100300420, 0x1095208406730, 0x9D51AE628C407B30};
+
+struct KeyWarp {
+  ulonglong2 h[kKeyValues];  // (value, word), then its hash
+  uint64_t lut[kKeyEntries];
+  uint4 rows[32];            // Xa, Za, Xb, Zb of each record over its targets
+  double p[32];
+  uint32_t ent[kKeyEntries]; // word | record << 18 | point a set << 26 | point b set << 27
+  uint32_t targets[kKeyTargets];
+  uint32_t pa[32], pb[32], moff[32];
+  uint16_t hb[kKeyEntries];  // first value of each entry
+  uint16_t tstart[32], vstart[32];  // first target and first value of each record
+  uint16_t join[32];         // selections that join components of one symptom (bit s)
+  uint16_t item[kKeyItems];  // record << 4 | s
+  uint64_t place[32];        // kPlace of the record's type
+  uint16_t present[32];      // the record's components (bit s)
+  uint8_t e0[32], e1[32];
+};
+
+// Probability that an odd number of `c` independent events of probability q happens.
+__device__ __forceinline__ double repeat_merge(double q, uint32_t c) {
+  double p = q;
+  uint32_t k = 1;
+  for (; 2 * k <= c; k *= 2) p = xor_merge(p, p);
+  for (; k < c; ++k) p = xor_merge(p, q);
+  return p;
+}
+
+// m with its bits permuted by s -> s ^ k.
+__device__ __forceinline__ uint32_t xor_bits16(uint32_t m, uint32_t k) {
+  if (k & 1u) m = ((m >> 1) & 0x5555u) | ((m & 0x5555u) << 1);
+  if (k & 2u) m = ((m >> 2) & 0x3333u) | ((m & 0x3333u) << 2);
+  if (k & 4u) m = ((m >> 4) & 0x0F0Fu) | ((m & 0x0F0Fu) << 4);
+  if (k & 8u) m = ((m >> 8) & 0x00FFu) | ((m & 0x00FFu) << 8);
+  return m;
+}
+
+// A record's subgroup of selections without a symptom, as far as it can join two of its components.
+__device__ __forceinline__ uint32_t joining(uint32_t type, uint32_t zero) {
+  return type >= REC_DEP2_L0 ? zero : type == REC_PAULI ? 0x1u : zero & 0xFu;
+}
+
+// One component of every coset with a symptom: the one with the smallest s.
+__device__ __forceinline__ uint32_t coset_heads(uint32_t present, uint32_t zero, uint32_t join) {
+  uint32_t heads = present & ~zero;
+  for (uint32_t ks = join & ~1u; ks; ks &= ks - 1) {
+    const uint32_t k = __ffs(ks) - 1u;
+    const uint32_t top = 31u - __clz(k);  // s ^ k < s where s has k's top bit
+    const uint32_t larger = top == 0 ? 0xAAAAu : top == 1 ? 0xCCCCu : top == 2 ? 0xF0F0u : 0xFF00u;
+    heads &= ~(xor_bits16(present, k) & larger);
   }
+  return heads;
+}
+
+// Files an item in its bucket: one 64-byte slot as two 32-byte stores.  The
+// bucket's counter counts items in its low half and mechanisms in its high
+// half: a bucket overflows by its mechanisms, whatever is merged beforehand.
+__device__ __forceinline__ void file_item(const KeyLaunch &L, uint32_t bbase, uint32_t bbits, uint32_t tcap, uint64_t hx,
+                                          uint64_t hy, uint32_t m, uint32_t cnt, uint32_t mult, double p,
+                                          const uint32_t (&l)[8]) {
+  if ((hx | hy) == 0) {  // a non-empty symptom hashed to 0
+    atomicOr(L.err, DEV_ERR_COLLISION);
+    return;
+  }
+  if (cnt > tcap) atomicOr(L.err, DEV_FLAG_LONG);
+  const uint32_t b = bbase + (uint32_t)(hx >> (64u - bbits));
+  const uint32_t old = atomicAdd(L.bucket_count + b, 1u | (mult << 16));
+  const uint32_t slot = old & 0xFFFFu;
+  if ((old >> 16) + mult > SLOT_CAP) atomicOr(L.err, DEV_FLAG_BIG_BUCKET);
+  if (slot >= SLOT_CAP) return;
+  Slot *s = L.slot + (size_t)b * SLOT_CAP + slot;
+  asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(s), "l"(hx), "l"(hy),
+               "l"((uint64_t)m | (uint64_t)(min(cnt, kSlotCount) | (mult << 24)) << 32), "l"(__double_as_longlong(p)));
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(&s->list[0]), "r"(l[0]), "r"(l[1]),
+               "r"(l[2]), "r"(l[3]), "r"(l[4]), "r"(l[5]), "r"(l[6]), "r"(l[7]));
+}
+
+// One record that holds more words, values or targets than the warp's arrays:
+// lane s follows selection s through the record's words, first to find the
+// selections without a symptom, then for the items' keys and targets.
+__device__ __noinline__ uint32_t key_record_direct(const KeyLaunch &L, const CircuitDev &C, uint32_t r, uint32_t *stage) {
+  const uint32_t lane = threadIdx.x & 31u;
   const uint64_t d = __ldg(C.rec + r);
-  const uint32_t ci = m - (one ? srm[r - r0] : __ldg(C.rec_moff + r));
+  const uint32_t pa = (uint32_t)(d & 0x0FFFFFFFu), pb = (uint32_t)((d >> 28) & 0x0FFFFFFFu);
   const uint32_t type = (uint32_t)((d >> 56) & 15u);
-  const uint32_t comp = type == 0 ? (uint32_t)((d >> 60) & 3u) | ((uint32_t)(d >> 62) << 2) : kComp[type][ci];
+  const uint32_t present = type == REC_PAULI ? 1u << ((uint32_t)(d >> 60) & 15u) : kPresent[type];
+  const bool has_a = (present & 0xEEEEu) != 0, has_b = (present & 0xFFF0u) != 0;
+  const uint32_t np = C.npoints, mw = C.mw, s = lane & 15u, inl = L.narrow ? 16u : 8u, tcap = C.tcap;
+  const unsigned long long *ma = C.nzm + (size_t)pa * mw, *mb = C.nzm + (size_t)pb * mw;
+  auto for_words = [&](auto &&f) {
+    for (uint32_t i = 0; i < mw; ++i) {
+      const uint64_t ba = has_a ? __ldg(ma + i) : 0ull, bb = has_b ? __ldg(mb + i) : 0ull;
+      for (uint64_t bits = ba | bb; bits; bits &= bits - 1) {
+        const uint32_t bit = (uint32_t)(__ffsll((long long)bits) - 1), j = i * 64u + bit;
+        const ulonglong2 *sj = C.snap + (size_t)j * np;
+        uint64_t v = 0;
+        if ((ba >> bit) & 1ull) v = pauli_sel(sj[pa], s & 3u);
+        if ((bb >> bit) & 1ull) v ^= pauli_sel(sj[pb], s >> 2);
+        if (v) f(j, v);
+      }
+    }
+  };
+  uint64_t any = 0;
+  for_words([&](uint32_t, uint64_t v) { any |= v; });
+  const uint32_t zero = __ballot_sync(0xFFFFFFFFu, any == 0) & 0xFFFFu;
+  const uint32_t join = joining(type, zero), heads = coset_heads(present, zero, join);
+  const bool item = lane < 16u && ((heads >> s) & 1u);
+  const uint32_t m = C.mbase + __ldg(C.rec_moff + r) + (uint32_t)(kPlace[type] >> (4u * s) & 15u);
+  uint64_t hx = 0, hy = 0;
+  uint32_t cnt = 0;
+  uint32_t *mine = stage + lane * 8u;  // 32 bytes: the item's first targets
+  if (item) {
+    uint32_t *far = L.tl + (size_t)m * L.tstride;
+    for (uint32_t i = 0; i < 8; ++i) mine[i] = 0;
+    for_words([&](uint32_t j, uint64_t v) {
+      const ulonglong2 h = word_hash(j, v);
+      hx ^= h.x;
+      hy ^= h.y;
+      for (uint64_t x = v; x; x &= x - 1, ++cnt) {
+        const uint32_t t = j * 64u + (uint32_t)(__ffsll((long long)x) - 1);
+        if (cnt >= inl) {
+          if (cnt < tcap) far[cnt - inl] = t;
+        } else if (L.narrow) {
+          reinterpret_cast<uint16_t *>(mine)[cnt] = (uint16_t)t;
+        } else {
+          mine[cnt] = t;
+        }
+      }
+    });
+    uint32_t l[8];
+    for (uint32_t i = 0; i < 8; ++i) l[i] = mine[i];
+    const uint32_t mult = (uint32_t)__popc(xor_bits16(join, s) & present);
+    file_item(L, C.bbase, C.bbits, C.tcap, hx, hy, m, cnt, mult, repeat_merge(__ldg(C.rec_p + r), mult), l);
+  }
+  return cnt;
+}
+
+__global__ void __launch_bounds__(kKeyWarps * 32, 4) key_items_kernel(const __grid_constant__ KeyLaunch L) {
+  __shared__ KeyWarp s_warp[kKeyWarps];
+  const uint32_t lane = threadIdx.x & 31u;
+  KeyWarp &S = s_warp[threadIdx.x >> 5];
+  const uint32_t w = blockIdx.x * kKeyWarps + (threadIdx.x >> 5);
+  if (w >= L.n_warps) return;
+  const uint32_t c = L.n_circ == 1 ? 0u : find_circuit_warp(L.kbase, L.n_circ, w);
+  const CircuitDev &C = L.circs[c];
+  const uint32_t r_end = w + 1 < L.n_warps ? L.first[w + 1] : 0u;  // (0: the last warp of its circuit)
+  const uint32_t mw = C.mw, np = C.npoints, bbase = C.bbase, bbits = C.bbits, tcap = C.tcap;
+  const ulonglong2 *const snap = C.snap;
+  constexpr uint32_t ALL = 0xFFFFFFFFu;
+  uint32_t listed = 0;  // targets written by this lane's items
+  // the records from r0 on, as many at a time as fit the warp's arrays
+  for (uint32_t r0 = L.first[w], r1 = r_end ? r_end : C.R; r0 < r1;) {
+    const uint32_t nrec = min(r1 - r0, 32u);
+    uint64_t d = 0;
+    uint32_t words = 0, present = 0;
+    bool has_a = false, has_b = false;
+    const unsigned long long *ma = C.nzm, *mb = C.nzm;
+    __syncwarp();
+    if (lane < nrec) {
+      d = __ldg(C.rec + r0 + lane);
+      const uint32_t pa = (uint32_t)(d & 0x0FFFFFFFu), pb = (uint32_t)((d >> 28) & 0x0FFFFFFFu);
+      const uint32_t type = (uint32_t)((d >> 56) & 15u);
+      S.p[lane] = __ldg(C.rec_p + r0 + lane);
+      S.moff[lane] = C.mbase + __ldg(C.rec_moff + r0 + lane);
+      S.pa[lane] = pa;
+      S.pb[lane] = pb;
+      S.place[lane] = kPlace[type];
+      S.rows[lane] = make_uint4(0, 0, 0, 0);
+      present = type == REC_PAULI ? 1u << ((uint32_t)(d >> 60) & 15u) : kPresent[type];
+      S.present[lane] = (uint16_t)present;
+      has_a = (present & 0xEEEEu) != 0;
+      has_b = (present & 0xFFF0u) != 0;
+      ma += (size_t)pa * mw;
+      mb += (size_t)pb * mw;
+      for (uint32_t i = 0; i < mw; ++i)
+        words += (uint32_t)__popcll((has_a ? __ldg(ma + i) : 0ull) | (has_b ? __ldg(mb + i) : 0ull));
+    }
+    // the next records whose words fit the entries
+    uint32_t inc = words;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(ALL, inc, o);
+      if (lane >= (uint32_t)o) inc += x;
+    }
+    uint32_t take = (uint32_t)__popc(__ballot_sync(ALL, lane < nrec && inc <= kKeyEntries));
+    uint32_t over = take;  // first record that does not fit the arrays below
+    const uint32_t E = take ? __shfl_sync(ALL, inc, take - 1u) : 0u;
+    if (lane < take) {
+      uint32_t at = inc - words;
+      S.e0[lane] = (uint8_t)at;
+      S.e1[lane] = (uint8_t)inc;
+      for (uint32_t i = 0; i < mw; ++i) {
+        const uint64_t ba = has_a ? __ldg(ma + i) : 0ull, bb = has_b ? __ldg(mb + i) : 0ull;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const uint32_t wa = (uint32_t)(ba >> (32 * half)), wb = (uint32_t)(bb >> (32 * half));
+          for (uint32_t bits = wa | wb; bits; bits &= bits - 1) {
+            const uint32_t low = bits & (0u - bits);
+            S.ent[at++] = (i * 64u + 32u * half + (uint32_t)(31 - __clz(low))) | (lane << 18) |
+                          (wa & low ? 1u << 26 : 0u) | (wb & low ? 1u << 27 : 0u);
+          }
+        }
+      }
+    }
+    __syncwarp();
+    uint32_t H = 0, TG = 0;  // values and targets of the entries so far
+    for (uint32_t x0 = 0; x0 < E; x0 += 32) {
+      const uint32_t x = x0 + lane;
+      const bool in = x < E;
+      const uint32_t en = in ? S.ent[x] : 0u, j = en & 0x3FFFFu, k = (en >> 18) & 255u;
+      const ulonglong2 *sj = snap + (size_t)j * np;
+      ulonglong2 ra = make_ulonglong2(0, 0), rb = ra;
+      if ((en >> 26) & 1u) ra = sj[S.pa[k]];  // (a point's snapshot of word j exists only where its bit is set)
+      if ((en >> 27) & 1u) rb = sj[S.pb[k]];
+      // coordinates c0..c3 of the rows in a basis b0..b3 of their span (n of them, in order of appearance)
+      const uint64_t v0 = ra.x, v1 = ra.y, v2 = rb.x, v3 = rb.y;
+      uint32_t span = 1, c0 = 0, c1 = 0, c2 = 0, c3 = 0;  // span: 2^n
+      auto fresh = [&]() -> uint32_t {
+        span *= 2;
+        return span / 2;
+      };
+      if (v0) c0 = fresh();
+      if (v1) c1 = v1 == v0 ? c0 : fresh();
+      if (v2) c2 = v2 == v0 ? c0 : v2 == v1 ? c1 : v2 == (v0 ^ v1) ? c0 ^ c1 : fresh();
+      if (v3) {
+        const uint64_t y = v3 ^ v2;
+        c3 = v3 == v0 ? c0 : v3 == v1 ? c1 : v3 == (v0 ^ v1) ? c0 ^ c1 : y == 0 ? c2 : y == v0 ? c2 ^ c0
+             : y == v1 ? c2 ^ c1 : y == (v0 ^ v1) ? c2 ^ c0 ^ c1 : fresh();
+      }
+      const uint32_t nv = span - 1u;
+      const uint64_t u = v0 | v1 | v2 | v3;
+      const uint32_t nt = (uint32_t)__popcll(u);
+      uint32_t both = nv << 16 | nt;  // inclusive scan of (values, targets)
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(ALL, both, o);
+        if (lane >= (uint32_t)o) both += y;
+      }
+      const uint32_t iv = both >> 16, it = both & 0xFFFFu;
+      const uint32_t hb = H + iv - nv, tb = TG + it - nt;
+      if (in && x == S.e0[k]) {
+        S.tstart[k] = (uint16_t)min(tb, 0xFFFFu);
+        S.vstart[k] = (uint16_t)min(hb, 0xFFFFu);
+      }
+      __syncwarp();
+      if (in) {
+        const uint32_t off = tb - S.tstart[k];
+        if (hb + nv > kKeyValues || off + nt > 32u || tb + nt > kKeyTargets) {
+          over = min(over, k);
+        } else {
+          uint64_t lut = (uint64_t)c0 << 4;
+          lut |= (lut ^ (c1 * 0x11u)) << 8;
+          lut |= (lut ^ (c2 * 0x1111u)) << 16;
+          lut |= (lut ^ (c3 * 0x11111111ull)) << 32;
+          S.lut[x] = lut;
+          S.hb[x] = (uint16_t)hb;
+          if (nv) {
+            const uint64_t b0 = v0 ? v0 : v1 ? v1 : v2 ? v2 : v3;
+            S.h[hb] = make_ulonglong2(b0, j);
+            if (nv > 1) {
+              const uint64_t b1 = c1 == 2u ? v1 : c2 == 2u ? v2 : v3;
+              S.h[hb + 1] = make_ulonglong2(b1, j);
+              S.h[hb + 2] = make_ulonglong2(b0 ^ b1, j);
+              if (nv > 3) {
+                const uint64_t b2 = c2 == 4u ? v2 : v3;
+                for (uint32_t y = 4; y <= nv; ++y) {
+                  const uint64_t v = (y & 1u ? b0 : 0ull) ^ (y & 2u ? b1 : 0ull) ^ (y & 4u ? b2 : 0ull) ^ (y & 8u ? v3 : 0ull);
+                  S.h[hb + y - 1u] = make_ulonglong2(v, j);
+                }
+              }
+            }
+          }
+          uint32_t m0 = 0, m1 = 0, m2 = 0, m3 = 0;
+          uint32_t at = 1u << off;
+          uint32_t *tg = S.targets + tb;
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            const uint32_t w0 = (uint32_t)(v0 >> (32 * half)), w1 = (uint32_t)(v1 >> (32 * half)),
+                           w2 = (uint32_t)(v2 >> (32 * half)), w3 = (uint32_t)(v3 >> (32 * half));
+            for (uint32_t bits = (uint32_t)(u >> (32 * half)); bits; bits &= bits - 1, at <<= 1) {
+              const uint32_t low = bits & (0u - bits);
+              *tg++ = j * 64u + (uint32_t)(31 - __clz(low)) + 32u * half;
+              if (w0 & low) m0 |= at;
+              if (w1 & low) m1 |= at;
+              if (w2 & low) m2 |= at;
+              if (w3 & low) m3 |= at;
+            }
+          }
+          if (m0) atomicOr(&S.rows[k].x, m0);
+          if (m1) atomicOr(&S.rows[k].y, m1);
+          if (m2) atomicOr(&S.rows[k].z, m2);
+          if (m3) atomicOr(&S.rows[k].w, m3);
+        }
+      }
+      H += __shfl_sync(ALL, iv, 31);
+      TG += __shfl_sync(ALL, it, 31);
+    }
+    over = __reduce_min_sync(ALL, over);
+    if (over == 0) {  // a record that does not fit alone
+      listed += key_record_direct(L, C, r0, reinterpret_cast<uint32_t *>(S.h));
+      ++r0;
+      continue;
+    }
+    if (over < take) {  // only the records before it (theirs is all in place)
+      take = over;
+      H = S.vstart[over];
+    }
+    __syncwarp();
+    for (uint32_t y = lane; y < H; y += 32) {
+      const ulonglong2 v = S.h[y];
+      S.h[y] = word_hash((uint32_t)v.y, v.x);
+    }
+    // the items of each record
+    uint32_t heads = 0;
+    if (lane < take) {
+      uint64_t z = 0;
+      for (uint32_t x = S.e0[lane]; x < S.e1[lane]; ++x) z |= S.lut[x];
+      z |= z >> 1;  // zero nibbles, gathered into 16 bits
+      z |= z >> 2;
+      z = ~z & 0x1111111111111111ull;
+      z = (z | z >> 3) & 0x0303030303030303ull;
+      z = (z | z >> 6) & 0x000F000F000F000Full;
+      z = (z | z >> 12) & 0x000000FF000000FFull;
+      const uint32_t zero = (uint32_t)(z | z >> 24) & 0xFFFFu;
+      const uint32_t join = joining((uint32_t)(d >> 56) & 15u, zero);
+      heads = coset_heads(present, zero, join);
+      S.join[lane] = (uint16_t)join;
+    }
+    uint32_t at = (uint32_t)__popc(heads);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(ALL, at, o);
+      if (lane >= (uint32_t)o) at += x;
+    }
+    take = (uint32_t)__popc(__ballot_sync(ALL, lane < take && at <= kKeyItems));
+    const uint32_t items = __shfl_sync(ALL, at, take - 1u);
+    at -= (uint32_t)__popc(heads);
+    if (lane >= take) heads = 0;
+    for (; heads; heads &= heads - 1) S.item[at++] = (uint16_t)(lane << 4 | (__ffs(heads) - 1u));
+    __syncwarp();
+    for (uint32_t q0 = 0; q0 < items; q0 += 32) {
+      const uint32_t q = q0 + lane;
+      const bool in = q < items;
+      const uint32_t it = in ? S.item[q] : 0u, k = it >> 4, s = it & 15u;
+      uint64_t hx = 0, hy = 0;
+      if (in) {
+        // (s's half of the 16 nibbles)
+        const uint32_t *lut = reinterpret_cast<const uint32_t *>(S.lut) + (s >> 3), sh = 4u * (s & 7u);
+        for (uint32_t x = S.e0[k], x1 = S.e1[k]; x < x1; ++x) {
+          const uint32_t id = (lut[2 * x] >> sh) & 15u;
+          if (id) {
+            const ulonglong2 h = S.h[S.hb[x] + id - 1u];
+            hx ^= h.x;
+            hy ^= h.y;
+          }
+        }
+      }
+      const uint4 rows = S.rows[k];
+      uint32_t t = in ? (s & 1u ? rows.x : 0u) ^ (s & 2u ? rows.y : 0u) ^ (s & 4u ? rows.z : 0u) ^ (s & 8u ? rows.w : 0u) : 0u;
+      const uint32_t cnt = (uint32_t)__popc(t);
+      const uint32_t *tg = S.targets + S.tstart[k];
+      uint32_t l[8] = {};
+      if (L.narrow) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          if (i % 4 == 0 && !__any_sync(ALL, t != 0)) break;
+          if (t) {
+            l[i / 2] |= tg[__ffs(t) - 1] << (i % 2 * 16);
+            t &= t - 1;
+          }
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (i % 4 == 0 && !__any_sync(ALL, t != 0)) break;
+          if (t) {
+            l[i] = tg[__ffs(t) - 1];
+            t &= t - 1;
+          }
+        }
+      }
+      if (!in) continue;
+      const uint32_t m = S.moff[k] + (uint32_t)(S.place[k] >> (4u * s) & 15u);
+      if (t) {  // the rest of a long list
+        uint32_t *far = L.tl + (size_t)m * L.tstride;
+        for (uint32_t i = 0; t; t &= t - 1, ++i)
+          if (i < L.tstride) far[i] = tg[__ffs(t) - 1];
+      }
+      const uint32_t mult = (uint32_t)__popc(xor_bits16(S.join[k], s) & S.present[k]);
+      listed += cnt;
+      file_item(L, bbase, bbits, tcap, hx, hy, m, cnt, mult, repeat_merge(S.p[k], mult), l);
+    }
+    r0 += take;
+  }
+  const uint32_t tot = __reduce_add_sync(ALL, listed);
+  if (lane == 0 && tot) red_add(L.list_total, tot);
+}
+
+
+// ---- records of mechanisms (global path, gradients; one circuit) --------------
+
+// Thread per key warp: its first record, the first that starts at or after the warp's first mechanism.
+__global__ void key_prep_kernel(KeyLaunch L) {
+  const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
+  if (w >= L.n_warps) return;
+  const uint32_t c = find_circuit(L.kbase, L.n_circ, w);
+  const CircuitDev &C = L.circs[c];
+  const uint32_t m = (w - L.kbase[c]) * L.chunk;
+  uint32_t lo = 0, hi = C.R;  // rec_moff[lo - 1] < m <= rec_moff[hi]
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (__ldg(C.rec_moff + mid) < m) lo = mid + 1;
+    else hi = mid;
+  }
+  L.first[w] = lo;
+}
+
+// Record of mechanism m (one circuit): a search of rec_moff from the record
+// before the first of m's key warp on (each record holds a mechanism at least,
+// so m's record lies within the warp's mechanisms of it).
+__device__ __forceinline__ uint32_t record_of(const uint32_t *first, uint32_t chunk, const uint32_t *rec_moff, uint32_t R,
+                                              uint32_t m) {
+  const uint32_t f = first[m / chunk];
+  uint32_t lo = f ? f - 1u : 0u;
+  uint32_t hi = min(R, lo + chunk + 2u);
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (__ldg(rec_moff + mid) <= m) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// Global path: every mechanism's descriptor, probability and 128-bit key, a thread each.
+__global__ void __launch_bounds__(KEY_THREADS) key_all_kernel(KeyLaunch L) {
+  const uint32_t m = blockIdx.x * KEY_THREADS + threadIdx.x;
+  if (m >= L.M) return;
+  const CircuitDev &C = L.circs[0];
+  const uint32_t r = record_of(L.first, L.chunk, C.rec_moff, C.R, m);
+  const uint64_t d = __ldg(C.rec + r);
+  const uint32_t type = (uint32_t)((d >> 56) & 15u);
+  const uint32_t comp = type == 0 ? (uint32_t)(d >> 60) & 15u : kComp[type][m - __ldg(C.rec_moff + r)];
   uint32_t pa = (uint32_t)(d & 0x0FFFFFFFu), pb = (uint32_t)((d >> 28) & 0x0FFFFFFFu);
   uint32_t Pa = comp & 3u, Pb = comp >> 2;
   if (Pa == 0) {  // a component on point b only is stored with b as its first point
@@ -170,39 +600,19 @@ __global__ void __launch_bounds__(KEY_THREADS, 5) key_kernel(KeyLaunch L) {
     Pb = 0;
   }
   if (Pb == 0) pb = 0;
-  const double prob = __ldg(C.rec_p + r);
-  const bool split = L.late_word != kNoSplit;
-  if (L.write_all || split) {  // descriptors and probabilities: global merge path, gradients, second pass
-    C.mdesc[m] = mk_desc(pa, Pa, pb, Pb);
-    C.mp[m] = prob;
-  }
-
-  const uint32_t tcap = C.tcap;
+  C.mdesc[m] = mk_desc(pa, Pa, pb, Pb);
+  C.mp[m] = __ldg(C.rec_p + r);
   uint64_t hx = 0, hy = 0;
-  uint32_t cnt = 0;
   bool nonzero = false;
-  uint32_t *out = C.tl + (size_t)m * tcap;
-  // the first eight targets are staged in shared memory and leave as two
-  // 16-byte stores (a row per thread: one scattered store per target would
-  // cost an L2 transaction each); later ones are stored as they come
-  auto put = [&](uint32_t c, uint32_t v) {
-    if (c < 8) stg[c][tid] = v;
-    else if (c < tcap) out[c] = v;
-  };
-  const ulonglong2 *snap = C.snap;
   const uint32_t np = C.npoints, mw = C.mw;
   const unsigned long long *ma = C.nzm + (size_t)pa * mw, *mb = C.nzm + (size_t)pb * mw;
-  const uint32_t jend = split ? L.late_word : mw * 64u;  // words of this pass: j < jend
-  for (uint32_t i = 0; i < mw && i * 64u < jend; ++i) {
+  for (uint32_t i = 0; i < mw; ++i) {
     // a point's snapshot of word j exists only where its own bit is set
     const uint64_t ba = __ldg(ma + i), bb = Pb ? __ldg(mb + i) : 0ull;
-    uint64_t bits = ba | bb;
-    if (jend - i * 64u < 64u) bits &= (1ull << (jend - i * 64u)) - 1ull;
-    while (bits) {
+    for (uint64_t bits = ba | bb; bits; bits &= bits - 1) {
       const uint32_t bit = (uint32_t)(__ffsll((long long)bits) - 1);
       const uint32_t j = i * 64u + bit;
-      bits &= bits - 1;
-      const ulonglong2 *sj = snap + (size_t)j * np;
+      const ulonglong2 *sj = C.snap + (size_t)j * np;
       uint64_t v = 0;
       if ((ba >> bit) & 1ull) v = pauli_sel(sj[pa], Pa);
       if ((bb >> bit) & 1ull) v ^= pauli_sel(sj[pb], Pb);
@@ -211,108 +621,10 @@ __global__ void __launch_bounds__(KEY_THREADS, 5) key_kernel(KeyLaunch L) {
       const ulonglong2 h = word_hash(j, v);
       hx ^= h.x;
       hy ^= h.y;
-      if (tcap) {
-        uint64_t x = v;
-        while (x) {
-          put(cnt, j * 64u + (uint32_t)(__ffsll((long long)x) - 1));
-          ++cnt;
-          x &= x - 1;
-        }
-      }
     }
   }
-  const ulonglong2 key = make_ulonglong2(hx, hy);
-  if (L.write_all || split) L.key[mg] = key;  // a split pass leaves the partial key
-  if (tcap) {
-    // rows are 16-byte aligned (tcap is a multiple of 4, at least 32)
-    // (both halves even for four targets or fewer: a whole 32-byte sector per row; entries past
-    // the count are never read)
-    if (cnt) {
-      reinterpret_cast<uint4 *>(out)[0] = make_uint4(stg[0][tid], stg[1][tid], stg[2][tid], stg[3][tid]);
-      reinterpret_cast<uint4 *>(out)[1] = make_uint4(stg[4][tid], stg[5][tid], stg[6][tid], stg[7][tid]);
-    }
-    C.tn[m] = cnt;
-    if (cnt > tcap) atomicOr(L.err, DEV_FLAG_LONG);
-    const uint32_t am = __activemask();
-    const uint32_t tot = __reduce_add_sync(am, cnt);
-    if (lane == (uint32_t)(__ffs(am) - 1) && tot) red_add(L.list_total, tot);
-  }
-  if (split) return;  // filed in its bucket by the second pass
-  if ((hx | hy) == 0) {
-    if (cnt || (!tcap && nonzero)) atomicOr(L.err, DEV_ERR_COLLISION);  // a non-empty symptom hashed to 0
-  } else {
-    const uint32_t b = C.bbase + (uint32_t)(hx >> (64u - C.bbits));
-    const uint32_t slot = atomicAdd(L.bucket_count + b, 1u);
-    if (slot < SLOT_CAP) {
-      const size_t pos = (size_t)b * SLOT_CAP + slot;
-      L.slot[pos] = Slot{key, SlotTail{mg, cnt, prob}};
-    } else {
-      atomicOr(L.err, DEV_FLAG_BIG_BUCKET);
-    }
-  }
-}
-
-// Second pass of a split key pass (one circuit, target lists on): adds the
-// words from late_word on to each mechanism's partial key, appends their
-// targets after the first pass's (they are the larger indices, so the list
-// stays ascending), and files the mechanism in its bucket.
-__global__ void __launch_bounds__(KEY_THREADS) key_late_kernel(KeyLaunch L) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t m = blockIdx.x * KEY_THREADS + threadIdx.x;
-  if (m >= L.M) return;
-  const CircuitDev &C = L.circs[0];
-  const uint64_t d = C.mdesc[m];
-  const uint32_t pa = (uint32_t)(d & 0x3FFFFFFFu), Pa = (uint32_t)((d >> 30) & 3u);
-  const uint32_t pb = (uint32_t)((d >> 32) & 0x3FFFFFFFu), Pb = (uint32_t)(d >> 62);
-  const double prob = C.mp[m];
-  ulonglong2 key = L.key[m];
-  const uint32_t tcap = C.tcap;
-  uint32_t *out = C.tl + (size_t)m * tcap;
-  const uint32_t cnt1 = C.tn[m];
-  uint32_t cnt = cnt1;
-  const ulonglong2 *snap = C.snap;
-  const uint32_t np = C.npoints, mw = C.mw, jbeg = L.late_word;
-  const unsigned long long *ma = C.nzm + (size_t)pa * mw, *mb = C.nzm + (size_t)pb * mw;
-  for (uint32_t i = jbeg / 64u; i < mw; ++i) {
-    const uint64_t ba = __ldg(ma + i), bb = Pb ? __ldg(mb + i) : 0ull;
-    uint64_t bits = ba | bb;
-    if (jbeg > i * 64u) bits &= ~((1ull << (jbeg - i * 64u)) - 1ull);
-    while (bits) {
-      const uint32_t bit = (uint32_t)(__ffsll((long long)bits) - 1);
-      const uint32_t j = i * 64u + bit;
-      bits &= bits - 1;
-      const ulonglong2 *sj = snap + (size_t)j * np;
-      uint64_t v = 0;
-      if ((ba >> bit) & 1ull) v = pauli_sel(sj[pa], Pa);
-      if ((bb >> bit) & 1ull) v ^= pauli_sel(sj[pb], Pb);
-      if (!v) continue;
-      const ulonglong2 h = word_hash(j, v);
-      key.x ^= h.x;
-      key.y ^= h.y;
-      for (uint64_t x = v; x; x &= x - 1) {
-        if (cnt < tcap) out[cnt] = j * 64u + (uint32_t)(__ffsll((long long)x) - 1);
-        ++cnt;
-      }
-    }
-  }
-  if (L.write_all) L.key[m] = key;
-  if (cnt != cnt1) C.tn[m] = cnt;
-  if (cnt > tcap) atomicOr(L.err, DEV_FLAG_LONG);
-  const uint32_t am = __activemask();
-  const uint32_t tot = __reduce_add_sync(am, cnt - cnt1);
-  if (lane == (uint32_t)(__ffs(am) - 1) && tot) red_add(L.list_total, tot);
-  if ((key.x | key.y) == 0) {
-    if (cnt) atomicOr(L.err, DEV_ERR_COLLISION);  // a non-empty symptom hashed to 0
-  } else {
-    const uint32_t b = C.bbase + (uint32_t)(key.x >> (64u - C.bbits));
-    const uint32_t slot = atomicAdd(L.bucket_count + b, 1u);
-    if (slot < SLOT_CAP) {
-      const size_t pos = (size_t)b * SLOT_CAP + slot;
-      L.slot[pos] = Slot{key, SlotTail{m, cnt, prob}};
-    } else {
-      atomicOr(L.err, DEV_FLAG_BIG_BUCKET);
-    }
-  }
+  L.key[m] = make_ulonglong2(hx, hy);
+  if (nonzero && (hx | hy) == 0) atomicOr(L.err, DEV_ERR_COLLISION);  // a non-empty symptom hashed to 0
 }
 
 // Exclusive scan of nb bucket counts (one block); offset[nb] = total.
@@ -573,9 +885,6 @@ __device__ __forceinline__ void warp_lookback(unsigned long long *status, uint32
   *pre_c = ec;
   *pre_t = et;
 }
-
-// a(1-b) + b(1-a), written as a + b(1-2a): two fused multiply-adds.
-__device__ __forceinline__ double xor_merge(double a, double b) { return fma(b, fma(-2.0, a, 1.0), a); }
 
 // Mask word i of the words where mechanism d's symptom can be non-zero: the
 // union of its points' non-zero masks (a word whose mask bit is clear has a
@@ -957,6 +1266,19 @@ constexpr uint32_t GW_WARPS = 8;  // buckets per group/emit block (one warp each
 
 __device__ __forceinline__ bool key_eq(ulonglong2 a, ulonglong2 b) { return a.x == b.x && a.y == b.y; }
 
+// The targets of two items: the slots' first ones as two 16-byte words (unused
+// entries are zero), the rest of longer lists from their rows.
+__device__ __forceinline__ bool slot_lists_equal(const GroupLaunch &L, const Slot *a, uint32_t ma, const Slot *b,
+                                                 uint32_t mb, uint32_t n) {
+  const uint4 *va = reinterpret_cast<const uint4 *>(a->list), *vb = reinterpret_cast<const uint4 *>(b->list);
+  const uint4 x0 = va[0], y0 = vb[0], x1 = va[1], y1 = vb[1];
+  if ((x0.x ^ y0.x) | (x0.y ^ y0.y) | (x0.z ^ y0.z) | (x0.w ^ y0.w) | (x1.x ^ y1.x) | (x1.y ^ y1.y) | (x1.z ^ y1.z) |
+      (x1.w ^ y1.w))
+    return false;
+  const uint32_t inl = L.narrow ? 16u : 8u;
+  return n <= inl || lists_equal(L.tl + (size_t)ma * L.tstride, L.tl + (size_t)mb * L.tstride, n - inl);
+}
+
 // One warp per bucket of at most WARP_CAP items; larger buckets are listed
 // for group_big_kernel.  Items are ordered by sub-bin (top 6 bits of the
 // key's second half), then by (key, m) inside the sub-bin: equal keys end up
@@ -974,15 +1296,14 @@ __global__ void __launch_bounds__(GW_WARPS * 32) group_warp_kernel(GroupLaunch L
   const uint32_t lane = threadIdx.x & 31u, wi = threadIdx.x >> 5;
   const uint32_t b = blockIdx.x * GW_WARPS + wi;
   if (b >= L.nb) return;
-  const uint32_t n = L.count[b];
+  const uint32_t n = bucket_items(L.count[b]);
   if (n == 0) {
     if (lane == 0) L.bagg[b] = make_uint2(0, 0);
     return;
   }
   if (n > WARP_CAP) {
     if (lane == 0) {
-      if (n > SLOT_CAP) {
-        atomicOr(L.err, DEV_FLAG_BIG_BUCKET);  // slots overflowed; the run is redone another way
+      if (n > SLOT_CAP) {  // (overflowed: flagged by the key pass, the run is redone another way)
         L.bagg[b] = make_uint2(0, 0);
       } else {
         L.big_list[atomicAdd(L.big_n, 1u)] = b;
@@ -999,9 +1320,8 @@ __global__ void __launch_bounds__(GW_WARPS * 32) group_warp_kernel(GroupLaunch L
   H[lane + 32] = 0;
   __syncwarp();
   for (uint32_t i = lane; i < n; i += 32) {
-    const Slot sl = L.slot[base + i];
-    const ulonglong2 k = sl.key;
-    const SlotTail t = sl.tail;
+    const ulonglong2 k = L.slot[base + i].key;
+    const SlotTail t = L.slot[base + i].tail;
     K[i] = k;
     Mm[i] = t.m;
     T[i] = t.t;
@@ -1041,7 +1361,10 @@ __global__ void __launch_bounds__(GW_WARPS * 32) group_warp_kernel(GroupLaunch L
   // the saved permutation for the adjoint: mechanism at each sorted position
   // (every key of this bucket is in shared memory already)
   Slot *const bslot = L.slot + base;
-  for (uint32_t s = lane; s < n; s += 32) slot_perm(bslot, s)[0] = Mm[O[s]];
+  for (uint32_t s = lane; s < n; s += 32) {
+    slot_perm(bslot, s)[0] = Mm[O[s]];
+    slot_perm(bslot, s)[3] = T[O[s]] >> 24;  // the mechanisms merged into the item
+  }
   // Groups, 32 sorted positions at a time.  Each group's probability is a
   // segmented inclusive scan of the XOR-merge over its run: log2(longest run
   // in the chunk) shuffle steps with every lane busy (FP64 throughput is
@@ -1059,7 +1382,7 @@ __global__ void __launch_bounds__(GW_WARPS * 32) group_warp_kernel(GroupLaunch L
     uint32_t i = 0, nt = 0;
     if (in) {
       i = O[s];
-      nt = T[i];
+      nt = T[i] & kSlotCount;
       head = s == 0 || !key_eq(K[O[s - 1]], K[i]);
     }
     const uint32_t hb = __ballot_sync(0xFFFFFFFFu, head);
@@ -1070,7 +1393,7 @@ __global__ void __launch_bounds__(GW_WARPS * 32) group_warp_kernel(GroupLaunch L
       // (a list longer than the stride holds only its first tcap targets; the
       // key pass flagged it and the run is redone with wider lists)
       if (in && !head && nt <= tcap &&
-          (T[ih] != nt || !lists_equal(L.tl + (size_t)Mm[i] * tcap, L.tl + (size_t)Mm[ih] * tcap, nt)))
+          ((T[ih] & kSlotCount) != nt || !slot_lists_equal(L, bslot + i, Mm[i], bslot + ih, Mm[ih], nt)))
         atomicOr(L.err, DEV_ERR_COLLISION);
       carry_head = __shfl_sync(0xFFFFFFFFu, ih, 31);
     }
@@ -1099,6 +1422,7 @@ __global__ void __launch_bounds__(GW_WARPS * 32) group_warp_kernel(GroupLaunch L
       bslot[gh].tail.m = Mm[i];
       bslot[gh].tail.t = tcount + inc - tv;
       slot_perm(bslot, gh)[1] = s;
+      slot_perm(bslot, gh)[2] = i;
     }
     if (in && (s + 1 >= n || !key_eq(K[O[s + 1]], K[i]))) {  // the run's last item holds its value
       const uint32_t g = seg < 0 ? gcount - 1u : gcount + __popc(hb & ((1u << seg0) - 1u));
@@ -1137,14 +1461,13 @@ __global__ void __launch_bounds__(GB_THREADS) group_big_kernel(GroupLaunch L) {
   const uint32_t tcap = L.tcap;
   for (uint32_t kb = blockIdx.x; kb < nbig; kb += gridDim.x) {
     const uint32_t b = L.big_list[kb];
-    const uint32_t n = L.count[b];  // WARP_CAP < n <= SLOT_CAP
+    const uint32_t n = bucket_items(L.count[b]);  // WARP_CAP < n <= SLOT_CAP
     const size_t base = (size_t)b * SLOT_CAP;
     if (tid < NBIN) sh[tid] = 0;
     __syncthreads();
     if (tid < n) {
-      const Slot sl = L.slot[base + tid];
-      const ulonglong2 k = sl.key;
-      const SlotTail t = sl.tail;
+      const ulonglong2 k = L.slot[base + tid].key;
+      const SlotTail t = L.slot[base + tid].tail;
       sk[tid] = k;
       sm[tid] = t.m;
       st[tid] = t.t;
@@ -1188,14 +1511,15 @@ __global__ void __launch_bounds__(GB_THREADS) group_big_kernel(GroupLaunch L) {
     uint32_t i = 0, nt = 0;
     if (in) {
       i = ord[s];
-      nt = st[i];
+      nt = st[i] & kSlotCount;
       head = true;
       if (s > 0) {
         const uint32_t ip = ord[s - 1];
         if (key_eq(sk[ip], sk[i])) {
           head = false;
           // (lists longer than the stride: flagged by the key pass, redone wider)
-          if (nt <= tcap && (st[ip] != nt || !lists_equal(L.tl + (size_t)sm[i] * tcap, L.tl + (size_t)sm[ip] * tcap, nt)))
+          const Slot *const bs = L.slot + base;
+          if (nt <= tcap && ((st[ip] & kSlotCount) != nt || !slot_lists_equal(L, bs + i, sm[i], bs + ip, sm[ip], nt)))
             atomicOr(L.err, DEV_ERR_COLLISION);
         }
       }
@@ -1244,12 +1568,16 @@ __global__ void __launch_bounds__(GB_THREADS) group_big_kernel(GroupLaunch L) {
     if (seg < 0) x = xor_merge(c_carry[warp], x);
     const uint32_t gb = c_gbase[warp];
     Slot *const bslot = L.slot + base;
-    if (in) slot_perm(bslot, s)[0] = sm[i];
+    if (in) {
+      slot_perm(bslot, s)[0] = sm[i];
+      slot_perm(bslot, s)[3] = st[i] >> 24;
+    }
     if (head) {
       const uint32_t g = gb + __popc(hb & ((1u << lane) - 1u));
       bslot[g].tail.m = sm[i];
       bslot[g].tail.t = c_tbase[warp] + inc - tv;
       slot_perm(bslot, g)[1] = s;
+      slot_perm(bslot, g)[2] = i;
     }
     if (in && (s + 1 >= n || !key_eq(sk[ord[s + 1]], sk[i]))) {
       const uint32_t g = seg < 0 ? gb - 1u : gb + __popc(hb & ((1u << seg0) - 1u));
@@ -1372,24 +1700,28 @@ __global__ void __launch_bounds__(GW_WARPS * 32) emit_kernel(GroupLaunch L) {
     }
     const uint32_t slot = out.x + g;
     const uint32_t toff = out.y + t.t;
-    const uint32_t m = t.m;
     L.out_prob[slot] = t.p;
     L.out_off[slot] = toff;
     // the group's targets run to the next group's (the bucket's total after
-    // the last); a list longer than the stride was flagged by the key pass
-    // and the run is redone with wider lists, so only the stride's targets
-    // are copied here
+    // the last); a list longer than the rows was flagged by the key pass and
+    // the run is redone with wider rows, so only the rows' targets are copied
     const uint32_t ntg = min((g + 1 < agg.x ? tn1.t : agg.y) - t.t, tcap);
     if ((uint64_t)toff + ntg <= L.tg_cap) {
-      const uint4 *src = reinterpret_cast<const uint4 *>(L.tl + (size_t)m * tcap);
-      for (uint32_t k = 0; k * 4 < ntg; ++k) {
-        const uint4 x = __ldg(src + k);
-        const uint32_t o = toff + k * 4, rem = ntg - k * 4;
-        L.out_tg[o] = x.x;
-        if (rem > 1) L.out_tg[o + 1] = x.y;
-        if (rem > 2) L.out_tg[o + 2] = x.z;
-        if (rem > 3) L.out_tg[o + 3] = x.w;
+      const uint4 *src = reinterpret_cast<const uint4 *>(L.slot[base + slot_perm(L.slot + base, g)[2]].list);
+      const uint4 x0 = src[0], x1 = src[1];
+      const uint32_t l[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+      uint32_t *out = L.out_tg + toff;
+      if (L.narrow) {
+#pragma unroll
+        for (uint32_t k = 0; k < 16; ++k)
+          if (k < ntg) out[k] = (l[k / 2] >> (k % 2 * 16)) & 0xFFFFu;
+      } else {
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k)
+          if (k < ntg) out[k] = l[k];
       }
+      const uint32_t inl = L.narrow ? 16u : 8u;
+      for (uint32_t k = inl; k < ntg; ++k) out[k] = __ldg(L.tl + (size_t)t.m * L.tstride + k - inl);
     }
   }
 }
@@ -1409,47 +1741,40 @@ __global__ void param_rec_kernel(ParamLaunch L) {
   L.rec_p[r] = L.qtab[(size_t)src * 3 + channel_kind((uint32_t)((L.rec[r] >> 56) & 15u))];
 }
 
-// Record of mechanism m (one circuit): a search of rec_moff between the
-// record of m's key block's first mechanism and KEY_THREADS + 15 records
-// after it (each record holds 1 to 15 mechanisms, so m's record lies there).
-__device__ __forceinline__ uint32_t record_of(const AdjointLaunch &A, uint32_t m) {
-  uint32_t lo = A.blk_info[m / KEY_THREADS].x;
-  uint32_t hi = min(A.R, lo + KEY_THREADS + 15u);
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (__ldg(A.rec_moff + mid) <= m) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-
+// An item of c mechanisms of probability q counts as (1 - 2q)^c in its run's
+// product; its first mechanism's entry takes the derivative by all c of them.
 __global__ void __launch_bounds__(GW_WARPS * 32) adjoint_group_kernel(AdjointLaunch A) {
-  __shared__ double s_q[GW_WARPS][SLOT_CAP];  // probability of the mechanism at each sorted position
+  __shared__ double s_q[GW_WARPS][SLOT_CAP];  // probability of the mechanisms at each sorted position
   const uint32_t lane = threadIdx.x & 31u, wi = threadIdx.x >> 5;
   const uint32_t b = blockIdx.x * GW_WARPS + wi;
   if (b >= A.nb) return;
-  const uint32_t n = A.count[b];
+  const uint32_t n = bucket_items(A.count[b]);
   if (n == 0 || n > SLOT_CAP) return;
   const uint32_t groups = A.bagg[b].x, out0 = A.bout[b].x;
   const Slot *const bslot = A.slot + (size_t)b * SLOT_CAP;
   double *q = s_q[wi];
   // the forward's mechanism probabilities, recomputed from the records (every
   // component of a record carries the record's probability)
-  for (uint32_t s = lane; s < n; s += 32) q[s] = __ldg(A.rec_p + record_of(A, slot_perm(bslot, s)[0]));
+  for (uint32_t s = lane; s < n; s += 32)
+    q[s] = __ldg(A.rec_p + record_of(A.first, A.chunk, A.rec_moff, A.R, slot_perm(bslot, s)[0]));
   __syncwarp();
   for (uint32_t g = lane; g < groups; g += 32) {
     const uint32_t s0 = slot_perm(bslot, g)[1], s1 = g + 1 < groups ? slot_perm(bslot, g + 1)[1] : n;
     const double dl = A.grad_out[out0 + g];
     double pre = 1.0;
     for (uint32_t s = s0; s < s1; ++s) {
-      A.gq[slot_perm(bslot, s)[0]] = pre;
-      pre *= 1.0 - 2.0 * q[s];
+      const double f = 1.0 - 2.0 * q[s];
+      const uint32_t c = slot_perm(bslot, s)[3];
+      for (uint32_t k = 1; k < c; ++k) pre *= f;  // (the item's other mechanisms)
+      A.gq[slot_perm(bslot, s)[0]] = pre * (double)c;
+      pre *= f;
     }
     double suf = 1.0;
     for (uint32_t s = s1; s-- > s0;) {
       const uint32_t m = slot_perm(bslot, s)[0];
       A.gq[m] = dl * A.gq[m] * suf;
-      suf *= 1.0 - 2.0 * q[s];
+      const double f = 1.0 - 2.0 * q[s];
+      for (uint32_t k = slot_perm(bslot, s)[3]; k > 0; --k) suf *= f;
     }
   }
 }
@@ -1492,21 +1817,31 @@ cudaError_t launch_adjoint(const AdjointLaunch &A, cudaStream_t s) {
 
 cudaError_t launch_key_prep(const KeyLaunch &L, cudaStream_t s) {
   if (L.M == 0) return cudaSuccess;
-  const uint32_t nblk = key_blocks(L.M);
-  key_prep_kernel<<<(nblk + 127) / 128, 128, 0, s>>>(L);
+  key_prep_kernel<<<(L.n_warps + 127) / 128, 128, 0, s>>>(L);
   return cudaGetLastError();
+}
+
+// A warp's steps cost about as much for two two-qubit records as for eight, but
+// a small run wants them side by side: as many mechanisms a warp as make one
+// wave of warps, 16 to 128.  Measured (16 / 36 / 64 / 128 mechanisms a warp,
+// us): [[72,12,6]] at L1 (28k mechanisms) 9.7 / 12 / 17 / 29, [[144,12,12]]
+// (164k) 22 / 17.5 / 20 / 29, surface d = 25 (979k) 98 / 59 / 46 / 46, 32 mixed
+// surface codes (4.0M) 382 / 212 / 153 / 126.
+uint32_t key_chunk(uint64_t mechanisms) {
+  const uint64_t wave = 152u * 4u * kKeyWarps;
+  return (uint32_t)std::min<uint64_t>(128, std::max<uint64_t>(16, (mechanisms + wave - 1) / wave));
 }
 
 cudaError_t launch_keys(const KeyLaunch &L, cudaStream_t s) {
   if (L.M == 0) return cudaSuccess;
-  key_kernel<<<key_blocks(L.M), KEY_THREADS, 0, s>>>(L);
+  key_items_kernel<<<(L.n_warps + kKeyWarps - 1) / kKeyWarps, kKeyWarps * 32, 0, s>>>(L);
   return cudaGetLastError();
 }
 
-cudaError_t launch_keys_late(const KeyLaunch &L, cudaStream_t s) {
+cudaError_t launch_keys_all(const KeyLaunch &L, cudaStream_t s) {
   if (L.M == 0) return cudaSuccess;
-  if (L.late_word == kNoSplit || L.n_circ != 1) return cudaErrorInvalidValue;
-  key_late_kernel<<<key_blocks(L.M), KEY_THREADS, 0, s>>>(L);
+  if (L.n_circ != 1) return cudaErrorInvalidValue;
+  key_all_kernel<<<(L.M + KEY_THREADS - 1) / KEY_THREADS, KEY_THREADS, 0, s>>>(L);
   return cudaGetLastError();
 }
 

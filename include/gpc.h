@@ -63,7 +63,7 @@ typedef struct gpc_options {
   int32_t walk_qpt;    /* qubits per thread of the walk (1,2,3,4,6,8,12,16; 0 = chosen per circuit) */
   int32_t bucket_mean; /* target mechanisms per merge bucket (8..128; 0 = default) */
   int32_t walk_words;  /* detector words per walk CTA (1, 2; 0 = two in batches, one for a single circuit) */
-  int32_t key_split;   /* one circuit: key the detector words beside the observables' walk (0 = when it pays, -1 = never) */
+  int32_t key_split;   /* accepted (0 or -1) and without effect: the keys are one pass after the walk */
   int32_t walk_queue;  /* batches: 1 = one persistent walk launch (resident CTAs take (circuit, word group) items
                           from a queue, longest first), -1 = one launch per thread-count class,
                           0 = classes unless gpc_autotune chose the persistent launch */
