@@ -75,7 +75,7 @@ constexpr int MERGE_THREADS = 256;
 constexpr int BUCKET_THREADS = 128;
 constexpr int BUCKET_CAP = 1024;  // items one CTA sorts in shared memory (allocation-free merge)
 constexpr uint32_t SLOT_CAP = 256;  // slots of one bucket in the compile pipeline
-constexpr uint32_t WARP_CAP = 128;  // bucket items one warp merges; larger buckets take a CTA
+constexpr uint32_t WARP_CAP = 128;  // bucket items of a warp's own shared memory
 constexpr uint32_t SCAN_TILE = 1024;    // bucket aggregates one scan block covers
 constexpr uint32_t SCAN_THREADS = 256;  // threads of a scan block (4 aggregates each)
 
@@ -170,11 +170,11 @@ bool walk_queue_supported(uint32_t qpt, uint32_t words);  // a persistent walk i
 // scattered sector per item for them (32 mixed surface codes: emission 42 -> 37
 // us with them here).
 // The group stage overwrites the tail of a bucket's first slots with one record
-// per group: (head mechanism, targets before the group inside the bucket,
-// probability), and the keys with four 32-bit words: of slot s, [0] the first
-// mechanism and [3] the mechanisms merged of the item at sorted position s;
-// for s < groups, [1] the first sorted position of group s and [2] the slot of
-// its head.
+// per group: (head mechanism, targets before the group inside the bucket << 8 |
+// the head's slot, probability).  For gradients it also overwrites the keys with
+// 32-bit words: of slot s, [0] the first mechanism and [3] the mechanisms merged
+// of the item at sorted position s; for s < groups, [1] the first sorted
+// position of group s.
 struct SlotTail {
   uint32_t m, t;
   double p;
@@ -250,28 +250,28 @@ cudaError_t launch_bucket_merge(const BucketMergeLaunch &L, cudaStream_t s);
 // Merge of the compile pipeline (no inter-CTA waits).  The key kernel has put
 // every item into a slot of its bucket (SLOT_CAP slots per bucket; more than
 // SLOT_CAP mechanisms raise DEV_FLAG_BIG_BUCKET).
-//  group: one warp per bucket of <= WARP_CAP items (one CTA per larger bucket)
-//         orders its items (by 64 sub-bins on the top bits of the key's second
-//         half, then by (key, m) inside a sub-bin), checks collisions, folds each group's
+//  group: one warp per bucket
+//         orders its items (by the top 6 bits of the key's second half, then by
+//         key, then by mechanism), checks collisions, folds each group's
 //         probability and overwrites the bucket's first slots with one record
-//         per group (head mechanism, probability, targets before it in the
-//         bucket); bucket aggregates (groups, targets) and their per-tile sums;
+//         per group (SlotTail); bucket aggregates (groups, targets) and their
+//         per-tile sums;
 //  scan:  exclusive scan of the bucket aggregates, one block per SCAN_TILE
-//         buckets (tile sums give each block its prefix);
+//         buckets (tile sums give each block its prefix); small runs fold it
+//         into the emission;
 //  emit:  one warp per bucket writes its groups' probabilities, offsets and
 //         target lists to the DEM arrays.
 struct GroupLaunch {
   const uint32_t *tl;       // [M][tstride] targets past a slot's
   uint32_t tcap, tstride, narrow;
-  Slot *slot;               // [nb * SLOT_CAP] items; afterwards the saved permutation in the
-                            // keys (slot_perm) and one group record per group in the tails
+  Slot *slot;               // [nb * SLOT_CAP] items; afterwards one group record per group in the tails and
+                            // (keep) the saved permutation in the keys (slot_perm)
+  uint32_t keep;
   const uint32_t *count;    // [nb] (bucket_items)
   uint32_t nb;
   uint2 *bagg;              // [nb] (groups, targets) of each bucket
   uint2 *bout;              // [nb] exclusive prefix of bagg
   uint2 *tsum;              // [ceil(nb / SCAN_TILE)] (zeroed) per-tile sums of bagg
-  uint32_t *big_n;          // (zeroed) buckets with more than WARP_CAP items
-  uint32_t *big_list;       // [nb]
   double *out_prob;
   uint32_t *out_off;
   uint32_t *out_tg;

@@ -158,8 +158,8 @@ struct Layout {
   size_t cdev, items, kbase, cbbase;
   size_t in_bytes;
   size_t ext_ops;  // bytes of page-locked tape ops
-  size_t mdesc, mp, tl, key, key_first, slot, bagg, bout, cout, big_list;
-  size_t zero, err, totals, bcount, tsum, big_n, wq, zero_bytes;
+  size_t mdesc, mp, tl, key, key_first, slot, bagg, bout, cout;
+  size_t zero, err, totals, bcount, tsum, wq, zero_bytes;
   size_t sk0, sk1, pm0, pm1, hik;  // global path (single circuit)
   size_t src_off, src_rec, gq, grad_rec, ptab;  // noise-rate gradients (single circuit)
   size_t gzero, sort_scr, merge_status, merge_ctr, gzero_bytes;
@@ -765,13 +765,11 @@ struct gpc_driver {
     L.slot = take(slots * sizeof(gpc::Slot));
     L.bagg = take((size_t)nb * 8);
     L.bout = take((size_t)nb * 8);
-    L.big_list = take((size_t)nb * 4);
     // each circuit's first output slot, the flags and the totals side by side: one copy reads a run's result sizes
     L.cout = take((size_t)N * 8);
     L.zero = o;
     L.err = take(4);
     L.totals = take(16);
-    L.big_n = take(4);
     L.wq = take(4);
     L.bcount = take((size_t)nb * 4);
     L.tsum = take(((size_t)nb + gpc::SCAN_TILE - 1) / gpc::SCAN_TILE * 8);
@@ -1443,8 +1441,7 @@ struct gpc_driver {
     gl.bagg = dptr<uint2>(L.bagg);
     gl.bout = dptr<uint2>(L.bout);
     gl.tsum = dptr<uint2>(L.tsum);
-    gl.big_n = dptr<uint32_t>(L.big_n);
-    gl.big_list = dptr<uint32_t>(L.big_list);
+    gl.keep = param ? 1u : 0u;
     gl.out_prob = dptr<double>(L.out_prob);
     gl.out_off = dptr<uint32_t>(L.out_off);
     gl.out_tg = static_cast<uint32_t *>(tgbuf.p);
@@ -1831,8 +1828,8 @@ struct gpc_driver {
       // records, snapshot words read, bucket slots written, targets past the slots' (at most all)
       out[1] = R * 20 + 16.0 * pts + (double)nonempty * 64;
     }
-    // slots read, group records and the permutation written, counts and aggregates
-    out[2] = (double)nonempty * (64 + 16) + groups * 16 + nb * 12;
+    // slots read, group records written, counts and aggregates
+    out[2] = (double)nonempty * 64 + groups * 16 + nb * 12;
     // aggregates and prefixes, group records and head lists read, targets, DEM probabilities and offsets
     out[3] = nb * 24 + groups * (32 + 32) + 4.0 * targets + groups * 12;
   }

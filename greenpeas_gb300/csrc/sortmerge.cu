@@ -11,9 +11,9 @@
 //    become one item, with a 128-bit key K = XOR_j H(j, word_j) over the
 //    symptom's words (H(j, 0) = 0, so the empty symptom has key 0) and its
 //    target list, filed in a slot of its bucket (the top bits of K).
-//  * group_warp_kernel, group_big_kernel: order a bucket's items by key, check
+//  * group_kernel: orders a bucket's items by key, checks
 //    every item's full target list against its run's (collision check) and
-//    fold the run's probabilities with p <- p(1-q) + q(1-p)
+//    folds the run's probabilities with p <- p(1-q) + q(1-p)
 //    (CUDAHandlers.hpp:124-139) in FP64; group_scan_kernel and emit_kernel
 //    write the groups to the DEM arrays.  The empty symptom is dropped
 //    (Driver.hpp:185).
@@ -1263,6 +1263,7 @@ __global__ void __launch_bounds__(BUCKET_THREADS) bucket_merge_kernel(BucketMerg
 // ---- merge of the compile pipeline ---------------------------------------
 
 constexpr uint32_t GW_WARPS = 8;  // buckets per group/emit block (one warp each)
+constexpr uint32_t kFoldBuckets = 32768;  // most buckets whose places the emission finds itself
 
 __device__ __forceinline__ bool key_eq(ulonglong2 a, ulonglong2 b) { return a.x == b.x && a.y == b.y; }
 
@@ -1279,91 +1280,180 @@ __device__ __forceinline__ bool slot_lists_equal(const GroupLaunch &L, const Slo
   return n <= inl || lists_equal(L.tl + (size_t)ma * L.tstride, L.tl + (size_t)mb * L.tstride, n - inl);
 }
 
-// One warp per bucket of at most WARP_CAP items; larger buckets are listed
-// for group_big_kernel.  Items are ordered by sub-bin (top 6 bits of the
-// key's second half), then by (key, m) inside the sub-bin: equal keys end up
-// adjacent in ascending mechanism order, at O(n) work per bucket.
-__global__ void __launch_bounds__(GW_WARPS * 32) group_warp_kernel(GroupLaunch L) {
-  constexpr uint32_t NBIN = 64;
-  __shared__ ulonglong2 s_k[GW_WARPS][WARP_CAP];
-  __shared__ uint32_t s_m[GW_WARPS][WARP_CAP];
-  __shared__ double s_p[GW_WARPS][WARP_CAP];
-  __shared__ uint32_t s_t[GW_WARPS][WARP_CAP];
-  __shared__ uint8_t s_o[GW_WARPS][WARP_CAP];   // sorted position -> item
-  __shared__ uint8_t s_q[GW_WARPS][WARP_CAP];   // item -> place inside its sub-bin (arrival order)
-  __shared__ uint8_t s_x[GW_WARPS][WARP_CAP];   // items grouped by sub-bin
-  __shared__ uint32_t s_h[GW_WARPS][NBIN];      // sub-bin counts, then offsets
-  const uint32_t lane = threadIdx.x & 31u, wi = threadIdx.x >> 5;
-  const uint32_t b = blockIdx.x * GW_WARPS + wi;
-  if (b >= L.nb) return;
-  const uint32_t n = bucket_items(L.count[b]);
-  if (n == 0) {
-    if (lane == 0) L.bagg[b] = make_uint2(0, 0);
-    return;
-  }
-  if (n > WARP_CAP) {
-    if (lane == 0) {
-      if (n > SLOT_CAP) {  // (overflowed: flagged by the key pass, the run is redone another way)
-        L.bagg[b] = make_uint2(0, 0);
+// What a bucket's grouping holds in shared memory: its items as they were
+// filed, and the sorted order.
+template <uint32_t CAP>
+struct GroupItems {
+  ulonglong2 key[CAP];
+  double p[CAP];
+  uint32_t m[CAP], t[CAP];
+  uint32_t sv[CAP];  // sorted position -> 24 key bits << 8 | item
+  uint8_t ord[CAP];  // sorted position -> item
+};
+
+// Bitonic sort of 32 R words, R per lane: word r * 32 + lane is v[r].
+template <int R>
+__device__ __forceinline__ void sort_words(uint32_t (&v)[R]) {
+  const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+  for (int k = 2; k <= 32 * R; k *= 2) {
+#pragma unroll
+    for (int j = k / 2; j > 0; j /= 2) {
+      if (j >= 32) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const int q = r ^ (j / 32);
+          if (q > r) {
+            const bool up = (r * 32 & k) == 0;
+            const uint32_t lo = min(v[r], v[q]), hi = max(v[r], v[q]);
+            v[r] = up ? lo : hi;
+            v[q] = up ? hi : lo;
+          }
+        }
       } else {
-        L.big_list[atomicAdd(L.big_n, 1u)] = b;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, v[r], j);
+          const bool up = k < 32 ? (lane & k) == 0 : (r * 32 & k) == 0;
+          v[r] = ((lane & j) == 0) == up ? min(v[r], o) : max(v[r], o);
+        }
       }
     }
-    return;
   }
-  ulonglong2 *K = s_k[wi];
-  uint32_t *Mm = s_m[wi], *T = s_t[wi], *H = s_h[wi];
-  double *P = s_p[wi];
-  uint8_t *O = s_o[wi], *Q = s_q[wi], *X = s_x[wi];
-  const size_t base = (size_t)b * SLOT_CAP;
-  H[lane] = 0;
-  H[lane + 32] = 0;
-  __syncwarp();
-  for (uint32_t i = lane; i < n; i += 32) {
-    const ulonglong2 k = L.slot[base + i].key;
-    const SlotTail t = L.slot[base + i].tail;
-    K[i] = k;
-    Mm[i] = t.m;
-    T[i] = t.t;
-    P[i] = t.p;
-    Q[i] = (uint8_t)atomicAdd(H + (uint32_t)(k.y >> 58), 1u);
-  }
-  __syncwarp();
-  {  // sub-bin offsets: lane owns bins 2*lane and 2*lane + 1
-    const uint32_t c0 = H[2 * lane], c1 = H[2 * lane + 1];
-    uint32_t inc = c0 + c1;
+}
+
+// The DEM's order inside a bucket: top 6 bits of the key's second half, then the key, then the mechanism.
+template <typename G_t>
+__device__ __forceinline__ bool item_before(const G_t &G, uint32_t a, uint32_t b) {
+  const uint32_t ba = (uint32_t)(G.key[a].y >> 58), bb = (uint32_t)(G.key[b].y >> 58);
+  return ba != bb ? ba < bb : item_less(G.key[a], G.m[a], G.key[b], G.m[b]);
+}
+
+// Orders the n <= 32 R items of G: G.ord.  The words sorted are 24 bits of the
+// order's key (6 of the second half, 18 of the first after the bits that all
+// items share) above the item's index: one shuffle and one min/max a step.
+// Items of equal words are then put in mechanism order; when two different
+// keys share a word (a few in 10^6 buckets) every item's place is counted
+// from the full keys instead.
+template <int R, typename G_t>
+__device__ __forceinline__ void order_items(G_t &G, uint32_t n) {
+  const uint32_t lane = threadIdx.x & 31u;
+  constexpr uint32_t ALL = 0xFFFFFFFFu;
+  uint64_t hx[R];
+  uint32_t differ = 0;
+  const uint64_t x0 = G.key[0].x;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-      if (lane >= (uint32_t)o) inc += a;
+  for (int r = 0; r < R; ++r) {
+    const uint32_t i = r * 32 + lane;
+    hx[r] = i < n ? G.key[i].x : x0;
+    differ |= (uint32_t)((hx[r] ^ x0) >> 32);
+  }
+  differ = __reduce_or_sync(ALL, differ);
+  const uint32_t same = differ ? (uint32_t)__clz(differ) : 32u;  // leading bits all share
+  uint32_t v[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const uint32_t i = r * 32 + lane;
+    v[r] = ALL;
+    if (i < n) v[r] = (uint32_t)(G.key[i].y >> 58) << 26 | ((uint32_t)((hx[r] << same) >> 32) >> 14) << 8 | i;
+  }
+  sort_words<R>(v);
+  bool mixed = false;
+  if constexpr (R == 1) {
+    const uint32_t i = v[0] & 255u;
+    uint32_t m = 0;
+    ulonglong2 k = make_ulonglong2(0, 0);
+    if (lane < n) {
+      m = G.m[i];
+      k = G.key[i];
     }
-    const uint32_t ex = inc - c0 - c1;
+    const uint32_t word = v[0] >> 8, left = __shfl_up_sync(ALL, word, 1);
+    const uint64_t lx = __shfl_up_sync(ALL, k.x, 1), ly = __shfl_up_sync(ALL, k.y, 1);
+    const bool start = lane == 0 || left != word || lane >= n;
+    mixed = !start && (lx != k.x || ly != k.y);
+    const uint32_t starts = __ballot_sync(ALL, start);
+    const uint32_t first = 31u - __clz(starts & (ALL >> (31u - lane)));
+    const uint32_t after = lane == 31u ? 0u : starts >> (lane + 1u);
+    const uint32_t end = after ? lane + (uint32_t)__ffs(after) : 32u;  // the run is lanes [first, end)
+    const uint32_t longest = __reduce_max_sync(ALL, end - first);
+    uint32_t place = first;
+    for (uint32_t o = 1; o < longest; ++o) {
+      const uint32_t a = __shfl_up_sync(ALL, m, o), b = __shfl_down_sync(ALL, m, o);
+      place += (lane >= first + o && a < m ? 1u : 0u) + (lane + o < end && b < m ? 1u : 0u);
+    }
+    if (lane < n) G.ord[place] = (uint8_t)i;
+  } else {
+#pragma unroll
+    for (int r = 0; r < R; ++r) G.sv[r * 32 + lane] = v[r];
     __syncwarp();
-    H[2 * lane] = ex;
-    H[2 * lane + 1] = ex + c0;
-  }
-  __syncwarp();
-  for (uint32_t i = lane; i < n; i += 32) X[H[(uint32_t)(K[i].y >> 58)] + Q[i]] = (uint8_t)i;
-  __syncwarp();
-  for (uint32_t i = lane; i < n; i += 32) {
-    const ulonglong2 ki = K[i];
-    const uint32_t mi = Mm[i];
-    const uint32_t bin = (uint32_t)(ki.y >> 58);
-    const uint32_t lo = H[bin], hi = bin + 1 < NBIN ? H[bin + 1] : n;
-    uint32_t r = lo;
-    for (uint32_t j = lo; j < hi; ++j) {
-      const uint32_t x = X[j];
-      r += item_less(K[x], Mm[x], ki, mi) ? 1u : 0u;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const uint32_t s = r * 32 + lane;
+      if (s >= n) continue;
+      const uint32_t i = v[r] & 255u, mi = G.m[i];
+      // its run of equal words: the items of smaller mechanisms come before it
+      uint32_t first = s, before = 0;
+      const ulonglong2 ki = G.key[i];
+      while (first > 0) {
+        const uint32_t w = G.sv[first - 1];
+        if ((w ^ v[r]) >> 8) break;
+        mixed |= !key_eq(G.key[w & 255u], ki);
+        before += G.m[w & 255u] < mi ? 1u : 0u;
+        --first;
+      }
+      for (uint32_t q = s + 1; q < n; ++q) {
+        const uint32_t w = G.sv[q];
+        if ((w ^ v[r]) >> 8) break;
+        before += G.m[w & 255u] < mi ? 1u : 0u;
+      }
+      G.ord[first + before] = (uint8_t)i;
     }
-    O[r] = (uint8_t)i;
+  }
+  if (__any_sync(ALL, mixed)) {
+    __syncwarp();
+    for (uint32_t i = lane; i < n; i += 32) {
+      uint32_t place = 0;
+      for (uint32_t q = 0; q < n; ++q) place += item_before(G, q, i) ? 1u : 0u;
+      G.ord[place] = (uint8_t)i;
+    }
   }
   __syncwarp();
-  // the saved permutation for the adjoint: mechanism at each sorted position
-  // (every key of this bucket is in shared memory already)
-  Slot *const bslot = L.slot + base;
-  for (uint32_t s = lane; s < n; s += 32) {
-    slot_perm(bslot, s)[0] = Mm[O[s]];
-    slot_perm(bslot, s)[3] = T[O[s]] >> 24;  // the mechanisms merged into the item
+}
+
+// A group's record: (head mechanism, targets before it in the bucket << 8 | the
+// head's slot) in the tail of slot g; its probability is written beside it.
+__device__ __forceinline__ void put_group(Slot *bslot, uint32_t g, uint32_t m, uint32_t before, uint32_t head, uint32_t s,
+                                          uint32_t keep) {
+  *reinterpret_cast<uint2 *>(&bslot[g].tail) = make_uint2(m, before << 8 | head);
+  if (keep) slot_perm(bslot, g)[1] = s;
+}
+
+// One warp's bucket of n <= CAP items.  Returns (groups, targets).
+template <uint32_t CAP>
+__device__ __forceinline__ uint2 group_warp(const GroupLaunch &L, GroupItems<CAP> &G, uint32_t b, uint32_t n) {
+  const uint32_t lane = threadIdx.x & 31u;
+  Slot *const bslot = L.slot + (size_t)b * SLOT_CAP;
+  for (uint32_t i = lane; i < n; i += 32) {
+    const ulonglong2 k = bslot[i].key;
+    const SlotTail t = bslot[i].tail;
+    G.key[i] = k;
+    G.m[i] = t.m;
+    G.t[i] = t.t;
+    G.p[i] = t.p;
+  }
+  __syncwarp();
+  if constexpr (CAP > 128) {
+    order_items<CAP / 32>(G, n);
+  } else {
+    if (n <= 32) order_items<1>(G, n);
+    else if (n <= 64) order_items<2>(G, n);
+    else order_items<4>(G, n);
+  }
+  if (L.keep) {  // the saved permutation for the adjoint
+    for (uint32_t s = lane; s < n; s += 32) {
+      slot_perm(bslot, s)[0] = G.m[G.ord[s]];
+      slot_perm(bslot, s)[3] = G.t[G.ord[s]] >> 24;  // the mechanisms merged into the item
+    }
   }
   // Groups, 32 sorted positions at a time.  Each group's probability is a
   // segmented inclusive scan of the XOR-merge over its run: log2(longest run
@@ -1378,22 +1468,29 @@ __global__ void __launch_bounds__(GW_WARPS * 32) group_warp_kernel(GroupLaunch L
   for (uint32_t s0 = 0; s0 < n; s0 += 32) {
     const uint32_t s = s0 + lane;
     const bool in = s < n;
-    bool head = false;
+    bool head = false, last = false;  // of its run
     uint32_t i = 0, nt = 0;
+    double x = 0.0;
     if (in) {
-      i = O[s];
-      nt = T[i] & kSlotCount;
-      head = s == 0 || !key_eq(K[O[s - 1]], K[i]);
+      i = G.ord[s];
+      nt = G.t[i] & kSlotCount;
+      x = G.p[i];
+      const ulonglong2 k = G.key[i];
+      head = s == 0 || !key_eq(G.key[G.ord[s - 1]], k);
+      last = s + 1 >= n || !key_eq(G.key[G.ord[s + 1]], k);
     }
     const uint32_t hb = __ballot_sync(0xFFFFFFFFu, head);
+    // the run of each position: it starts at lane `seg` of this chunk, or
+    // (seg < 0) continues the run open at the end of the previous chunk
+    const uint32_t le = hb & (0xFFFFFFFFu >> (31u - lane));
+    const int seg = le ? 31 - __clz(le) : -1;
+    const uint32_t seg0 = seg < 0 ? 0u : (uint32_t)seg;
     {
       // collision check: every item of a run against the run's head (full target lists)
-      const uint32_t le0 = hb & (0xFFFFFFFFu >> (31u - lane));
-      const uint32_t ih = le0 ? (uint32_t)O[s0 + 31 - __clz(le0)] : carry_head;
-      // (a list longer than the stride holds only its first tcap targets; the
-      // key pass flagged it and the run is redone with wider lists)
+      const uint32_t ih = seg < 0 ? carry_head : (uint32_t)G.ord[s0 + seg0];
+      // (a list longer than the rows was flagged by the key pass and the run is redone with wider rows)
       if (in && !head && nt <= tcap &&
-          ((T[ih] & kSlotCount) != nt || !slot_lists_equal(L, bslot + i, Mm[i], bslot + ih, Mm[ih], nt)))
+          ((G.t[ih] & kSlotCount) != nt || !slot_lists_equal(L, bslot + i, G.m[i], bslot + ih, G.m[ih], nt)))
         atomicOr(L.err, DEV_ERR_COLLISION);
       carry_head = __shfl_sync(0xFFFFFFFFu, ih, 31);
     }
@@ -1404,27 +1501,15 @@ __global__ void __launch_bounds__(GW_WARPS * 32) group_warp_kernel(GroupLaunch L
       const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, inc, o);
       if (lane >= (uint32_t)o) inc += a;
     }
-    // the run of each position: it starts at lane `seg` of this chunk, or
-    // (seg < 0) continues the run open at the end of the previous chunk
-    const uint32_t le = hb & (0xFFFFFFFFu >> (31u - lane));
-    const int seg = le ? 31 - __clz(le) : -1;
-    const uint32_t seg0 = seg < 0 ? 0u : (uint32_t)seg;
-    double x = in ? P[i] : 0.0;
     const uint32_t maxlen = __reduce_max_sync(0xFFFFFFFFu, in ? lane - seg0 + 1 : 0u);
     for (uint32_t d = 1; d < maxlen; d <<= 1) {
       const double y = __shfl_up_sync(0xFFFFFFFFu, x, d);
       if (lane >= d && lane - d >= seg0) x = xor_merge(y, x);
     }
     if (seg < 0) x = xor_merge(carry, x);
-    const uint32_t gh = gcount + __popc(hb & ((1u << lane) - 1u));  // group of a head at this lane
-    // every slot of this bucket was read into shared memory above
-    if (head) {
-      bslot[gh].tail.m = Mm[i];
-      bslot[gh].tail.t = tcount + inc - tv;
-      slot_perm(bslot, gh)[1] = s;
-      slot_perm(bslot, gh)[2] = i;
-    }
-    if (in && (s + 1 >= n || !key_eq(K[O[s + 1]], K[i]))) {  // the run's last item holds its value
+    // (every slot of this bucket was read into shared memory, and no list is written over)
+    if (head) put_group(bslot, gcount + __popc(hb & ((1u << lane) - 1u)), G.m[i], tcount + inc - tv, i, s, L.keep);
+    if (last) {  // the run's last item holds its value
       const uint32_t g = seg < 0 ? gcount - 1u : gcount + __popc(hb & ((1u << seg0) - 1u));
       bslot[g].tail.p = x;
     }
@@ -1432,173 +1517,62 @@ __global__ void __launch_bounds__(GW_WARPS * 32) group_warp_kernel(GroupLaunch L
     gcount += __popc(hb);
     tcount += __shfl_sync(0xFFFFFFFFu, inc, 31);
   }
+  return make_uint2(gcount, tcount);
+}
+
+// One warp per bucket.  A bucket of more than WARP_CAP items (repeated symptoms)
+// is left to the block's last warp to finish, which then has the block's
+// shared memory to itself; no warp waits for another.
+// Bound by latency and instructions (a warp's chain is two DRAM round trips,
+// the sort and the scan; the FP64 pipe is a third busy).  Ordering by a sort of
+// 32-bit words took the place of a counting sort into 64 sub-bins with a rank
+// inside each: 32 mixed surface codes (94k buckets of ~30 items) 153 -> 145 us,
+// and the launch for large buckets is gone ([[144,12,12]]: grouping, scan and
+// emission 23.9 -> 19.2 us).  A block barrier before the large buckets cost
+// 13 us of 158.
+__global__ void __launch_bounds__(GW_WARPS * 32) group_kernel(const __grid_constant__ GroupLaunch L) {
+  __shared__ union Shared {
+    GroupItems<WARP_CAP> w[GW_WARPS];
+    GroupItems<SLOT_CAP> all;
+    __device__ Shared() {}
+  } S;
+  __shared__ uint32_t s_done;
+  if (threadIdx.x == 0) s_done = 0;
+  __syncthreads();
+  const uint32_t lane = threadIdx.x & 31u, wi = threadIdx.x >> 5;
+  const uint32_t b0 = blockIdx.x * GW_WARPS, b = b0 + wi;
+  const uint32_t n = b < L.nb ? bucket_items(L.count[b]) : 0u;
+  auto put = [&](uint32_t bucket, uint2 a, uint32_t items) {
+    if (lane != 0) return;
+    L.bagg[bucket] = a;
+    if (a.x == 0) return;
+    red_add(&L.tsum[bucket / SCAN_TILE].x, a.x);
+    red_add(&L.tsum[bucket / SCAN_TILE].y, a.y);
+    red_add(L.totals + 3, items);
+  };
+  // (a bucket past SLOT_CAP items overflowed: flagged by the key pass, the run is redone another way)
+  const bool big = n > WARP_CAP && n <= SLOT_CAP;
+  if (b < L.nb && !big) {
+    uint2 agg = make_uint2(0, 0);
+    if (n && n <= WARP_CAP) agg = group_warp(L, S.w[wi], b, n);
+    put(b, agg, n);
+  }
+  __syncwarp();
+  uint32_t done = 0;
   if (lane == 0) {
-    L.bagg[b] = make_uint2(gcount, tcount);
-    red_add(&L.tsum[b / SCAN_TILE].x, gcount);
-    red_add(&L.tsum[b / SCAN_TILE].y, tcount);
-    red_add(L.totals + 3, n);
+    __threadfence_block();
+    done = atomicAdd(&s_done, big ? 0x101u : 1u) + (big ? 0x101u : 1u);
   }
-}
-
-// One CTA per listed bucket (WARP_CAP < items <= SLOT_CAP), persistent over
-// the list; one thread per slot.  Same order and arithmetic as
-// group_warp_kernel: sub-bin counting sort, rank inside a sub-bin, then each
-// warp takes 32 sorted positions (heads, target offsets, segmented scan of
-// the XOR-merge) and one thread chains the runs across the warps' chunks.
-constexpr uint32_t GB_THREADS = SLOT_CAP;
-__global__ void __launch_bounds__(GB_THREADS) group_big_kernel(GroupLaunch L) {
-  constexpr uint32_t NBIN = 64, NWARP = GB_THREADS / 32;
-  __shared__ ulonglong2 sk[SLOT_CAP];
-  __shared__ uint32_t sm[SLOT_CAP], st[SLOT_CAP];
-  __shared__ double sp[SLOT_CAP];
-  __shared__ uint16_t ord[SLOT_CAP], sx[SLOT_CAP];
-  __shared__ uint8_t sq[SLOT_CAP];
-  __shared__ uint32_t sh[NBIN];
-  __shared__ uint32_t c_groups[NWARP], c_targets[NWARP], c_head[NWARP], c_gbase[NWARP], c_tbase[NWARP];
-  __shared__ double c_tail[NWARP], c_carry[NWARP];
-  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  const uint32_t nbig = *L.big_n;
-  const uint32_t tcap = L.tcap;
-  for (uint32_t kb = blockIdx.x; kb < nbig; kb += gridDim.x) {
-    const uint32_t b = L.big_list[kb];
-    const uint32_t n = bucket_items(L.count[b]);  // WARP_CAP < n <= SLOT_CAP
-    const size_t base = (size_t)b * SLOT_CAP;
-    if (tid < NBIN) sh[tid] = 0;
-    __syncthreads();
-    if (tid < n) {
-      const ulonglong2 k = L.slot[base + tid].key;
-      const SlotTail t = L.slot[base + tid].tail;
-      sk[tid] = k;
-      sm[tid] = t.m;
-      st[tid] = t.t;
-      sp[tid] = t.p;
-      sq[tid] = (uint8_t)atomicAdd(sh + (uint32_t)(k.y >> 58), 1u);
-    }
-    __syncthreads();
-    if (warp == 0) {
-      const uint32_t c0 = sh[2 * lane], c1 = sh[2 * lane + 1];
-      uint32_t inc = c0 + c1;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-        if (lane >= (uint32_t)o) inc += a;
-      }
-      const uint32_t ex = inc - c0 - c1;
-      __syncwarp();
-      sh[2 * lane] = ex;
-      sh[2 * lane + 1] = ex + c0;
-    }
-    __syncthreads();
-    if (tid < n) sx[sh[(uint32_t)(sk[tid].y >> 58)] + sq[tid]] = (uint16_t)tid;
-    __syncthreads();
-    if (tid < n) {
-      const ulonglong2 ki = sk[tid];
-      const uint32_t mi = sm[tid];
-      const uint32_t bin = (uint32_t)(ki.y >> 58);
-      const uint32_t lo = sh[bin], hi = bin + 1 < NBIN ? sh[bin + 1] : n;
-      uint32_t r = lo;
-      for (uint32_t j = lo; j < hi; ++j) {
-        const uint32_t x = sx[j];
-        r += item_less(sk[x], sm[x], ki, mi) ? 1u : 0u;
-      }
-      ord[r] = (uint16_t)tid;
-    }
-    __syncthreads();
-    // position s = tid: heads, collisions, per-chunk scans
-    const uint32_t s = tid;
-    const bool in = s < n;
-    bool head = false;
-    uint32_t i = 0, nt = 0;
-    if (in) {
-      i = ord[s];
-      nt = st[i] & kSlotCount;
-      head = true;
-      if (s > 0) {
-        const uint32_t ip = ord[s - 1];
-        if (key_eq(sk[ip], sk[i])) {
-          head = false;
-          // (lists longer than the stride: flagged by the key pass, redone wider)
-          const Slot *const bs = L.slot + base;
-          if (nt <= tcap && ((st[ip] & kSlotCount) != nt || !slot_lists_equal(L, bs + i, sm[i], bs + ip, sm[ip], nt)))
-            atomicOr(L.err, DEV_ERR_COLLISION);
-        }
-      }
-    }
-    const uint32_t hb = __ballot_sync(0xFFFFFFFFu, head);
-    const uint32_t tv = head ? nt : 0u;
-    uint32_t inc = tv;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-      if (lane >= (uint32_t)o) inc += a;
-    }
-    const uint32_t le = hb & (0xFFFFFFFFu >> (31u - lane));
-    const int seg = le ? 31 - __clz(le) : -1;
-    const uint32_t seg0 = seg < 0 ? 0u : (uint32_t)seg;
-    double x = in ? sp[i] : 0.0;
-    const uint32_t maxlen = __reduce_max_sync(0xFFFFFFFFu, in ? lane - seg0 + 1 : 0u);
-    for (uint32_t d = 1; d < maxlen; d <<= 1) {
-      const double y = __shfl_up_sync(0xFFFFFFFFu, x, d);
-      if (lane >= d && lane - d >= seg0) x = xor_merge(y, x);
-    }
-    if (lane == 31) {
-      c_groups[warp] = __popc(hb);
-      c_targets[warp] = inc;
-      c_head[warp] = hb != 0u;
-      c_tail[warp] = x;
-    }
-    __syncthreads();
-    if (tid == 0) {  // chain the chunks: group/target bases and the run carried into each chunk
-      uint32_t g = 0, t = 0;
-      double run = 0.0;
-      for (uint32_t c = 0; c < NWARP; ++c) {
-        c_gbase[c] = g;
-        c_tbase[c] = t;
-        c_carry[c] = run;
-        g += c_groups[c];
-        t += c_targets[c];
-        run = c_head[c] ? c_tail[c] : xor_merge(run, c_tail[c]);
-      }
-      L.bagg[b] = make_uint2(g, t);
-      red_add(&L.tsum[b / SCAN_TILE].x, g);
-      red_add(&L.tsum[b / SCAN_TILE].y, t);
-      red_add(L.totals + 3, n);
-    }
-    __syncthreads();
-    if (seg < 0) x = xor_merge(c_carry[warp], x);
-    const uint32_t gb = c_gbase[warp];
-    Slot *const bslot = L.slot + base;
-    if (in) {
-      slot_perm(bslot, s)[0] = sm[i];
-      slot_perm(bslot, s)[3] = st[i] >> 24;
-    }
-    if (head) {
-      const uint32_t g = gb + __popc(hb & ((1u << lane) - 1u));
-      bslot[g].tail.m = sm[i];
-      bslot[g].tail.t = c_tbase[warp] + inc - tv;
-      slot_perm(bslot, g)[1] = s;
-      slot_perm(bslot, g)[2] = i;
-    }
-    if (in && (s + 1 >= n || !key_eq(sk[ord[s + 1]], sk[i]))) {
-      const uint32_t g = seg < 0 ? gb - 1u : gb + __popc(hb & ((1u << seg0) - 1u));
-      bslot[g].tail.p = x;
-    }
-    __syncthreads();
+  done = __shfl_sync(0xFFFFFFFFu, done, 0);
+  if ((done & 255u) < GW_WARPS || (done >> 8) == 0) return;
+  __threadfence_block();
+  for (uint32_t k = 0; k < GW_WARPS && b0 + k < L.nb; ++k) {
+    const uint32_t nk = bucket_items(L.count[b0 + k]);
+    if (nk <= WARP_CAP || nk > SLOT_CAP) continue;
+    const uint2 a = group_warp(L, S.all, b0 + k, nk);
+    put(b0 + k, a, nk);
+    __syncwarp();
   }
-}
-
-// Block sum of a pair over 1024 threads (result in every thread).
-__device__ __forceinline__ uint2 block_sum1024(uint2 v, uint2 *scratch) {
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  v.x = __reduce_add_sync(0xFFFFFFFFu, v.x);
-  v.y = __reduce_add_sync(0xFFFFFFFFu, v.y);
-  if (lane == 0) scratch[warp] = v;
-  __syncthreads();
-  uint2 a = lane < 32 ? scratch[lane] : make_uint2(0, 0);
-  a.x = __reduce_add_sync(0xFFFFFFFFu, a.x);
-  a.y = __reduce_add_sync(0xFFFFFFFFu, a.y);
-  __syncthreads();
-  return a;
 }
 
 // Exclusive scan of the bucket aggregates: block t covers buckets
@@ -1679,51 +1653,104 @@ __global__ void __launch_bounds__(SCAN_THREADS) group_scan_kernel(GroupLaunch L)
   }
 }
 
-// One warp per bucket: the bucket's groups to the DEM arrays.  Block 0 also
-// writes each circuit's first output slot and target.
-__global__ void __launch_bounds__(GW_WARPS * 32) emit_kernel(GroupLaunch L) {
-  if (blockIdx.x == 0)
-    for (uint32_t c = threadIdx.x; c < L.n_circ; c += GW_WARPS * 32) L.cout[c] = L.bout[L.cbbase[c]];
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t b = blockIdx.x * GW_WARPS + (threadIdx.x >> 5);
-  if (b >= L.nb) return;
-  const size_t base = (size_t)b * SLOT_CAP;
-  // the first records load beside the bucket's aggregate and offset (a slot
-  // past the groups holds whatever it held: only the ones below agg.x are used)
-  SlotTail t = L.slot[base + lane].tail, tn1 = L.slot[base + lane + 1].tail;
-  const uint2 agg = L.bagg[b], out = L.bout[b];
-  const uint32_t tcap = L.tcap;
+// One warp's bucket: its groups to the DEM arrays from slot `out.x` and target `out.y` on.
+__device__ __forceinline__ void emit_bucket(const GroupLaunch &L, uint32_t b, uint2 agg, uint2 out, SlotTail t, SlotTail tn1) {
+  const uint32_t lane = threadIdx.x & 31u, tcap = L.tcap;
+  const Slot *const bslot = L.slot + (size_t)b * SLOT_CAP;
   for (uint32_t g = lane; g < agg.x; g += 32) {
     if (g != lane) {
-      t = L.slot[base + g].tail;
-      if (g + 1 < agg.x) tn1 = L.slot[base + g + 1].tail;  // (slot g + 1 <= SLOT_CAP - 1)
+      t = bslot[g].tail;
+      if (g + 1 < agg.x) tn1 = bslot[g + 1].tail;  // (slot g + 1 <= SLOT_CAP - 1)
     }
-    const uint32_t slot = out.x + g;
-    const uint32_t toff = out.y + t.t;
+    const uint32_t slot = out.x + g, toff = out.y + (t.t >> 8);
     L.out_prob[slot] = t.p;
     L.out_off[slot] = toff;
     // the group's targets run to the next group's (the bucket's total after
     // the last); a list longer than the rows was flagged by the key pass and
     // the run is redone with wider rows, so only the rows' targets are copied
-    const uint32_t ntg = min((g + 1 < agg.x ? tn1.t : agg.y) - t.t, tcap);
+    const uint32_t ntg = min((g + 1 < agg.x ? tn1.t >> 8 : agg.y) - (t.t >> 8), tcap);
     if ((uint64_t)toff + ntg <= L.tg_cap) {
-      const uint4 *src = reinterpret_cast<const uint4 *>(L.slot[base + slot_perm(L.slot + base, g)[2]].list);
+      const uint4 *src = reinterpret_cast<const uint4 *>(bslot[t.t & 255u].list);
       const uint4 x0 = src[0], x1 = src[1];
       const uint32_t l[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-      uint32_t *out = L.out_tg + toff;
+      uint32_t *o = L.out_tg + toff;
       if (L.narrow) {
 #pragma unroll
         for (uint32_t k = 0; k < 16; ++k)
-          if (k < ntg) out[k] = (l[k / 2] >> (k % 2 * 16)) & 0xFFFFu;
+          if (k < ntg) o[k] = (l[k / 2] >> (k % 2 * 16)) & 0xFFFFu;
       } else {
 #pragma unroll
         for (uint32_t k = 0; k < 8; ++k)
-          if (k < ntg) out[k] = l[k];
+          if (k < ntg) o[k] = l[k];
       }
       const uint32_t inl = L.narrow ? 16u : 8u;
-      for (uint32_t k = inl; k < ntg; ++k) out[k] = __ldg(L.tl + (size_t)t.m * L.tstride + k - inl);
+      for (uint32_t k = inl; k < ntg; ++k) o[k] = __ldg(L.tl + (size_t)t.m * L.tstride + k - inl);
     }
   }
+}
+
+// One warp per bucket: the bucket's groups to the DEM arrays.  FOLD: the blocks
+// find their buckets' places themselves (the tile sums before the block's tile
+// and the aggregates before it in the tile: a few loads a thread for up to
+// kFoldBuckets buckets), which saves a small run the scan kernel; the block of
+// a circuit's first bucket writes the circuit's place, the last block the
+// totals.
+template <bool FOLD>
+__global__ void __launch_bounds__(GW_WARPS * 32) emit_kernel(const __grid_constant__ GroupLaunch L) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, wi = tid >> 5;
+  const uint32_t b0 = blockIdx.x * GW_WARPS, b = b0 + wi;
+  // the first records load beside the bucket's aggregate and offset (a slot
+  // past the groups holds whatever it held: only the ones below agg.x are used)
+  SlotTail t{}, tn1{};
+  uint2 agg = make_uint2(0, 0), out;
+  if (b < L.nb) {
+    t = L.slot[(size_t)b * SLOT_CAP + lane].tail;
+    tn1 = L.slot[(size_t)b * SLOT_CAP + lane + 1].tail;
+    agg = L.bagg[b];
+  }
+  if constexpr (FOLD) {
+    __shared__ uint2 s_sum[GW_WARPS], s_agg[GW_WARPS];
+    const uint32_t tile = b0 / SCAN_TILE;
+    uint2 pre = make_uint2(0, 0);
+    for (uint32_t k = tid; k < tile; k += GW_WARPS * 32) {
+      const uint2 a = L.tsum[k];
+      pre.x += a.x;
+      pre.y += a.y;
+    }
+    for (uint32_t k = tile * SCAN_TILE + tid; k < b0; k += GW_WARPS * 32) {
+      const uint2 a = L.bagg[k];
+      pre.x += a.x;
+      pre.y += a.y;
+    }
+    pre.x = __reduce_add_sync(0xFFFFFFFFu, pre.x);
+    pre.y = __reduce_add_sync(0xFFFFFFFFu, pre.y);
+    if (lane == 0) {
+      s_sum[wi] = pre;
+      s_agg[wi] = agg;
+    }
+    __syncthreads();
+    out = make_uint2(0, 0);
+#pragma unroll
+    for (uint32_t k = 0; k < GW_WARPS; ++k) {
+      out.x += s_sum[k].x + (k < wi ? s_agg[k].x : 0u);
+      out.y += s_sum[k].y + (k < wi ? s_agg[k].y : 0u);
+    }
+    if (b < L.nb && lane == 0) L.bout[b] = out;
+    if (b == L.nb - 1 && lane == 0) {
+      const uint2 end = make_uint2(out.x + agg.x, out.y + agg.y);
+      L.totals[0] = end.x;
+      L.totals[1] = end.y;
+      L.out_off[end.x] = end.y;  // the closing offset
+      if (end.y > L.tg_cap) atomicOr(L.err, DEV_FLAG_TG_OVF);
+    }
+    for (uint32_t c = lane; c < L.n_circ; c += 32)
+      if (L.cbbase[c] == b) L.cout[c] = out;
+  } else {
+    if (blockIdx.x == 0)
+      for (uint32_t c = tid; c < L.n_circ; c += GW_WARPS * 32) L.cout[c] = L.bout[L.cbbase[c]];
+    out = b < L.nb ? L.bout[b] : make_uint2(0, 0);
+  }
+  if (b < L.nb) emit_bucket(L, b, agg, out, t, tn1);
 }
 
 // ---- noise-rate gradients ---------------------------------------------------
@@ -1861,15 +1888,19 @@ cudaError_t launch_bucket_scatter(const ulonglong2 *key, uint32_t M, uint32_t bu
 
 cudaError_t launch_group(const GroupLaunch &L, cudaStream_t s) {
   if (L.nb == 0) return cudaSuccess;
-  group_warp_kernel<<<(L.nb + GW_WARPS - 1) / GW_WARPS, GW_WARPS * 32, 0, s>>>(L);
-  group_big_kernel<<<2 * 152, GB_THREADS, 0, s>>>(L);
+  group_kernel<<<(L.nb + GW_WARPS - 1) / GW_WARPS, GW_WARPS * 32, 0, s>>>(L);
   return cudaGetLastError();
 }
 
 cudaError_t launch_scan_emit(const GroupLaunch &L, cudaStream_t s) {
   if (L.nb == 0) return cudaSuccess;
-  group_scan_kernel<<<(L.nb + SCAN_TILE - 1) / SCAN_TILE, SCAN_THREADS, 0, s>>>(L);
-  emit_kernel<<<(L.nb + GW_WARPS - 1) / GW_WARPS, GW_WARPS * 32, 0, s>>>(L);
+  const uint32_t blocks = (L.nb + GW_WARPS - 1) / GW_WARPS;
+  if (L.nb <= kFoldBuckets) {
+    emit_kernel<true><<<blocks, GW_WARPS * 32, 0, s>>>(L);
+  } else {
+    group_scan_kernel<<<(L.nb + SCAN_TILE - 1) / SCAN_TILE, SCAN_THREADS, 0, s>>>(L);
+    emit_kernel<false><<<blocks, GW_WARPS * 32, 0, s>>>(L);
+  }
   return cudaGetLastError();
 }
 
