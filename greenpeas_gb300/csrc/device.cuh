@@ -207,6 +207,7 @@ struct KeyLaunch {
   Slot *slot;               // [buckets * SLOT_CAP] bucket slots
   uint32_t *tl;             // [M][tstride] targets past a slot's
   uint32_t tstride, narrow;
+  uint32_t keep;            // gradients (one circuit): an item's m is its record << 4 | its first component
   uint32_t *list_total;     // += targets written to the lists (for traffic accounting)
   uint32_t *err;
   ulonglong2 *key;          // [M] global path (one circuit)
@@ -266,7 +267,8 @@ struct GroupLaunch {
   uint32_t tcap, tstride, narrow;
   Slot *slot;               // [nb * SLOT_CAP] items; afterwards one group record per group in the tails and
                             // (keep) the saved permutation in the keys (slot_perm)
-  uint32_t keep;
+  uint32_t keep;            // gradients: keep the permutation; an item's m is its record << 4 | its first component
+  const uint32_t *rec_moff; // (keep) first mechanism of each record
   const uint32_t *count;    // [nb] (bucket_items)
   uint32_t nb;
   uint2 *bagg;              // [nb] (groups, targets) of each bucket
@@ -303,24 +305,20 @@ cudaError_t launch_param_rec(const ParamLaunch &L, cudaStream_t s);
 //  group:  one warp per bucket, a lane per group: dL/dq_m = dL/dp_g *
 //          prod_{j in g, j != m} (1 - 2 q_j) from prefix and suffix products
 //          along the group's run in the saved permutation;
-//  record: dL/dp_r = (sum of its mechanisms' dL/dq) * dq/dp, the split's
-//          slope at the source's rate (stab[src][kind], filled by the host);
-//  source: dL/dnoise[e] = sum over the records of source e, in record order.
+//  source: dL/dnoise[e] = sum over the records of source e of (the sum of the
+//          record's mechanisms' dL/dq) * dq/dp, the split's slope at the
+//          source's rate (stab[src][kind], filled by the host).
 struct AdjointLaunch {
   const Slot *slot;        // saved permutation (see GroupLaunch)
   const uint32_t *count;
   const uint2 *bagg, *bout;
   uint32_t nb;
-  const uint32_t *first;   // [key warps] first record of each key warp (launch_key_prep)
-  uint32_t chunk;
   const double *rec_p;     // [R] each record's component probability of the forward (from the noise tensor)
   const double *grad_out;  // [groups] dL/dp of each merged mechanism
   double *gq;              // [M] (zeroed) dL/dq summed over each item's mechanisms, at its first mechanism
   const uint64_t *rec;
-  const uint32_t *rec_src, *rec_moff;
-  uint32_t R;
+  const uint32_t *rec_moff;
   const double *stab;      // [n_src][3] dq/dp of each source and channel kind
-  double *grad_rec;        // [R]
   const uint32_t *src_off, *src_rec;  // records of each source (CSR, record order)
   uint32_t n_src;
   double *grad_noise;      // [n_src]

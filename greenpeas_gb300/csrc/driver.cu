@@ -161,7 +161,7 @@ struct Layout {
   size_t mdesc, mp, tl, key, key_first, slot, bagg, bout, cout;
   size_t zero, err, totals, bcount, tsum, wq, zero_bytes;
   size_t sk0, sk1, pm0, pm1, hik;  // global path (single circuit)
-  size_t src_off, src_rec, gq, grad_rec, ptab;  // noise-rate gradients (single circuit)
+  size_t src_off, src_rec, gq, ptab;  // noise-rate gradients (single circuit)
   size_t gzero, sort_scr, merge_status, merge_ctr, gzero_bytes;
   size_t out_prob, out_off;
   size_t seg_items, seg_aff, seg_state, seg_xcnt, seg_xlst;  // segmented walk (single circuit)
@@ -793,7 +793,6 @@ struct gpc_driver {
     L.merge_tiles = gpc::merge_tiles(Mg);
     L.sort_words = Mg ? gpc::sort_scratch_words(Mg, 64) : 0;
     L.gq = take(param ? (size_t)M * 8 : 0);
-    L.grad_rec = take(param ? tapes[0].rec.size() * 8 : 0);
     L.ptab = take(param ? (size_t)tapes[0].n_ticks * gpc::SRC_CLASSES * 6 * 8 : 0);  // q and dq/dp tables
     L.gzero = o;
     L.sort_scr = take(L.sort_words * 4);
@@ -1388,6 +1387,7 @@ struct gpc_driver {
     kl.tl = dptr<uint32_t>(L.tl);
     kl.tstride = tstride;
     kl.narrow = narrow ? 1u : 0u;
+    kl.keep = param ? 1u : 0u;
     kl.list_total = dptr<uint32_t>(L.totals) + 2;
     kl.err = dptr<uint32_t>(L.err);
     kl.key = dptr<ulonglong2>(L.key);
@@ -1442,6 +1442,7 @@ struct gpc_driver {
     gl.bout = dptr<uint2>(L.bout);
     gl.tsum = dptr<uint2>(L.tsum);
     gl.keep = param ? 1u : 0u;
+    gl.rec_moff = dptr<uint32_t>(L.c[0].rec_moff);
     gl.out_prob = dptr<double>(L.out_prob);
     gl.out_off = dptr<uint32_t>(L.out_off);
     gl.out_tg = static_cast<uint32_t *>(tgbuf.p);
@@ -1759,7 +1760,6 @@ struct gpc_driver {
     if (!grad_out || !grad_noise) throw gpc::Error(GPC_ERR_INVALID, "null gradient buffer");
     CK(cudaSetDevice(device));
     wait_caller(caller);
-    const Tape &T = tapes[0];
     CK(cudaMemsetAsync(dptr<char>(L.gq), 0, (size_t)L.M * 8, stream));
     gpc::AdjointLaunch A{};
     A.slot = dptr<gpc::Slot>(L.slot);
@@ -1767,17 +1767,12 @@ struct gpc_driver {
     A.bagg = dptr<uint2>(L.bagg);
     A.bout = dptr<uint2>(L.bout);
     A.nb = L.nb;
-    A.first = dptr<uint32_t>(L.key_first);
-    A.chunk = L.key_chunk;
     A.rec_p = dptr<double>(L.c[0].rec_p);
     A.grad_out = grad_out;
     A.gq = dptr<double>(L.gq);
     A.rec = dptr<uint64_t>(L.c[0].rec);
-    A.rec_src = dptr<uint32_t>(L.c[0].rec_src);
     A.rec_moff = dptr<uint32_t>(L.c[0].rec_moff);
-    A.R = (uint32_t)T.rec.size();
     A.stab = dptr<double>(L.ptab) + (size_t)n_src() * 3;
-    A.grad_rec = dptr<double>(L.grad_rec);
     A.src_off = dptr<uint32_t>(L.src_off);
     A.src_rec = dptr<uint32_t>(L.src_rec);
     A.n_src = n_src();

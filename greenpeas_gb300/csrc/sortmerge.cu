@@ -204,6 +204,12 @@ __device__ __forceinline__ uint32_t coset_heads(uint32_t present, uint32_t zero,
   return heads;
 }
 
+// An item's name when the gradients need its record: the record and the place
+// of its first component (in the same order as the first mechanisms).
+__device__ __forceinline__ uint32_t item_id(uint32_t r, uint32_t type, uint32_t s) {
+  return r << 4 | ((uint32_t)(kPlace[type] >> (4u * s)) & 15u);
+}
+
 // Files an item in its bucket: one 64-byte slot as two 32-byte stores.  The
 // bucket's counter counts items in its low half and mechanisms in its high
 // half: a bucket overflows by its mechanisms, whatever is merged beforehand.
@@ -282,7 +288,7 @@ __device__ __noinline__ uint32_t key_record_direct(const KeyLaunch &L, const Cir
     uint32_t l[8];
     for (uint32_t i = 0; i < 8; ++i) l[i] = mine[i];
     const uint32_t mult = (uint32_t)__popc(xor_bits16(join, s) & present);
-    file_item(L, C.bbase, C.bbits, C.tcap, hx, hy, m, cnt, mult, repeat_merge(__ldg(C.rec_p + r), mult), l);
+    file_item(L, C.bbase, C.bbits, C.tcap, hx, hy, L.keep ? item_id(r, type, s) : m, cnt, mult, repeat_merge(__ldg(C.rec_p + r), mult), l);
   }
   return cnt;
 }
@@ -532,7 +538,7 @@ __global__ void __launch_bounds__(kKeyWarps * 32, 4) key_items_kernel(const __gr
         }
       }
       if (!in) continue;
-      const uint32_t m = S.moff[k] + (uint32_t)(S.place[k] >> (4u * s) & 15u);
+      const uint32_t place = (uint32_t)(S.place[k] >> (4u * s)) & 15u, m = S.moff[k] + place;
       if (t) {  // the rest of a long list
         uint32_t *far = L.tl + (size_t)m * L.tstride;
         for (uint32_t i = 0; t; t &= t - 1, ++i)
@@ -540,7 +546,7 @@ __global__ void __launch_bounds__(kKeyWarps * 32, 4) key_items_kernel(const __gr
       }
       const uint32_t mult = (uint32_t)__popc(xor_bits16(S.join[k], s) & S.present[k]);
       listed += cnt;
-      file_item(L, bbase, bbits, tcap, hx, hy, m, cnt, mult, repeat_merge(S.p[k], mult), l);
+      file_item(L, bbase, bbits, tcap, hx, hy, L.keep ? (r0 + k) << 4 | place : m, cnt, mult, repeat_merge(S.p[k], mult), l);
     }
     r0 += take;
   }
@@ -1267,6 +1273,12 @@ constexpr uint32_t kFoldBuckets = 32768;  // most buckets whose places the emiss
 
 __device__ __forceinline__ bool key_eq(ulonglong2 a, ulonglong2 b) { return a.x == b.x && a.y == b.y; }
 
+// Row of an item's later targets: its first mechanism.
+__device__ __forceinline__ const uint32_t *far_targets(const GroupLaunch &L, uint32_t m) {
+  if (L.keep) m = __ldg(L.rec_moff + (m >> 4)) + (m & 15u);
+  return L.tl + (size_t)m * L.tstride;
+}
+
 // The targets of two items: the slots' first ones as two 16-byte words (unused
 // entries are zero), the rest of longer lists from their rows.
 __device__ __forceinline__ bool slot_lists_equal(const GroupLaunch &L, const Slot *a, uint32_t ma, const Slot *b,
@@ -1277,7 +1289,7 @@ __device__ __forceinline__ bool slot_lists_equal(const GroupLaunch &L, const Slo
       (x1.w ^ y1.w))
     return false;
   const uint32_t inl = L.narrow ? 16u : 8u;
-  return n <= inl || lists_equal(L.tl + (size_t)ma * L.tstride, L.tl + (size_t)mb * L.tstride, n - inl);
+  return n <= inl || lists_equal(far_targets(L, ma), far_targets(L, mb), n - inl);
 }
 
 // What a bucket's grouping holds in shared memory: its items as they were
@@ -1684,7 +1696,10 @@ __device__ __forceinline__ void emit_bucket(const GroupLaunch &L, uint32_t b, ui
           if (k < ntg) o[k] = l[k];
       }
       const uint32_t inl = L.narrow ? 16u : 8u;
-      for (uint32_t k = inl; k < ntg; ++k) o[k] = __ldg(L.tl + (size_t)t.m * L.tstride + k - inl);
+      if (ntg > inl) {
+        const uint32_t *far = far_targets(L, t.m);
+        for (uint32_t k = inl; k < ntg; ++k) o[k] = __ldg(far + k - inl);
+      }
     }
   }
 }
@@ -1768,63 +1783,134 @@ __global__ void param_rec_kernel(ParamLaunch L) {
   L.rec_p[r] = L.qtab[(size_t)src * 3 + channel_kind((uint32_t)((L.rec[r] >> 56) & 15u))];
 }
 
-// An item of c mechanisms of probability q counts as (1 - 2q)^c in its run's
-// product; its first mechanism's entry takes the derivative by all c of them.
-__global__ void __launch_bounds__(GW_WARPS * 32) adjoint_group_kernel(AdjointLaunch A) {
-  __shared__ double s_q[GW_WARPS][SLOT_CAP];  // probability of the mechanisms at each sorted position
+// One warp per bucket, a lane per sorted position.  An item of c mechanisms of
+// probability q counts as f^c, f = 1 - 2q, in its run's product; its entry
+// (first mechanism) takes the derivative by all c of them, dL/dp_g * c f^(c-1)
+// * the run's other items'.  The products before and after an item are
+// segmented scans, forward over the chunks of 32 positions and then backward.
+// Bound by latency and the FP64 pipe (two multiplications a cycle and SM): with
+// a lane per run that walked it, every step of the longest run of 32 took the
+// pipe for 16 cycles (43 us on [[144,12,12]] walking in global memory with a
+// search of each item's record, 24 in shared memory; now 16).
+constexpr uint32_t ADJ_THREADS = 128;
+__global__ void __launch_bounds__(GW_WARPS * 32) adjoint_group_kernel(const __grid_constant__ AdjointLaunch A) {
+  __shared__ double s_pre[GW_WARPS][SLOT_CAP];
+  __shared__ uint32_t s_start[GW_WARPS][SLOT_CAP / 32];  // bit per sorted position: a run starts there
+  constexpr uint32_t ALL = 0xFFFFFFFFu;
   const uint32_t lane = threadIdx.x & 31u, wi = threadIdx.x >> 5;
   const uint32_t b = blockIdx.x * GW_WARPS + wi;
   if (b >= A.nb) return;
   const uint32_t n = bucket_items(A.count[b]);
-  if (n == 0 || n > SLOT_CAP) return;
   const uint32_t groups = A.bagg[b].x, out0 = A.bout[b].x;
+  if (n == 0 || n > SLOT_CAP) return;
   const Slot *const bslot = A.slot + (size_t)b * SLOT_CAP;
-  double *q = s_q[wi];
-  // the forward's mechanism probabilities, recomputed from the records (every
-  // component of a record carries the record's probability)
-  for (uint32_t s = lane; s < n; s += 32)
-    q[s] = __ldg(A.rec_p + record_of(A.first, A.chunk, A.rec_moff, A.R, slot_perm(bslot, s)[0]));
+  double *pre = s_pre[wi];
+  uint32_t *start = s_start[wi];
+  if (lane < SLOT_CAP / 32) start[lane] = 0;
   __syncwarp();
-  for (uint32_t g = lane; g < groups; g += 32) {
-    const uint32_t s0 = slot_perm(bslot, g)[1], s1 = g + 1 < groups ? slot_perm(bslot, g + 1)[1] : n;
-    const double dl = A.grad_out[out0 + g];
-    double pre = 1.0;
-    for (uint32_t s = s0; s < s1; ++s) {
-      const double f = 1.0 - 2.0 * q[s];
-      const uint32_t c = slot_perm(bslot, s)[3];
-      for (uint32_t k = 1; k < c; ++k) pre *= f;  // (the item's other mechanisms)
-      A.gq[slot_perm(bslot, s)[0]] = pre * (double)c;
-      pre *= f;
+  for (uint32_t k = lane; k < groups; k += 32) {
+    const uint32_t s = slot_perm(bslot, k)[1];
+    atomicOr(start + s / 32, 1u << (s & 31u));
+  }
+  __syncwarp();
+  // an item's f and count; its power f^c
+  auto item = [&](uint32_t s, uint32_t &id, uint32_t &c, double &f) {
+    const uint4 w = *reinterpret_cast<const uint4 *>(slot_perm(bslot, s));
+    id = w.x;
+    c = w.w;
+    f = 1.0 - 2.0 * __ldg(A.rec_p + (w.x >> 4));  // (the forward's, from the noise tensor)
+  };
+  auto power = [&](double f, uint32_t c) {
+    double x = c & 1u ? f : 1.0;
+    for (uint32_t k = c >> 1; k; k >>= 1) {
+      f *= f;
+      if (k & 1u) x *= f;
     }
-    double suf = 1.0;
-    for (uint32_t s = s1; s-- > s0;) {
-      const uint32_t m = slot_perm(bslot, s)[0];
-      A.gq[m] = dl * A.gq[m] * suf;
-      const double f = 1.0 - 2.0 * q[s];
-      for (uint32_t k = slot_perm(bslot, s)[3]; k > 0; --k) suf *= f;
+    return x;
+  };
+  const uint32_t chunks = (n + 31u) / 32u;
+  uint32_t id = 0, c = 1, g1 = 0;  // the last chunk's items stay in registers for the way back; g1: runs before the chunk
+  double f = 1.0, carry = 1.0;
+  for (uint32_t k = 0; k < chunks; ++k) {
+    const uint32_t s = k * 32 + lane, hb = start[k];
+    const uint32_t le = hb & (ALL >> (31u - lane));
+    const uint32_t first = le ? 31u - __clz(le) : 0u;
+    id = 0;
+    c = 1;
+    f = 1.0;
+    if (s < n) item(s, id, c, f);
+    double x = power(f, c);
+    const uint32_t longest = __reduce_max_sync(ALL, lane - first + 1u);
+    for (uint32_t o = 1; o < longest; o <<= 1) {
+      const double y = __shfl_up_sync(ALL, x, o);
+      if (lane >= first + o) x *= y;
     }
+    if (le == 0) x *= carry;
+    double before = __shfl_up_sync(ALL, x, 1);  // inclusive -> exclusive
+    if (lane == 0) before = carry;
+    if ((hb >> lane) & 1u) before = 1.0;
+    if (s < n) pre[s] = before;
+    carry = __shfl_sync(ALL, x, 31);
+    if (k + 1 < chunks) g1 += (uint32_t)__popc(hb);
+  }
+  carry = 1.0;         // product of the items of the chunk after that go on with the open run
+  bool open = false;   // the chunk after starts inside a run
+  for (uint32_t k = chunks; k-- > 0;) {
+    const uint32_t s = k * 32 + lane, hb = start[k];
+    if (k + 1 < chunks) {
+      id = 0;
+      c = 1;
+      f = 1.0;
+      if (s < n) item(s, id, c, f);
+      g1 -= (uint32_t)__popc(hb);
+    }
+    const uint32_t after = lane == 31u ? 0u : hb >> (lane + 1u);
+    const uint32_t end = after ? lane + (uint32_t)__ffs(after) : 32u;  // the run is lanes .. end - 1 of the chunk
+    double x = power(f, c);
+    const uint32_t longest = __reduce_max_sync(ALL, end - lane);
+    for (uint32_t o = 1; o < longest; o <<= 1) {
+      const double y = __shfl_down_sync(ALL, x, o);
+      if (lane + o < end) x *= y;
+    }
+    const bool goes_on = end == 32u && open;
+    if (goes_on) x *= carry;
+    double behind = __shfl_down_sync(ALL, x, 1);
+    if (lane == 31) behind = open ? carry : 1.0;
+    if (lane + 1u == end && end < 32u) behind = 1.0;
+    if (s < n) {
+      const uint32_t g = g1 + (uint32_t)__popc(hb & (ALL >> (31u - lane))) - 1u;  // (a run open at the chunk's start: the one before)
+      double v = A.grad_out[out0 + g] * pre[s] * behind;
+      if (c > 1) v *= (double)c * power(f, c - 1);
+      A.gq[__ldg(A.rec_moff + (id >> 4)) + (id & 15u)] = v;
+    }
+    carry = __shfl_sync(ALL, x, 0);
+    open = (hb & 1u) == 0;
   }
 }
 
-__global__ void adjoint_record_kernel(AdjointLaunch A) {
-  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= A.R) return;
-  const uint32_t src = A.rec_src[r];
-  if (src >= A.n_src) {
-    A.grad_rec[r] = 0.0;
-    return;
+// One block per source: dL/dnoise[e] = the sum over the source's records of
+// (the sum of the record's entries) * the split's slope.  A thread takes every
+// ADJ_THREADS-th record, then shuffle trees and the warps in order: a fixed
+// order (one thread per source, one record after another: 26 us on
+// [[144,12,12]]; a warp per source 10, now 6).
+__global__ void __launch_bounds__(ADJ_THREADS) adjoint_source_kernel(const __grid_constant__ AdjointLaunch A) {
+  __shared__ double s_sum[ADJ_THREADS / 32];
+  const uint32_t lane = threadIdx.x & 31u, e = blockIdx.x;
+  double sum = 0.0;
+  for (uint32_t k = A.src_off[e] + threadIdx.x, end = A.src_off[e + 1]; k < end; k += ADJ_THREADS) {
+    const uint32_t r = A.src_rec[k];
+    double q = 0.0;
+    for (uint32_t m = A.rec_moff[r], m1 = A.rec_moff[r + 1]; m < m1; ++m) q += A.gq[m];
+    sum += q * A.stab[(size_t)e * 3 + channel_kind((uint32_t)((A.rec[r] >> 56) & 15u))];
   }
-  double sum = 0.0;
-  for (uint32_t m = A.rec_moff[r]; m < A.rec_moff[r + 1]; ++m) sum += A.gq[m];
-  A.grad_rec[r] = sum * A.stab[(size_t)src * 3 + channel_kind((uint32_t)((A.rec[r] >> 56) & 15u))];
-}
-
-__global__ void adjoint_source_kernel(AdjointLaunch A) {
-  const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= A.n_src) return;
-  double sum = 0.0;
-  for (uint32_t k = A.src_off[e]; k < A.src_off[e + 1]; ++k) sum += A.grad_rec[A.src_rec[k]];
-  A.grad_noise[e] = sum;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xFFFFFFFFu, sum, o);
+  if (lane == 0) s_sum[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (uint32_t k = 1; k < ADJ_THREADS / 32; ++k) sum += s_sum[k];
+    A.grad_noise[e] = sum;
+  }
 }
 
 }  // namespace
@@ -1837,8 +1923,7 @@ cudaError_t launch_param_rec(const ParamLaunch &L, cudaStream_t s) {
 
 cudaError_t launch_adjoint(const AdjointLaunch &A, cudaStream_t s) {
   if (A.nb) adjoint_group_kernel<<<(A.nb + GW_WARPS - 1) / GW_WARPS, GW_WARPS * 32, 0, s>>>(A);
-  if (A.R) adjoint_record_kernel<<<(A.R + 255) / 256, 256, 0, s>>>(A);
-  if (A.n_src) adjoint_source_kernel<<<(A.n_src + 255) / 256, 256, 0, s>>>(A);
+  if (A.n_src) adjoint_source_kernel<<<A.n_src, ADJ_THREADS, 0, s>>>(A);
   return cudaGetLastError();
 }
 
