@@ -36,8 +36,6 @@ struct CircuitDev {
   const uint32_t *rec_moff;   // [R + 1]
   uint64_t *mdesc;            // [M] mechanism descriptors (global path)
   double *mp;                 // [M] mechanism probabilities (global path)
-  uint32_t *tl;               // allocation-free merge: [M][tcap] targets of each mechanism, ascending
-  uint32_t *tn;               // allocation-free merge: [M] number of targets of each mechanism
   uint32_t nq, qpad, n_epochs, w;
   uint32_t npoints, M, R;
   uint32_t tcap;              // most targets of a listed symptom (0: no target lists, merge from snapshots)
@@ -72,8 +70,6 @@ constexpr int SORT_TILE = SORT_THREADS * SORT_IPT;
 constexpr int RADIX_BITS = 8;
 constexpr int RADIX = 1 << RADIX_BITS;
 constexpr int MERGE_THREADS = 256;
-constexpr int BUCKET_THREADS = 128;
-constexpr int BUCKET_CAP = 1024;  // items one CTA sorts in shared memory (allocation-free merge)
 constexpr uint32_t SLOT_CAP = 256;  // slots of one bucket in the compile pipeline
 constexpr uint32_t WARP_CAP = 128;  // bucket items of a warp's own shared memory
 constexpr uint32_t SCAN_TILE = 1024;    // bucket aggregates one scan block covers
@@ -220,33 +216,6 @@ cudaError_t launch_key_prep(const KeyLaunch &L, cudaStream_t s);
 cudaError_t launch_keys(const KeyLaunch &L, cudaStream_t s);
 // Global path: every mechanism's key, descriptor and probability.
 cudaError_t launch_keys_all(const KeyLaunch &L, cudaStream_t s);
-
-// Exclusive scan of the bucket counts into bucket offsets (+ total at [nb]).
-cudaError_t launch_bucket_scan(const uint32_t *count, uint32_t *offset, uint32_t nb, cudaStream_t s);
-
-// Moves every non-empty mechanism to its bucket: items (key, m).
-cudaError_t launch_bucket_scatter(const ulonglong2 *key, uint32_t M, uint32_t bucket_bits, const uint32_t *offset,
-                                  uint32_t *cursor, ulonglong2 *bkey, uint32_t *bm, cudaStream_t s);
-
-struct BucketMergeLaunch {
-  const CircuitDev *c_dev;
-  uint32_t w;
-  const ulonglong2 *bkey;   // bucketed keys
-  const uint32_t *bm;       // bucketed mechanism ids
-  const uint32_t *count;    // [nb]
-  const uint32_t *offset;   // [nb]
-  uint32_t nb;
-  uint32_t max_groups;      // capacity of out_prob / out_off (the mechanism count)
-  double *out_prob;
-  uint32_t *out_off;
-  uint32_t *out_tg;
-  uint32_t tg_cap;
-  unsigned long long *status;  // [nb]
-  uint32_t *ticket;
-  uint32_t *totals;  // [0] groups, [1] targets
-  uint32_t *err;
-};
-cudaError_t launch_bucket_merge(const BucketMergeLaunch &L, cudaStream_t s);
 
 // Merge of the compile pipeline (no inter-CTA waits).  The key kernel has put
 // every item into a slot of its bucket (SLOT_CAP slots per bucket; more than

@@ -17,10 +17,6 @@
 //    (CUDAHandlers.hpp:124-139) in FP64; group_scan_kernel and emit_kernel
 //    write the groups to the DEM arrays.  The empty symptom is dropped
 //    (Driver.hpp:185).
-//  * bucket scan + scatter, bucket_merge_kernel: the allocation-free merge of
-//    raw mechanisms (static_merge.cu): one CTA per bucket sorts its items in
-//    shared memory and gets its output slot from a warp-wide decoupled
-//    look-back over the preceding buckets.
 //  * global path, used when a bucket overflows (more than SLOT_CAP mechanisms):
 //    key_all_kernel keys every mechanism on its own; LSD onesweep radix sort of all keys (one
 //    kernel per 8-bit digit, tile ranks by warp match/popc, decoupled
@@ -29,6 +25,7 @@
 #include <cstdint>
 
 #include "device.cuh"
+#include "group.cuh"
 #include "lower.hpp"
 
 namespace gpc {
@@ -40,23 +37,6 @@ __device__ __forceinline__ unsigned long long globaltimer() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
-}
-
-// murmur3 64-bit finaliser (a published bijective mixer).
-__device__ __forceinline__ uint64_t fmix64(uint64_t k) {
-  k ^= k >> 33;
-  k *= 0xff51afd7ed558ccdull;
-  k ^= k >> 33;
-  k *= 0xc4ceb9fe1a85ec53ull;
-  k ^= k >> 33;
-  return k;
-}
-
-// Two independent mixes of (word index, non-zero word value).
-__device__ __forceinline__ ulonglong2 word_hash(uint32_t j, uint64_t v) {
-  const uint64_t jj = (uint64_t)j + 1;
-  return make_ulonglong2(fmix64(v * 0x9E3779B97F4A7C15ull + jj * 0xC2B2AE3D27D4EB4Full),
-                         fmix64(v * 0xD6E8FEB86659FD93ull + jj * 0xA0761D6478BD642Full + 0x8EBC6AF09C88C6E3ull));
 }
 
 __device__ __forceinline__ uint64_t pauli_sel(ulonglong2 s, uint32_t P) {
@@ -93,9 +73,6 @@ __constant__ uint8_t kComp[6][15] = {
      PP(2, 0), PP(2, 1), PP(2, 3), PP(2, 2)},
 };
 #undef PP
-
-// a(1-b) + b(1-a), written as a + b(1-2a): two fused multiply-adds.
-__device__ __forceinline__ double xor_merge(double a, double b) { return fma(b, fma(-2.0, a, 1.0), a); }
 
 // find_circuit by a warp: 32 places per round of loads.
 __device__ __forceinline__ uint32_t find_circuit_warp(const uint32_t *base, uint32_t n, uint32_t x) {
@@ -633,45 +610,6 @@ __global__ void __launch_bounds__(KEY_THREADS) key_all_kernel(KeyLaunch L) {
   if (nonzero && (hx | hy) == 0) atomicOr(L.err, DEV_ERR_COLLISION);  // a non-empty symptom hashed to 0
 }
 
-// Exclusive scan of nb bucket counts (one block); offset[nb] = total.
-__global__ void __launch_bounds__(1024) bucket_scan_kernel(const uint32_t *__restrict__ count,
-                                                           uint32_t *__restrict__ offset, uint32_t nb) {
-  __shared__ uint32_t part[1024];
-  const uint32_t t = threadIdx.x;
-  const uint32_t per = (nb + 1023) / 1024;
-  const uint32_t lo = min(nb, t * per), hi = min(nb, lo + per);
-  uint32_t sum = 0;
-  for (uint32_t i = lo; i < hi; ++i) sum += count[i];
-  part[t] = sum;
-  __syncthreads();
-  for (uint32_t off = 1; off < 1024; off <<= 1) {
-    const uint32_t v = t >= off ? part[t - off] : 0;
-    __syncthreads();
-    part[t] += v;
-    __syncthreads();
-  }
-  uint32_t run = part[t] - sum;
-  for (uint32_t i = lo; i < hi; ++i) {
-    const uint32_t c = count[i];
-    offset[i] = run;
-    run += c;
-  }
-  if (t == 1023) offset[nb] = part[1023];
-}
-
-__global__ void bucket_scatter_kernel(const ulonglong2 *__restrict__ key, uint32_t M, uint32_t shift,
-                                      const uint32_t *__restrict__ offset, uint32_t *__restrict__ cursor,
-                                      ulonglong2 *__restrict__ bkey, uint32_t *__restrict__ bm) {
-  for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
-    const ulonglong2 k = key[m];
-    if ((k.x | k.y) == 0) continue;
-    const uint32_t b = (uint32_t)(k.x >> shift);
-    const uint32_t pos = offset[b] + atomicAdd(cursor + b, 1u);
-    bkey[pos] = k;
-    bm[pos] = m;
-  }
-}
-
 // ---- onesweep radix sort ----------------------------------------------------
 
 // Key i of a sort: every `stride`-th u64 (2: the first halves of 128-bit keys).
@@ -1109,169 +1047,10 @@ __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(MergeLaunch L) {
   }
 }
 
-// ---- bucket sort + merge ---------------------------------------------------
-
-// (key, m) order: key.x, then key.y, then mechanism id.
-__device__ __forceinline__ bool item_less(ulonglong2 a, uint32_t ma, ulonglong2 b, uint32_t mb) {
-  if (a.x != b.x) return a.x < b.x;
-  if (a.y != b.y) return a.y < b.y;
-  return ma < mb;
-}
-
-// Loads a target list as 16-byte vectors (rows are 16-byte aligned).
-__device__ __forceinline__ bool lists_equal(const uint32_t *a, const uint32_t *b, uint32_t n) {
-  const uint4 *va = reinterpret_cast<const uint4 *>(a), *vb = reinterpret_cast<const uint4 *>(b);
-  for (uint32_t k = 0; k * 4 < n; ++k) {
-    const uint4 x = __ldg(va + k), y = __ldg(vb + k);
-    const uint32_t rem = n - k * 4;
-    if (x.x != y.x || (rem > 1 && x.y != y.y) || (rem > 2 && x.z != y.z) || (rem > 3 && x.w != y.w)) return false;
-  }
-  return true;
-}
-
-__global__ void __launch_bounds__(BUCKET_THREADS) bucket_merge_kernel(BucketMergeLaunch L) {
-  constexpr int NT = BUCKET_THREADS;
-  constexpr int NW = NT / 32;
-  __shared__ ulonglong2 sk[BUCKET_CAP];
-  __shared__ uint32_t sm[BUCKET_CAP];
-  __shared__ uint16_t ord[BUCKET_CAP];
-  __shared__ uint32_t sntg[BUCKET_CAP];  // targets of a group starting at a sorted position, else ~0u
-  __shared__ uint2 sexc[BUCKET_CAP];     // exclusive (groups, targets) before each sorted position
-  __shared__ uint32_t wc[NW], wt[NW];
-  __shared__ uint32_t s_b, s_pre_c, s_pre_t;
-  extern __shared__ uint2 sband[];
-  const CircuitDev C = *L.c_dev;
-  const uint32_t w = L.w;
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  for (uint32_t j = threadIdx.x; j < w; j += NT) sband[j] = C.band[j];
-  if (threadIdx.x == 0) s_b = atomicAdd(L.ticket, 1u);
-  __syncthreads();
-  const uint32_t b = s_b;
-  uint32_t n = L.count[b];
-  const uint32_t base = L.offset[b];
-  if (n > (uint32_t)BUCKET_CAP) {
-    if (threadIdx.x == 0) atomicOr(L.err, DEV_FLAG_BIG_BUCKET);
-    n = 0;
-  }
-  for (uint32_t i = threadIdx.x; i < n; i += NT) {
-    sk[i] = L.bkey[base + i];
-    sm[i] = L.bm[base + i];
-  }
-  __syncthreads();
-  // rank sort by (key, m): every key is distinct once m is included
-  for (uint32_t i = threadIdx.x; i < n; i += NT) {
-    const ulonglong2 ki = sk[i];
-    const uint32_t mi = sm[i];
-    uint32_t r = 0;
-    for (uint32_t k = 0; k < n; ++k) r += item_less(sk[k], sm[k], ki, mi) ? 1u : 0u;
-    ord[r] = (uint16_t)i;
-  }
-  __syncthreads();
-  // group heads, collision checks (full target lists), target counts
-  // A caller's list longer than the stride was reported (and cut to the
-  // stride) by the key pass; every read of a count here is cut the same way,
-  // so no list is read past its row.
-  const uint32_t tcap = C.tcap;
-  for (uint32_t s = threadIdx.x; s < n; s += NT) {
-    const uint32_t i = ord[s];
-    const uint32_t m = sm[i];
-    const uint32_t nt = min(__ldg(C.tn + m), tcap);
-    bool head = true;
-    if (s > 0) {
-      const uint32_t ip = ord[s - 1];
-      if (sk[ip].x == sk[i].x && sk[ip].y == sk[i].y) {
-        head = false;
-        const uint32_t mq = sm[ip];
-        if (min(__ldg(C.tn + mq), tcap) != nt ||
-            !lists_equal(C.tl + (size_t)m * tcap, C.tl + (size_t)mq * tcap, nt))
-          atomicOr(L.err, DEV_ERR_COLLISION);
-      }
-    }
-    sntg[s] = head ? nt : ~0u;
-  }
-  __syncthreads();
-  // block-wide exclusive scan of (heads, targets) over sorted positions, NT at a time
-  uint32_t carry_c = 0, carry_t = 0;
-  for (uint32_t r0 = 0; r0 < n; r0 += NT) {
-    const uint32_t s = r0 + threadIdx.x;
-    const uint32_t v = s < n ? sntg[s] : ~0u;
-    const uint32_t c_in = v != ~0u ? 1u : 0u, t_in = v != ~0u ? v : 0u;
-    uint32_t ic = c_in, it = t_in;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, ic, o), bb = __shfl_up_sync(0xFFFFFFFFu, it, o);
-      if (lane >= (uint32_t)o) {
-        ic += a;
-        it += bb;
-      }
-    }
-    if (lane == 31) {
-      wc[warp] = ic;
-      wt[warp] = it;
-    }
-    __syncthreads();
-    uint32_t pc = carry_c, pt = carry_t;
-    for (uint32_t x = 0; x < warp; ++x) {
-      pc += wc[x];
-      pt += wt[x];
-    }
-    if (s < n) sexc[s] = make_uint2(pc + ic - c_in, pt + it - t_in);
-    for (uint32_t x = 0; x < (uint32_t)NW; ++x) {
-      carry_c += wc[x];
-      carry_t += wt[x];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x < 32) {
-    uint32_t pc = 0, pt = 0;
-    warp_lookback(L.status, b, carry_c, carry_t, L.err, kSpinLimitNs, &pc, &pt);
-    if (threadIdx.x == 0) {
-      s_pre_c = pc;
-      s_pre_t = pt;
-      if (b == L.nb - 1) {
-        L.totals[0] = pc + carry_c;
-        L.totals[1] = pt + carry_t;
-        if ((uint64_t)pt + carry_t > L.tg_cap) atomicOr(L.err, DEV_FLAG_TG_OVF);
-      }
-    }
-  }
-  __syncthreads();
-  for (uint32_t s = threadIdx.x; s < n; s += NT) {
-    const uint32_t ntg = sntg[s];
-    if (ntg == ~0u) continue;
-    const uint32_t slot = s_pre_c + sexc[s].x, toff = s_pre_t + sexc[s].y;
-    if (slot >= L.max_groups) continue;  // only after a timed-out look-back
-    const uint32_t i = ord[s];
-    const uint32_t m = sm[i];
-    double p = __ldg(C.mp + m);
-    for (uint32_t s2 = s + 1; s2 < n; ++s2) {
-      const uint32_t i2 = ord[s2];
-      if (sk[i2].x != sk[i].x || sk[i2].y != sk[i].y) break;
-      const double q = __ldg(C.mp + sm[i2]);
-      p = p * (1.0 - q) + q * (1.0 - p);
-    }
-    L.out_prob[slot] = p;
-    L.out_off[slot] = toff;
-    if ((uint64_t)toff + ntg <= L.tg_cap) {
-      const uint4 *src = reinterpret_cast<const uint4 *>(C.tl + (size_t)m * tcap);
-      for (uint32_t k = 0; k * 4 < ntg; ++k) {
-        const uint4 x = __ldg(src + k);
-        const uint32_t o = toff + k * 4, rem = ntg - k * 4;
-        L.out_tg[o] = x.x;
-        if (rem > 1) L.out_tg[o + 1] = x.y;
-        if (rem > 2) L.out_tg[o + 2] = x.z;
-        if (rem > 3) L.out_tg[o + 3] = x.w;
-      }
-    }
-  }
-}
-
 // ---- merge of the compile pipeline ---------------------------------------
 
 constexpr uint32_t GW_WARPS = 8;  // buckets per group/emit block (one warp each)
 constexpr uint32_t kFoldBuckets = 32768;  // most buckets whose places the emission finds itself
-
-__device__ __forceinline__ bool key_eq(ulonglong2 a, ulonglong2 b) { return a.x == b.x && a.y == b.y; }
 
 // Row of an item's later targets: its first mechanism.
 __device__ __forceinline__ const uint32_t *far_targets(const GroupLaunch &L, uint32_t m) {
@@ -1292,153 +1071,24 @@ __device__ __forceinline__ bool slot_lists_equal(const GroupLaunch &L, const Slo
   return n <= inl || lists_equal(far_targets(L, ma), far_targets(L, mb), n - inl);
 }
 
-// What a bucket's grouping holds in shared memory: its items as they were
-// filed, and the sorted order.
-template <uint32_t CAP>
-struct GroupItems {
-  ulonglong2 key[CAP];
-  double p[CAP];
-  uint32_t m[CAP], t[CAP];
-  uint32_t sv[CAP];  // sorted position -> 24 key bits << 8 | item
-  uint8_t ord[CAP];  // sorted position -> item
+// A bucket's groups in its slots.  A group's record: (head mechanism, targets
+// before it in the bucket << 8 | the head's slot) in the tail of slot g, its
+// probability beside it (every slot of the bucket has been read into shared
+// memory, and no list is written over).
+struct SlotRuns {
+  const GroupLaunch &L;
+  Slot *bslot;
+  const uint32_t *m;
+  __device__ __forceinline__ uint32_t count(uint32_t t) const { return t & kSlotCount; }
+  __device__ __forceinline__ bool equal(uint32_t a, uint32_t b, uint32_t n) const {
+    return slot_lists_equal(L, bslot + a, m[a], bslot + b, m[b], n);
+  }
+  __device__ __forceinline__ void group(uint32_t g, uint32_t head, uint32_t before, uint32_t s) const {
+    *reinterpret_cast<uint2 *>(&bslot[g].tail) = make_uint2(m[head], before << 8 | head);
+    if (L.keep) slot_perm(bslot, g)[1] = s;
+  }
+  __device__ __forceinline__ void prob(uint32_t g, double p) const { bslot[g].tail.p = p; }
 };
-
-// Bitonic sort of 32 R words, R per lane: word r * 32 + lane is v[r].
-template <int R>
-__device__ __forceinline__ void sort_words(uint32_t (&v)[R]) {
-  const uint32_t lane = threadIdx.x & 31u;
-#pragma unroll
-  for (int k = 2; k <= 32 * R; k *= 2) {
-#pragma unroll
-    for (int j = k / 2; j > 0; j /= 2) {
-      if (j >= 32) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int q = r ^ (j / 32);
-          if (q > r) {
-            const bool up = (r * 32 & k) == 0;
-            const uint32_t lo = min(v[r], v[q]), hi = max(v[r], v[q]);
-            v[r] = up ? lo : hi;
-            v[q] = up ? hi : lo;
-          }
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, v[r], j);
-          const bool up = k < 32 ? (lane & k) == 0 : (r * 32 & k) == 0;
-          v[r] = ((lane & j) == 0) == up ? min(v[r], o) : max(v[r], o);
-        }
-      }
-    }
-  }
-}
-
-// The DEM's order inside a bucket: top 6 bits of the key's second half, then the key, then the mechanism.
-template <typename G_t>
-__device__ __forceinline__ bool item_before(const G_t &G, uint32_t a, uint32_t b) {
-  const uint32_t ba = (uint32_t)(G.key[a].y >> 58), bb = (uint32_t)(G.key[b].y >> 58);
-  return ba != bb ? ba < bb : item_less(G.key[a], G.m[a], G.key[b], G.m[b]);
-}
-
-// Orders the n <= 32 R items of G: G.ord.  The words sorted are 24 bits of the
-// order's key (6 of the second half, 18 of the first after the bits that all
-// items share) above the item's index: one shuffle and one min/max a step.
-// Items of equal words are then put in mechanism order; when two different
-// keys share a word (a few in 10^6 buckets) every item's place is counted
-// from the full keys instead.
-template <int R, typename G_t>
-__device__ __forceinline__ void order_items(G_t &G, uint32_t n) {
-  const uint32_t lane = threadIdx.x & 31u;
-  constexpr uint32_t ALL = 0xFFFFFFFFu;
-  uint64_t hx[R];
-  uint32_t differ = 0;
-  const uint64_t x0 = G.key[0].x;
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const uint32_t i = r * 32 + lane;
-    hx[r] = i < n ? G.key[i].x : x0;
-    differ |= (uint32_t)((hx[r] ^ x0) >> 32);
-  }
-  differ = __reduce_or_sync(ALL, differ);
-  const uint32_t same = differ ? (uint32_t)__clz(differ) : 32u;  // leading bits all share
-  uint32_t v[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const uint32_t i = r * 32 + lane;
-    v[r] = ALL;
-    if (i < n) v[r] = (uint32_t)(G.key[i].y >> 58) << 26 | ((uint32_t)((hx[r] << same) >> 32) >> 14) << 8 | i;
-  }
-  sort_words<R>(v);
-  bool mixed = false;
-  if constexpr (R == 1) {
-    const uint32_t i = v[0] & 255u;
-    uint32_t m = 0;
-    ulonglong2 k = make_ulonglong2(0, 0);
-    if (lane < n) {
-      m = G.m[i];
-      k = G.key[i];
-    }
-    const uint32_t word = v[0] >> 8, left = __shfl_up_sync(ALL, word, 1);
-    const uint64_t lx = __shfl_up_sync(ALL, k.x, 1), ly = __shfl_up_sync(ALL, k.y, 1);
-    const bool start = lane == 0 || left != word || lane >= n;
-    mixed = !start && (lx != k.x || ly != k.y);
-    const uint32_t starts = __ballot_sync(ALL, start);
-    const uint32_t first = 31u - __clz(starts & (ALL >> (31u - lane)));
-    const uint32_t after = lane == 31u ? 0u : starts >> (lane + 1u);
-    const uint32_t end = after ? lane + (uint32_t)__ffs(after) : 32u;  // the run is lanes [first, end)
-    const uint32_t longest = __reduce_max_sync(ALL, end - first);
-    uint32_t place = first;
-    for (uint32_t o = 1; o < longest; ++o) {
-      const uint32_t a = __shfl_up_sync(ALL, m, o), b = __shfl_down_sync(ALL, m, o);
-      place += (lane >= first + o && a < m ? 1u : 0u) + (lane + o < end && b < m ? 1u : 0u);
-    }
-    if (lane < n) G.ord[place] = (uint8_t)i;
-  } else {
-#pragma unroll
-    for (int r = 0; r < R; ++r) G.sv[r * 32 + lane] = v[r];
-    __syncwarp();
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const uint32_t s = r * 32 + lane;
-      if (s >= n) continue;
-      const uint32_t i = v[r] & 255u, mi = G.m[i];
-      // its run of equal words: the items of smaller mechanisms come before it
-      uint32_t first = s, before = 0;
-      const ulonglong2 ki = G.key[i];
-      while (first > 0) {
-        const uint32_t w = G.sv[first - 1];
-        if ((w ^ v[r]) >> 8) break;
-        mixed |= !key_eq(G.key[w & 255u], ki);
-        before += G.m[w & 255u] < mi ? 1u : 0u;
-        --first;
-      }
-      for (uint32_t q = s + 1; q < n; ++q) {
-        const uint32_t w = G.sv[q];
-        if ((w ^ v[r]) >> 8) break;
-        before += G.m[w & 255u] < mi ? 1u : 0u;
-      }
-      G.ord[first + before] = (uint8_t)i;
-    }
-  }
-  if (__any_sync(ALL, mixed)) {
-    __syncwarp();
-    for (uint32_t i = lane; i < n; i += 32) {
-      uint32_t place = 0;
-      for (uint32_t q = 0; q < n; ++q) place += item_before(G, q, i) ? 1u : 0u;
-      G.ord[place] = (uint8_t)i;
-    }
-  }
-  __syncwarp();
-}
-
-// A group's record: (head mechanism, targets before it in the bucket << 8 | the
-// head's slot) in the tail of slot g; its probability is written beside it.
-__device__ __forceinline__ void put_group(Slot *bslot, uint32_t g, uint32_t m, uint32_t before, uint32_t head, uint32_t s,
-                                          uint32_t keep) {
-  *reinterpret_cast<uint2 *>(&bslot[g].tail) = make_uint2(m, before << 8 | head);
-  if (keep) slot_perm(bslot, g)[1] = s;
-}
 
 // One warp's bucket of n <= CAP items.  Returns (groups, targets).
 template <uint32_t CAP>
@@ -1455,11 +1105,11 @@ __device__ __forceinline__ uint2 group_warp(const GroupLaunch &L, GroupItems<CAP
   }
   __syncwarp();
   if constexpr (CAP > 128) {
-    order_items<CAP / 32>(G, n);
+    order_items<CAP / 32, true>(G, n);
   } else {
-    if (n <= 32) order_items<1>(G, n);
-    else if (n <= 64) order_items<2>(G, n);
-    else order_items<4>(G, n);
+    if (n <= 32) order_items<1, true>(G, n);
+    else if (n <= 64) order_items<2, true>(G, n);
+    else order_items<4, true>(G, n);
   }
   if (L.keep) {  // the saved permutation for the adjoint
     for (uint32_t s = lane; s < n; s += 32) {
@@ -1467,69 +1117,7 @@ __device__ __forceinline__ uint2 group_warp(const GroupLaunch &L, GroupItems<CAP
       slot_perm(bslot, s)[3] = G.t[G.ord[s]] >> 24;  // the mechanisms merged into the item
     }
   }
-  // Groups, 32 sorted positions at a time.  Each group's probability is a
-  // segmented inclusive scan of the XOR-merge over its run: log2(longest run
-  // in the chunk) shuffle steps with every lane busy (FP64 throughput is
-  // scarce on this part), plus the value carried in from the previous chunk.
-  // The scan is a tree, so its rounding differs from a left-to-right fold by
-  // a few ulps; it is deterministic.
-  const uint32_t tcap = L.tcap;
-  uint32_t gcount = 0, tcount = 0;
-  uint32_t carry_head = 0;  // item of the run open at the end of the previous chunk
-  double carry = 0.0;
-  for (uint32_t s0 = 0; s0 < n; s0 += 32) {
-    const uint32_t s = s0 + lane;
-    const bool in = s < n;
-    bool head = false, last = false;  // of its run
-    uint32_t i = 0, nt = 0;
-    double x = 0.0;
-    if (in) {
-      i = G.ord[s];
-      nt = G.t[i] & kSlotCount;
-      x = G.p[i];
-      const ulonglong2 k = G.key[i];
-      head = s == 0 || !key_eq(G.key[G.ord[s - 1]], k);
-      last = s + 1 >= n || !key_eq(G.key[G.ord[s + 1]], k);
-    }
-    const uint32_t hb = __ballot_sync(0xFFFFFFFFu, head);
-    // the run of each position: it starts at lane `seg` of this chunk, or
-    // (seg < 0) continues the run open at the end of the previous chunk
-    const uint32_t le = hb & (0xFFFFFFFFu >> (31u - lane));
-    const int seg = le ? 31 - __clz(le) : -1;
-    const uint32_t seg0 = seg < 0 ? 0u : (uint32_t)seg;
-    {
-      // collision check: every item of a run against the run's head (full target lists)
-      const uint32_t ih = seg < 0 ? carry_head : (uint32_t)G.ord[s0 + seg0];
-      // (a list longer than the rows was flagged by the key pass and the run is redone with wider rows)
-      if (in && !head && nt <= tcap &&
-          ((G.t[ih] & kSlotCount) != nt || !slot_lists_equal(L, bslot + i, G.m[i], bslot + ih, G.m[ih], nt)))
-        atomicOr(L.err, DEV_ERR_COLLISION);
-      carry_head = __shfl_sync(0xFFFFFFFFu, ih, 31);
-    }
-    const uint32_t tv = head ? nt : 0u;
-    uint32_t inc = tv;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-      if (lane >= (uint32_t)o) inc += a;
-    }
-    const uint32_t maxlen = __reduce_max_sync(0xFFFFFFFFu, in ? lane - seg0 + 1 : 0u);
-    for (uint32_t d = 1; d < maxlen; d <<= 1) {
-      const double y = __shfl_up_sync(0xFFFFFFFFu, x, d);
-      if (lane >= d && lane - d >= seg0) x = xor_merge(y, x);
-    }
-    if (seg < 0) x = xor_merge(carry, x);
-    // (every slot of this bucket was read into shared memory, and no list is written over)
-    if (head) put_group(bslot, gcount + __popc(hb & ((1u << lane) - 1u)), G.m[i], tcount + inc - tv, i, s, L.keep);
-    if (last) {  // the run's last item holds its value
-      const uint32_t g = seg < 0 ? gcount - 1u : gcount + __popc(hb & ((1u << seg0) - 1u));
-      bslot[g].tail.p = x;
-    }
-    carry = __shfl_sync(0xFFFFFFFFu, x, 31);
-    gcount += __popc(hb);
-    tcount += __shfl_sync(0xFFFFFFFFu, inc, 31);
-  }
-  return make_uint2(gcount, tcount);
+  return fold_runs(G, n, L.tcap, L.err, SlotRuns{L, bslot, G.m});
 }
 
 // One warp per bucket.  A bucket of more than WARP_CAP items (repeated symptoms)
@@ -1957,20 +1545,6 @@ cudaError_t launch_keys_all(const KeyLaunch &L, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_bucket_scan(const uint32_t *count, uint32_t *offset, uint32_t nb, cudaStream_t s) {
-  bucket_scan_kernel<<<1, 1024, 0, s>>>(count, offset, nb);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_bucket_scatter(const ulonglong2 *key, uint32_t M, uint32_t bucket_bits, const uint32_t *offset,
-                                  uint32_t *cursor, ulonglong2 *bkey, uint32_t *bm, cudaStream_t s) {
-  if (M == 0) return cudaSuccess;
-  uint32_t blocks = (M + 255) / 256;
-  if (blocks > 152u * 16u) blocks = 152u * 16u;
-  bucket_scatter_kernel<<<blocks, 256, 0, s>>>(key, M, 64u - bucket_bits, offset, cursor, bkey, bm);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_group(const GroupLaunch &L, cudaStream_t s) {
   if (L.nb == 0) return cudaSuccess;
   group_kernel<<<(L.nb + GW_WARPS - 1) / GW_WARPS, GW_WARPS * 32, 0, s>>>(L);
@@ -1986,12 +1560,6 @@ cudaError_t launch_scan_emit(const GroupLaunch &L, cudaStream_t s) {
     group_scan_kernel<<<(L.nb + SCAN_TILE - 1) / SCAN_TILE, SCAN_THREADS, 0, s>>>(L);
     emit_kernel<false><<<blocks, GW_WARPS * 32, 0, s>>>(L);
   }
-  return cudaGetLastError();
-}
-
-cudaError_t launch_bucket_merge(const BucketMergeLaunch &L, cudaStream_t s) {
-  if (L.nb == 0) return cudaSuccess;
-  bucket_merge_kernel<<<L.nb, BUCKET_THREADS, (size_t)L.w * sizeof(uint2), s>>>(L);
   return cudaGetLastError();
 }
 
