@@ -478,7 +478,7 @@ struct gpc_driver {
   uint32_t sort_bits = 64;
   bool sort_auto = true;  // no sort_bits given: the global path sorts on as many top key bits as its size needs
   cudaStream_t stream = nullptr;
-  static constexpr int kAux = 4;
+  static constexpr int kAux = 8;  // walk classes side by side (9 classes of a mixed batch: 4 streams 310 us, 8 224; see launch_walks)
   cudaStream_t aux[kAux] = {};
   cudaEvent_t fork_ev = nullptr, join_ev[kAux] = {};
   std::vector<Tape> tapes;
@@ -665,11 +665,17 @@ struct gpc_driver {
   void init_streams() {
     CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&wait_ev, cudaEventBlockingSync | cudaEventDisableTiming));
-    for (auto &a : aux) CK(cudaStreamCreateWithFlags(&a, cudaStreamNonBlocking));
     for (auto &e : ev) CK(cudaEventCreate(&e));
     for (auto &e : tune_ev) CK(cudaEventCreate(&e));
     CK(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming));
-    for (auto &e : join_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  }
+  // The first n auxiliary streams (made when a run first wants them: a single circuit uses one, a batch one
+  // per walk class).
+  void want_aux(uint32_t n) {
+    for (uint32_t a = 0; a < n; ++a) {
+      if (!aux[a]) CK(cudaStreamCreateWithFlags(&aux[a], cudaStreamNonBlocking));
+      if (!join_ev[a]) CK(cudaEventCreateWithFlags(&join_ev[a], cudaEventDisableTiming));
+    }
   }
 
   template <typename T>
@@ -829,12 +835,17 @@ struct gpc_driver {
           gpc::walk_smem_bytes(wc.qpad, wc.chunk_cap, gpc::walk_table_bytes(wc.max_epochs, wc.max_chunks), 2) <=
               227 * 1024 - 1024)
         wc.words = 2;
-      for (uint32_t x = k; x < e; ++x) {
-        const uint32_t i = order[x];
-        circ_words[i] = wc.words;
-        for (uint32_t j = 0; j < tapes[i].w; j += wc.words) walk_items.push_back(make_uint2(i, j));
-        wc.n_items += (tapes[i].w + wc.words - 1) / wc.words;
-      }
+      // the words holding observables walk to the end, the others a few rounds: those first
+      for (const bool obs : {true, false})
+        for (uint32_t x = k; x < e; ++x) {
+          const uint32_t i = order[x];
+          circ_words[i] = wc.words;
+          for (uint32_t j = 0; j < tapes[i].w; j += wc.words)
+            if (((uint64_t)(j + wc.words) * 64 > tapes[i].ndet) == obs) {
+              walk_items.push_back(make_uint2(i, j));
+              ++wc.n_items;
+            }
+        }
       item += wc.n_items;
       L.classes.push_back(wc);
       k = e;
@@ -1103,6 +1114,7 @@ struct gpc_driver {
     }
     plan_segments();
     layout();
+    want_aux(std::min<uint32_t>((uint32_t)std::max<size_t>(1, L.classes.size()), kAux));
     // The stream may still be reading the old arena: finish before regrowing.
     wait();
     uint32_t want_tg = std::max<uint32_t>(1024u, (uint32_t)std::min<uint64_t>(0xFFFFFFF0ull, (uint64_t)L.M * 16));
