@@ -592,6 +592,7 @@ struct gpc_driver {
   // once (the bucket pass, its wait and the second key pass cost 60 us of 250 on 118k mechanisms).
   // Set by a run, forgotten with the circuit.
   bool overflowed = false;
+  bool mixed = false;      // the global sort's top key bits did not tell two of its symptoms apart: sort on 64
   bool lists_off = false;  // symptoms too long for target lists: merge from snapshots
   uint64_t last_d2h = 0;   // bytes copied device -> host by the last fetch
   uint64_t last_h2d = 0;   // bytes copied host -> device by the last prepare (a chunked batch: all of its chunks)
@@ -1074,7 +1075,7 @@ struct gpc_driver {
     if (T.empty()) throw gpc::Error(GPC_ERR_INVALID, "empty batch");
     param = false;
     tcap = 32;
-    lists_off = overflowed = false;
+    lists_off = overflowed = mixed = false;
     if (ops_in_flight) wait();
     tapes.swap(T);
     have_tape = true;
@@ -1093,7 +1094,7 @@ struct gpc_driver {
     if (texts) {
       if (n == 0) throw gpc::Error(GPC_ERR_INVALID, "empty batch");
       tcap = 32;
-      lists_off = overflowed = false;
+      lists_off = overflowed = mixed = false;
       const auto t0 = HostClock::now();
       lower_all(texts, lens, n);
       host_ms[0] = ms_since(t0);
@@ -1478,19 +1479,21 @@ struct gpc_driver {
   }
 
   // Key bits a sort of M mechanisms compares: from the top bit down, as many whole digits as keep the
-  // chance that two different keys agree on them under ~2^-10 (M^2 / 2 pairs), so that the order is the
-  // 64-bit order at 6 passes instead of 8 for ~100k mechanisms.  The merge reports such a pair
-  // (DEV_FLAG_MIXED) and the sort is done again on 64 bits.
+  // chance that two different keys agree on them under 2^-7 (M^2 / 2 pairs), so that the order is the
+  // 64-bit order at 5 passes instead of 8 for ~100k mechanisms (6.8 us each; a chance of 2^-10 would
+  // take the sixth).  The merge reports such a pair (DEV_FLAG_MIXED): the sort is done again on 64 bits,
+  // and the circuit's later runs start there.
   static uint32_t auto_sort_bits(uint32_t M) {
     uint32_t lg = 0;
     while (lg < 32 && (1ull << lg) < M) ++lg;
-    const uint32_t bits = (2 * lg + 9 + gpc::RADIX_BITS - 1) / gpc::RADIX_BITS * gpc::RADIX_BITS;
+    const uint32_t bits = (2 * lg + 6 + gpc::RADIX_BITS - 1) / gpc::RADIX_BITS * gpc::RADIX_BITS;
     return std::min(64u, bits);
   }
   SortKey sorted_on = SortKey::Auto;  // of the last global run
   uint32_t sorted_bits = 64;
 
   void sort_and_merge(SortKey key) {
+    if (key == SortKey::Auto && sort_auto && mixed) key = SortKey::Half;
     const bool full = key == SortKey::Full;
     const uint32_t M = L.M;
     uint32_t *sw = dptr<uint32_t>(L.sort_scr);
@@ -1624,6 +1627,7 @@ struct gpc_driver {
         continue;
       }
       if (used_global && (err & gpc::DEV_FLAG_MIXED) && sorted_on == SortKey::Auto && sort_auto && sorted_bits < 64) {
+        mixed = true;
         CK(cudaMemsetAsync(dptr<char>(L.err), 0, 4, stream));
         run_global(SortKey::Half);
         continue;
@@ -2043,7 +2047,7 @@ struct gpc_driver {
         tapes.clear();
         tapes.push_back(std::move(T[i]));
         tcap = 32;
-        lists_off = overflowed = false;
+        lists_off = overflowed = mixed = false;
         prepare(nullptr, nullptr, 0);
         run();
         std::vector<gpc_dem *> one;

@@ -629,22 +629,6 @@ __global__ void sort_hist_kernel(const uint64_t *__restrict__ keys, uint32_t str
   }
 }
 
-// Exclusive scan of each pass's histogram (one block of RADIX threads per pass).
-__global__ void sort_scan_kernel(uint32_t *__restrict__ hist) {
-  __shared__ uint32_t s[RADIX];
-  uint32_t *h = hist + blockIdx.x * RADIX;
-  const uint32_t t = threadIdx.x;
-  s[t] = h[t];
-  __syncthreads();
-  for (uint32_t off = 1; off < RADIX; off <<= 1) {
-    const uint32_t v = t >= off ? s[t - off] : 0;
-    __syncthreads();
-    s[t] += v;
-    __syncthreads();
-  }
-  h[t] = s[t] - h[t];
-}
-
 constexpr uint32_t ST_AGG = 1u << 30;     // tile aggregate published
 constexpr uint32_t ST_PREFIX = 2u << 30;  // inclusive prefix published
 constexpr uint32_t ST_MASK = (1u << 30) - 1;
@@ -653,21 +637,35 @@ constexpr uint32_t ST_MASK = (1u << 30) - 1;
 // keys are every `stride`-th u64.
 // Bound by the look-back's latency (118k items are 58 tiles, all resident at once, and a pass moves
 // 2.8 MB): a thread loads the status of kLook predecessors before it uses any, so a chain of tiles
-// whose counts are published costs one round trip per kLook tiles (10.1 -> 8.9 us a pass; 32 at a time
-// and tiles of 512 or 1,024 items: 10-11 us).
+// whose counts are published costs one round trip per kLook tiles (10.1 -> 6.8 us a pass; 32 at a time
+// and tiles of 512 or 1,024 items: 10-11 us; of 4,096: 8.0).  Each block scans the pass's histogram
+// itself, while its keys are on the way (a launch of its own for that: 2.5 us).
 constexpr int kLook = 8;
 __global__ void __launch_bounds__(SORT_THREADS) sort_pass_kernel(
     const uint64_t *__restrict__ kin, uint32_t stride, const uint32_t *__restrict__ vin, uint64_t *__restrict__ kout,
-    uint32_t *__restrict__ vout, uint32_t n, uint32_t shift, const uint32_t *__restrict__ gofs,
+    uint32_t *__restrict__ vout, uint32_t n, uint32_t shift, const uint32_t *__restrict__ hist,
     uint32_t *__restrict__ status, uint32_t *__restrict__ tile_ctr, uint32_t *__restrict__ err,
     unsigned long long spin_ns, uint32_t hold_tile0) {
   constexpr int WARPS = SORT_THREADS / 32;
   __shared__ uint32_t wcount[WARPS][RADIX];
   __shared__ uint32_t dbase[RADIX];
+  __shared__ uint32_t s_wtot[RADIX / 32];  // each digit warp's share of the histogram
   __shared__ uint32_t s_tile;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   for (uint32_t i = threadIdx.x; i < WARPS * RADIX; i += SORT_THREADS) (&wcount[0][0])[i] = 0;
   if (threadIdx.x == 0) s_tile = atomicAdd(tile_ctr, 1u);
+  uint32_t gofs = 0;  // the digit's first position: a scan of the pass's histogram, each block its own
+  if (threadIdx.x < RADIX) {
+    const uint32_t own = hist[threadIdx.x];
+    gofs = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, gofs, o);
+      if (lane >= (uint32_t)o) gofs += v;
+    }
+    if (lane == 31) s_wtot[warp] = gofs;
+    gofs -= own;
+  }
   __syncthreads();
   const uint32_t tile = s_tile;
   const uint32_t base = tile * SORT_TILE + warp * (32 * SORT_IPT) + lane;
@@ -703,8 +701,9 @@ __global__ void __launch_bounds__(SORT_THREADS) sort_pass_kernel(
   }
   __syncthreads();
   // per digit: exclusive scan over warps, tile count, look-back
-  {
-    const uint32_t d = threadIdx.x;  // SORT_THREADS == RADIX
+  if (threadIdx.x < RADIX) {
+    const uint32_t d = threadIdx.x;
+    for (uint32_t v = 0; v < warp; ++v) gofs += s_wtot[v];
     uint32_t sum = 0;
 #pragma unroll
     for (int w = 0; w < WARPS; ++w) {
@@ -715,7 +714,7 @@ __global__ void __launch_bounds__(SORT_THREADS) sort_pass_kernel(
     volatile uint32_t *st = status;
     if (tile == 0) {
       if (!hold_tile0) st[d] = ST_PREFIX | sum;  // (held: a test of the waits below)
-      dbase[d] = gofs[d];
+      dbase[d] = gofs;
     } else {
       st[(size_t)tile * RADIX + d] = ST_AGG | sum;
       uint32_t excl = 0;
@@ -747,7 +746,7 @@ __global__ void __launch_bounds__(SORT_THREADS) sort_pass_kernel(
       }
       // (no fence: the status word is all that is passed on)
       st[(size_t)tile * RADIX + d] = ST_PREFIX | (excl + sum);
-      dbase[d] = gofs[d] + excl;
+      dbase[d] = gofs + excl;
     }
   }
   __syncthreads();
@@ -779,32 +778,51 @@ __device__ __forceinline__ unsigned long long ms_pack(uint32_t cnt, uint32_t tg)
 }
 
 // Warp 0 resolves the exclusive prefix of tile `tile` over tiles [0, tile)
-// by decoupled look-back: 32 predecessors per step.  `agg` is this tile's
-// (count, targets) aggregate.  Returns the prefix in every lane.
+// by decoupled look-back, kWide predecessors a lane and step, after the tile
+// published its (count, targets) aggregate with publish_aggregate.  Returns
+// the prefix in every lane.
+constexpr int kWide = 4;
+
+__device__ __forceinline__ void publish_aggregate(unsigned long long *status, uint32_t tile, uint32_t agg_c,
+                                                  uint32_t agg_t) {
+  *(volatile unsigned long long *)(status + tile) = (tile == 0 ? MS_PREFIX : MS_AGG) | ms_pack(agg_c, agg_t);
+}
+
 __device__ __forceinline__ void warp_lookback(unsigned long long *status, uint32_t tile, uint32_t agg_c,
                                               uint32_t agg_t, uint32_t *err, unsigned long long spin_ns,
                                               uint32_t *pre_c, uint32_t *pre_t) {
   const uint32_t lane = threadIdx.x & 31u;
   volatile unsigned long long *st = status;
-  if (tile == 0) {
-    if (lane == 0) st[0] = MS_PREFIX | ms_pack(agg_c, agg_t);
-    *pre_c = 0;
-    *pre_t = 0;
-    return;
-  }
-  if (lane == 0) st[tile] = MS_AGG | ms_pack(agg_c, agg_t);
   uint32_t ec = 0, et = 0;
   int32_t base = (int32_t)tile - 1;
   unsigned long long t0 = 0;
-  while (base >= 0) {
-    const int32_t idx = base - (int32_t)lane;
-    const unsigned long long s = idx >= 0 ? st[idx] : (MS_PREFIX | 0ull);
-    const uint32_t flag = (uint32_t)(s >> 62);
-    const uint32_t ready = __ballot_sync(0xFFFFFFFFu, flag != 0);
-    const uint32_t pref = __ballot_sync(0xFFFFFFFFu, flag == 2u);
-    // lanes up to (and including) the nearest prefix must all be ready
-    const uint32_t need = pref ? ((pref & (0u - pref)) << 1) - 1u : 0xFFFFFFFFu;
-    if ((ready & need) != need) {
+  bool done = base < 0;
+  while (!done) {
+    unsigned long long s[kWide];
+#pragma unroll
+    for (int k = 0; k < kWide; ++k) {
+      const int32_t idx = base - k * 32 - (int32_t)lane;
+      s[k] = idx >= 0 ? st[idx] : (MS_PREFIX | 0ull);
+    }
+    uint32_t c = 0, t = 0;
+    int used = 0;
+#pragma unroll
+    for (int k = 0; k < kWide; ++k) {
+      const uint32_t flag = (uint32_t)(s[k] >> 62);
+      const uint32_t ready = __ballot_sync(0xFFFFFFFFu, flag != 0);
+      const uint32_t pref = __ballot_sync(0xFFFFFFFFu, flag == 2u);
+      // lanes up to (and including) the nearest prefix must all be ready
+      const uint32_t need = pref ? ((pref & (0u - pref)) << 1) - 1u : 0xFFFFFFFFu;
+      if (used == k && !done && (ready & need) == need) {
+        used = k + 1;
+        done = pref != 0;
+        if ((need >> lane) & 1u) {
+          c += (uint32_t)((s[k] >> 32) & 0x3FFFFFFFu);
+          t += (uint32_t)s[k];
+        }
+      }
+    }
+    if (used == 0) {
       if (t0 == 0) t0 = globaltimer();
       else if (globaltimer() - t0 > spin_ns) {
         if (lane == 0) atomicOr(err, DEV_ERR_TIMEOUT);
@@ -813,19 +831,17 @@ __device__ __forceinline__ void warp_lookback(unsigned long long *status, uint32
       continue;
     }
     t0 = 0;
-    uint32_t c = (need >> lane) & 1u ? (uint32_t)((s >> 32) & 0x3FFFFFFFu) : 0u;
-    uint32_t t = (need >> lane) & 1u ? (uint32_t)s : 0u;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
-      t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
-    }
     ec += c;
     et += t;
-    if (pref) break;
-    base -= 32;
+    base -= used * 32;
   }
-  if (lane == 0) st[tile] = MS_PREFIX | ms_pack(ec + agg_c, et + agg_t);  // (no fence: the word is all that is passed on)
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    ec += __shfl_xor_sync(0xFFFFFFFFu, ec, o);
+    et += __shfl_xor_sync(0xFFFFFFFFu, et, o);
+  }
+  // (no fence: the word is all that is passed on)
+  if (lane == 0 && tile != 0) st[tile] = MS_PREFIX | ms_pack(ec + agg_c, et + agg_t);
   *pre_c = ec;
   *pre_t = et;
 }
@@ -842,11 +858,15 @@ __device__ __forceinline__ uint64_t symptom_mask(const CircuitDev &C, uint64_t d
   return b;
 }
 
-// One thread per sorted position.  A run's probability is a segmented scan of the XOR-merge over its
-// positions: a tree inside a tile, and a run still open at its tile's end is followed by the whole
-// block, MERGE_THREADS positions at a time (one thread following its run alone waited for three
-// dependent loads per position: 503 us for the 118k mechanisms of a circuit whose runs are 300 long,
-// against 26 us).  The tree is deterministic and differs from a left-to-right fold by a few ulps.
+// One thread per sorted position; one warp folds the tile's runs.  FP64 runs at 2 lanes a cycle and SM,
+// so lanes that fold nothing new are what a fold must avoid: with 8 positions a lane and then a segmented
+// scan over the lanes, a tile of 256 costs 13 warp-wide merges (every warp scanning its 32 positions: 40,
+// and the carries as many again).  A run still open at its tile's end is read on by the block,
+// MERGE_THREADS positions at a time, and folded by the same warp; the tile's counts are published before
+// that and its predecessors' read after, 128 a step.  118k mechanisms in runs of 300: 26 -> 17.5 us
+// (one thread following its run alone: 503).  What is left is a chain of ~10 dependent loads (4.5k
+// cycles to the keys and symptoms, 4k in the open run, 3k in the look-back).  The tree is deterministic
+// and differs from a left-to-right fold by a few ulps.
 __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(MergeLaunch L) {
   constexpr uint32_t NW = MERGE_THREADS / 32;
   const CircuitDev C = *L.c_dev;
@@ -854,12 +874,12 @@ __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(MergeLaunch L) {
   __shared__ uint32_t s_tile;
   __shared__ uint32_t wsum_c[MERGE_THREADS / 32], wsum_t[MERGE_THREADS / 32];
   __shared__ uint32_t s_pre_c, s_pre_t;
-  __shared__ double s_p[MERGE_THREADS];        // folded probability of the run that starts at a position
-  __shared__ double s_tail[NW], s_more[NW];    // each warp's open run; a chunk past the tile
-  __shared__ uint32_t s_last[NW];              // each warp's last run start (position in the tile + 1; 0: none)
-  __shared__ uint32_t s_first[NW];             // a run starts at the warp's first position
-  __shared__ ulonglong2 s_key;                 // the key of the run open at the tile's end
-  __shared__ uint32_t s_open;                  // its first position in the tile (MERGE_THREADS: none follows)
+  constexpr uint32_t FP = MERGE_THREADS / 32;   // positions a lane of the folding warp takes
+  __shared__ double s_q[32 * (FP + 1)];         // the positions' probabilities, a padded row per folding lane
+  __shared__ double s_p[MERGE_THREADS];         // folded probability of the run that starts at a position
+  __shared__ uint32_t s_head[NW];               // where runs start, a bit per position
+  __shared__ ulonglong2 s_key;                  // the key of the run open at the tile's end
+  __shared__ uint32_t s_open;                   // its first position in the tile (MERGE_THREADS: none follows)
   const uint32_t w = L.w;
   for (uint32_t j = threadIdx.x; j < w; j += blockDim.x) sband[j] = C.band[j];
   if (threadIdx.x == 0) s_tile = atomicAdd(L.tile_ctr, 1u);
@@ -883,37 +903,36 @@ __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(MergeLaunch L) {
     k = L.key[m];
     q = __ldg(C.mp + m);
     const uint64_t d = __ldg(C.mdesc + m);
-    const uint32_t mp = i > 0 ? L.perm[i - 1] : 0u;
-    if (i > 0 && mp < n) {
+    const uint32_t mp = i > 0 ? L.perm[i - 1] : n;
+    uint64_t dp = 0;
+    if (mp < n) {
       const ulonglong2 kp = L.key[mp];
-      if (kp.x == k.x && kp.y == k.y) {
-        newgroup = false;
-        const uint64_t dp = __ldg(C.mdesc + mp);
-        // the full symptoms, compared on the words either can be non-zero in
-        bool diff = false;
-        for (uint32_t mi = 0; mi < C.mw && !diff; ++mi)
-          for (uint64_t bits = symptom_mask(C, d, mi) | symptom_mask(C, dp, mi); bits && !diff; bits &= bits - 1) {
-            const uint32_t j = mi * 64u + (uint32_t)(__ffsll((long long)bits) - 1);
-            diff = j < w && symptom_word(C, d, j, sband[j]) != symptom_word(C, dp, j, sband[j]);
-          }
-        if (diff) atomicOr(L.err, DEV_ERR_COLLISION);
-      } else if (((L.sortkey[i] ^ L.sortkey[i - 1]) & L.sort_mask) == 0 && L.sort_mask) {
-        atomicOr(L.err, DEV_FLAG_MIXED);
-      }
+      dp = __ldg(C.mdesc + mp);
+      newgroup = kp.x != k.x || kp.y != k.y;
+      if (newgroup && ((L.sortkey[i] ^ L.sortkey[i - 1]) & L.sort_mask) == 0 && L.sort_mask) atomicOr(L.err, DEV_FLAG_MIXED);
     }
-    const bool empty = (k.x | k.y) == 0;
-    if (newgroup) {
-      // a non-empty symptom hashed to zero is a collision; a head counts its targets
-      bool nonzero = false;
-      for (uint32_t mi = 0; mi < C.mw; ++mi)
-        for (uint64_t bits = symptom_mask(C, d, mi); bits; bits &= bits - 1) {
-          const uint32_t j = mi * 64u + (uint32_t)(__ffsll((long long)bits) - 1);
-          const uint32_t c = j < w ? __popcll(symptom_word(C, d, j, sband[j])) : 0u;
-          nonzero |= c != 0;
-          ntg += c;
+    // One loop for both kinds of position, two words at a time: a head counts its targets, another one's
+    // full symptom is compared with its predecessor's on the words either can be non-zero in.
+    bool diff = false;
+    for (uint32_t mi = 0; mi < C.mw; ++mi)
+      for (uint64_t bits = symptom_mask(C, d, mi) | (newgroup ? 0ull : symptom_mask(C, dp, mi)); bits;) {
+        const uint32_t j0 = mi * 64u + (uint32_t)(__ffsll((long long)bits) - 1);
+        bits &= bits - 1;
+        const uint32_t j1 = bits ? mi * 64u + (uint32_t)(__ffsll((long long)bits) - 1) : w;
+        bits &= bits - 1;
+        const uint64_t a0 = j0 < w ? symptom_word(C, d, j0, sband[j0]) : 0ull;
+        const uint64_t a1 = j1 < w ? symptom_word(C, d, j1, sband[j1]) : 0ull;
+        if (newgroup) {
+          ntg += __popcll(a0) + __popcll(a1);
+        } else {
+          const uint64_t b0 = j0 < w ? symptom_word(C, dp, j0, sband[j0]) : 0ull;
+          const uint64_t b1 = j1 < w ? symptom_word(C, dp, j1, sband[j1]) : 0ull;
+          diff |= a0 != b0 || a1 != b1;
         }
-      if (empty && nonzero) atomicOr(L.err, DEV_ERR_COLLISION);
-    }
+      }
+    const bool empty = (k.x | k.y) == 0;
+    // (a non-empty symptom hashed to zero is a collision too)
+    if (diff || (newgroup && empty && ntg)) atomicOr(L.err, DEV_ERR_COLLISION);
     head = newgroup && !empty;
     if (!head) ntg = 0;
   }
@@ -933,42 +952,13 @@ __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(MergeLaunch L) {
     wsum_c[warp] = c_inc;
     wsum_t[warp] = t_inc;
   }
-  __syncthreads();
-  // runs inside the warp: the segmented inclusive scan of q
+  const uint32_t qi = threadIdx.x / FP * (FP + 1) + threadIdx.x % FP;
+  s_q[qi] = q;
   const uint32_t hb = __ballot_sync(0xFFFFFFFFu, newgroup);
-  const uint32_t le = hb & (0xFFFFFFFFu >> (31u - lane));
-  const uint32_t seg0 = le ? 31u - __clz(le) : 0u;
-  double x = q;
-#pragma unroll
-  for (uint32_t o = 1; o < 32; o <<= 1) {
-    const double y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-    if (lane >= o && lane - o >= seg0) x = xor_merge(y, x);
-  }
-  if (lane == 31) {
-    s_tail[warp] = x;
-    s_last[warp] = hb ? warp * 32u + 32u - __clz(hb) : 0u;
-    s_first[warp] = hb & 1u;
-  }
+  if (lane == 0) s_head[warp] = hb;
+  if (threadIdx.x == MERGE_THREADS - 1) s_key = k;
   __syncthreads();
-  {
-    // the run open at the warp's start: its value over the warps before, and where it starts (0: before the tile)
-    double carry = 0.0;
-    uint32_t open = 0;
-    for (uint32_t v = 0; v < warp; ++v) {
-      carry = s_last[v] ? s_tail[v] : xor_merge(carry, s_tail[v]);
-      open = s_last[v] ? s_last[v] : open;
-    }
-    if (le == 0) x = xor_merge(carry, x);
-    else open = warp * 32u + seg0 + 1u;
-    const bool last = lane == 31 ? threadIdx.x == MERGE_THREADS - 1 || s_first[warp + 1]
-                                 : ((hb >> (lane + 1u)) & 1u) != 0u;
-    // (the run's last position in the tile: positions past n start runs of their own)
-    if (last && open) s_p[open - 1] = x;
-    if (threadIdx.x == MERGE_THREADS - 1) {
-      s_open = open && i < n && (k.x | k.y) != 0 ? open - 1u : MERGE_THREADS;
-      s_key = k;
-    }
-  }
+  uint32_t agg_c = 0, agg_t = 0;  // the tile's, in warp 0
   if (threadIdx.x < 32) {
     const uint32_t wc = lane < NW ? wsum_c[lane] : 0u, wt = lane < NW ? wsum_t[lane] : 0u;
     uint32_t ec = wc, et = wt;
@@ -985,46 +975,92 @@ __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(MergeLaunch L) {
       wsum_c[lane] = ec - wc;
       wsum_t[lane] = et - wt;
     }
+    if (lane == 0) publish_aggregate(L.status, tile, ac, at);
+    agg_c = ac;
+    agg_t = at;
+  } else if (warp == 1) {
+    // lane l folds positions [FP l, FP l + FP); a run that starts there goes on over the lanes after
+    const uint32_t h = (s_head[lane * FP / 32] >> (lane * FP % 32)) & ((1u << FP) - 1u);
+    double acc = 0.0, lead = 0.0;  // the run open after the lane's positions; what precedes its first start
+    uint32_t cur = MERGE_THREADS;
+#pragma unroll
+    for (uint32_t e = 0; e < FP; ++e) {
+      const double v = s_q[lane * (FP + 1) + e];
+      if ((h >> e) & 1u) {
+        if (cur < MERGE_THREADS) s_p[cur] = acc;
+        else lead = acc;
+        cur = lane * FP + e;
+        acc = v;
+      } else {
+        acc = xor_merge(acc, v);
+      }
+    }
+    const uint32_t starts = __ballot_sync(0xFFFFFFFFu, h != 0);
+    // x: the fold from the lane's first position to the next start
+    const uint32_t stop = starts >> lane ? lane + (uint32_t)__ffs((int)(starts >> lane)) - 1u : 31u;
+    double x = h ? lead : acc;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+      const double y = __shfl_down_sync(0xFFFFFFFFu, x, o);
+      if (lane + o <= stop) x = xor_merge(x, y);
+    }
+    const double y = __shfl_down_sync(0xFFFFFFFFu, x, 1);
+    if (h) s_p[cur] = lane == 31 ? acc : xor_merge(acc, y);
+    const uint32_t last = starts ? 31u - (uint32_t)__clz((int)starts) : 0u;  // the lane of the tile's last start
+    if (lane == last) {
+      const bool full = (uint64_t)(tile + 1) * MERGE_THREADS <= n;
+      s_open = h && full && (s_key.x | s_key.y) != 0 ? cur : MERGE_THREADS;
+    }
+  }
+  __syncthreads();
+  // A run still open at the tile's end: the block reads its positions in the tiles after, warp 1 folds them.
+  if (s_open < MERGE_THREADS) {
+    const ulonglong2 ko = s_key;
+    double acc = 0.0;
+    uint32_t i2 = (tile + 1) * MERGE_THREADS + threadIdx.x;
+    for (uint32_t m2 = i2 < n ? L.perm[i2] : n;;) {
+      double q2 = 0.0;
+      bool same = false;
+      i2 += MERGE_THREADS;
+      const uint32_t next = i2 < n ? L.perm[i2] : n;
+      if (m2 < n) {  // (past n: the end, or a stale entry after a timed-out sort pass)
+        const ulonglong2 k2 = L.key[m2];
+        const double p2 = __ldg(C.mp + m2);
+        same = k2.x == ko.x && k2.y == ko.y;
+        if (same) q2 = p2;
+      }
+      m2 = next;
+      s_q[qi] = q2;
+      const int all = __syncthreads_and(same ? 1 : 0);
+      if (warp == 1) {
+#pragma unroll
+        for (uint32_t e = 0; e < FP; ++e) acc = xor_merge(acc, s_q[lane * (FP + 1) + e]);
+      }
+      if (!all) break;
+      __syncthreads();
+    }
+    if (warp == 1) {
+#pragma unroll
+      for (uint32_t o = 16; o > 0; o >>= 1) acc = xor_merge(acc, __shfl_down_sync(0xFFFFFFFFu, acc, o));
+      if (lane == 0) s_p[s_open] = xor_merge(s_p[s_open], acc);
+    }
+  }
+  // (the predecessors' aggregates are published by now)
+  if (threadIdx.x < 32) {
     uint32_t pc = 0, pt = 0;
-    warp_lookback(L.status, tile, ac, at, L.err, L.spin_ns, &pc, &pt);
+    warp_lookback(L.status, tile, agg_c, agg_t, L.err, L.spin_ns, &pc, &pt);
     if (lane == 0) {
       s_pre_c = pc;
       s_pre_t = pt;
       if (tile == ntiles - 1) {
-        L.totals[0] = pc + ac;
-        L.totals[1] = pt + at;
-        if (pc + ac <= n) L.out_off[pc + ac] = pt + at;  // the closing offset (past n only after a timed-out look-back)
-        if (pt + at > L.tg_cap) atomicOr(L.err, DEV_FLAG_TG_OVF);
+        L.totals[0] = pc + agg_c;
+        L.totals[1] = pt + agg_t;
+        if (pc + agg_c <= n) L.out_off[pc + agg_c] = pt + agg_t;  // the closing offset (past n only after a timed-out look-back)
+        if (pt + agg_t > L.tg_cap) atomicOr(L.err, DEV_FLAG_TG_OVF);
       }
     }
   }
   __syncthreads();
-  // a run still open at the tile's end: the block folds its positions in the tiles after
-  if (s_open < MERGE_THREADS) {
-    const ulonglong2 ko = s_key;
-    for (uint32_t i2 = (tile + 1) * MERGE_THREADS + threadIdx.x;; i2 += MERGE_THREADS) {
-      double q2 = 0.0;
-      bool same = false;
-      const uint32_t m2 = i2 < n ? L.perm[i2] : n;
-      if (m2 < n) {  // (past n: the end, or a stale entry after a timed-out sort pass)
-        const ulonglong2 k2 = L.key[m2];
-        same = k2.x == ko.x && k2.y == ko.y;
-        if (same) q2 = __ldg(C.mp + m2);
-      }
-#pragma unroll
-      for (uint32_t o = 16; o > 0; o >>= 1) q2 = xor_merge(q2, __shfl_down_sync(0xFFFFFFFFu, q2, o));
-      if (lane == 0) s_more[warp] = q2;
-      const int all = __syncthreads_and(same ? 1 : 0);
-      if (threadIdx.x == 0) {
-        double p = s_p[s_open];
-#pragma unroll
-        for (uint32_t v = 0; v < NW; ++v) p = xor_merge(p, s_more[v]);
-        s_p[s_open] = p;
-      }
-      __syncthreads();
-      if (!all) break;
-    }
-  }
   if (!head) return;
   const uint32_t slot = s_pre_c + wsum_c[warp] + c_inc - c_in;
   if (slot >= n) return;  // only after a timed-out look-back
@@ -1580,7 +1616,6 @@ cudaError_t launch_sort(const uint64_t *first, uint32_t stride, bool index_vals,
   uint32_t hb = (n + 1023) / 1024;
   if (hb > 152u * 4u) hb = 152u * 4u;
   sort_hist_kernel<<<hb, 1024, 0, s>>>(first, stride, n, shift0, passes, scr.hist);
-  sort_scan_kernel<<<passes, RADIX, 0, s>>>(scr.hist);
   uint64_t *ki = keys, *ko = keys_alt;
   uint32_t *vi = vals, *vo = vals_alt;
   for (uint32_t p = 0; p < passes; ++p) {

@@ -65,3 +65,27 @@ def test_two_symptoms_that_agree_on_the_sorted_bits():
     dem = gp.get_driver(text, global_sort=True).compile(text)
     assert {a, b} <= {t for t, _ in dem.errors()}
     _check(dem, text)
+
+
+def test_later_runs_of_such_a_circuit_sort_on_64_bits():
+    """The next run of that circuit starts on 64 bits: same result; the driver's next circuit is not bound by it."""
+    triples = list(itertools.combinations(range(64), 3))
+    v = np.array([sum(1 << t for t in c) for c in triples], dtype=np.uint64)
+    top = _top_bits(v, 24)
+    order = np.argsort(top, kind="stable")
+    k = int(np.flatnonzero(top[order][1:] == top[order][:-1])[0])
+    a, b = triples[order[k]], triples[order[k + 1]]
+    text = "R " + " ".join(map(str, range(66))) + "\n" + "X_ERROR(0.001) 64 65\nTICK\n" * 10
+    text += "".join(f"CX 64 {t}\n" for t in a) + "".join(f"CX 65 {t}\n" for t in b)
+    text += "X_ERROR(0.002) " + " ".join(map(str, range(64))) + "\nM " + " ".join(map(str, range(64))) + "\n"
+    text += "".join(f"DETECTOR rec[-{64 - q}]\n" for q in range(64))
+    drv = gp.get_driver(text, global_sort=True)
+    drv.prepare(text)
+    dems = []
+    for _ in range(3):
+        drv.run_device()
+        dems.append(drv.fetch())
+    _check(dems[0], text)
+    assert dems[0] == dems[1] == dems[2]
+    small = "R 0 1\nX_ERROR(0.01) 0\nX_ERROR(0.02) 1\nM 0 1\nDETECTOR rec[-1]\nDETECTOR rec[-2]\n"
+    _check(drv.compile(small), small)
