@@ -519,9 +519,15 @@ struct gpc_driver {
   cudaEvent_t ev[5] = {};
   cudaEvent_t tune_ev[2] = {};  // the autotuner's timing of whole runs
   // last run's global-path sort result
-  uint32_t *perm_sorted = nullptr;
-  uint64_t *sk_sorted = nullptr;
-  uint64_t sort_mask = ~0ull;
+  enum class SortKey { Auto, Half, Full };  // sort_bits (or as many as the size needs) / 64 bits / 128 bits
+  struct Sorted {  // what the last global sort left, read by the merge and its reruns
+    uint32_t *perm = nullptr;
+    uint64_t *key = nullptr;
+    uint64_t mask = ~0ull;
+    SortKey on = SortKey::Auto;
+    uint32_t bits = 64;
+  };
+  Sorted sorted, graph_sorted;  // graph_sorted: of the sort in the captured graph
   bool force_global = false;  // test option: skip the bucket path (single circuits)
   uint32_t walk_qpt = 0;      // qubits per walk thread (0: chosen per circuit)
   uint32_t walk_words = 0;    // detector words per walk CTA (0: two in batches, one for a single circuit)
@@ -1191,9 +1197,12 @@ struct gpc_driver {
     sizes.known = false;
     const bool single_global = global_plan();
     if (ncirc() == 1 && overflowed && !force_global && !lists_off) ++fallbacks[1];
-    // (a graph with the stage events is another graph)
-    const uint64_t sig = cfg_sig ^ (stage_timing ? 0x9e3779b97f4a7c15ull : 0ull);
-    const bool graphable = use_graph && !single_global && ((graph_exec && graph_sig == sig) || last_run_sig == sig);
+    // (a graph with the stage events is another graph, and so is the one of the global path, which a run
+    // of the prepared circuit can turn to)
+    const uint64_t sig = cfg_sig ^ (stage_timing ? 0x9e3779b97f4a7c15ull : 0ull) ^
+                         (single_global ? 0xd1b54a32d192ed03ull : 0ull) ^ (mixed ? 0x8cb92ba72f3d8dd7ull : 0ull);
+    // (a run that a test holds a tile of is never captured)
+    const bool graphable = use_graph && !(single_global && hold_runs) && ((graph_exec && graph_sig == sig) || last_run_sig == sig);
     last_run_sig = sig;
     if (graphable && graph_sig != sig) drop_graph();
     if (graphable && !graph_exec) {
@@ -1209,12 +1218,18 @@ struct gpc_driver {
         throw;
       }
       capturing = false;
+      graph_sorted = sorted;
       CK(cudaStreamEndCapture(stream, &graph));
       CK(cudaGraphInstantiate(&graph_exec, graph, 0));
       graph_sig = sig;
     }
-    if (graphable) CK(cudaGraphLaunch(graph_exec, stream));
-    else enqueue();
+    if (graphable) {
+      CK(cudaGraphLaunch(graph_exec, stream));
+      used_global = single_global;
+      if (single_global) sorted = graph_sorted;  // (a rerun of the sort may have left another)
+    } else {
+      enqueue();
+    }
     ran = true;
     timed_run = stage_timing;
   }
@@ -1470,7 +1485,6 @@ struct gpc_driver {
 
   // Global path (single circuit): sort every mechanism (on sort_bits, or all
   // 128 bits) and merge from the snapshots.
-  enum class SortKey { Auto, Half, Full };  // sort_bits (or as many as the size needs) / 64 bits / 128 bits
   void run_global(SortKey full) {
     used_global = true;
     CK(cudaMemsetAsync(dptr<char>(L.gzero), 0, L.gzero_bytes, stream));
@@ -1489,9 +1503,6 @@ struct gpc_driver {
     const uint32_t bits = (2 * lg + 6 + gpc::RADIX_BITS - 1) / gpc::RADIX_BITS * gpc::RADIX_BITS;
     return std::min(64u, bits);
   }
-  SortKey sorted_on = SortKey::Auto;  // of the last global run
-  uint32_t sorted_bits = 64;
-
   void sort_and_merge(SortKey key) {
     if (key == SortKey::Auto && sort_auto && mixed) key = SortKey::Half;
     const bool full = key == SortKey::Full;
@@ -1511,8 +1522,6 @@ struct gpc_driver {
     bool alt = false;
     const uint32_t bits = key != SortKey::Auto ? 64u : sort_auto ? auto_sort_bits(M) : sort_bits;
     const uint32_t shift0 = key == SortKey::Auto && sort_auto ? 64u - bits : 0u;
-    sorted_on = key;
-    sorted_bits = bits;
     CK(gpc::launch_sort(dptr<uint64_t>(L.key), 2, true, k0, k1, p0, p1, M, shift0, bits, s1, stream, &alt));
     uint64_t *ks = alt ? k1 : k0;
     uint32_t *ps = alt ? p1 : p0;
@@ -1527,9 +1536,8 @@ struct gpc_driver {
       ks = alt2 ? hk_alt : hk;
       ps = alt2 ? ps_alt : ps;
     }
-    perm_sorted = ps;
-    sk_sorted = ks;
-    sort_mask = full ? 0ull : (bits >= 64 ? ~0ull : ((1ull << bits) - 1) << shift0);
+    const uint64_t mask = full ? 0ull : (bits >= 64 ? ~0ull : ((1ull << bits) - 1) << shift0);
+    sorted = Sorted{ps, ks, mask, key, bits};
     rec(3);
     launch_merge_now();
     rec(4);
@@ -1539,9 +1547,9 @@ struct gpc_driver {
     gpc::MergeLaunch ml{};
     ml.c_dev = dptr<CircuitDev>(L.cdev);
     ml.w = tapes[0].w;
-    ml.perm = perm_sorted;
-    ml.sortkey = sk_sorted;
-    ml.sort_mask = sort_mask;
+    ml.perm = sorted.perm;
+    ml.sortkey = sorted.key;
+    ml.sort_mask = sorted.mask;
     ml.key = dptr<ulonglong2>(L.key);
     ml.n = L.M;
     ml.out_prob = dptr<double>(L.out_prob);
@@ -1626,7 +1634,7 @@ struct gpc_driver {
         run_global(SortKey::Auto);
         continue;
       }
-      if (used_global && (err & gpc::DEV_FLAG_MIXED) && sorted_on == SortKey::Auto && sort_auto && sorted_bits < 64) {
+      if (used_global && (err & gpc::DEV_FLAG_MIXED) && sorted.on == SortKey::Auto && sort_auto && sorted.bits < 64) {
         mixed = true;
         CK(cudaMemsetAsync(dptr<char>(L.err), 0, 4, stream));
         run_global(SortKey::Half);

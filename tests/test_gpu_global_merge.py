@@ -89,3 +89,24 @@ def test_later_runs_of_such_a_circuit_sort_on_64_bits():
     assert dems[0] == dems[1] == dems[2]
     small = "R 0 1\nX_ERROR(0.01) 0\nX_ERROR(0.02) 1\nM 0 1\nDETECTOR rec[-1]\nDETECTOR rec[-2]\n"
     _check(drv.compile(small), small)
+
+
+@pytest.mark.parametrize("forced", [False, True])
+@pytest.mark.parametrize("copies", [300, 4000])
+def test_repeated_runs_take_a_graph(forced, copies):
+    """Runs of a prepared circuit on the global path (the third and later ones replay a graph), then another
+    circuit of the same driver and the first one again."""
+    def text(p):
+        t = "R 0 1 2 3\n" + f"X_ERROR({p}) 0\nTICK\n" * copies + "DEPOLARIZE2(0.001) 0 2 1 3\nM 0 1 2 3\n"
+        return t + "".join(f"DETECTOR rec[-{k}]\n" for k in range(1, 5))
+    drv = gp.get_driver(text(0.0001), global_sort=forced)
+    for p in (0.0001, 0.0002, 0.0001):  # the same sizes: one graph serves them all
+        drv.prepare(text(p))
+        dems = []
+        for _ in range(5):
+            drv.run_device()
+            dems.append(drv.fetch())
+        _check(dems[0], text(p))
+        assert all(d == dems[0] for d in dems)
+    small = "R 0\nX_ERROR(0.01) 0\nM 0\nDETECTOR rec[-1]\n"
+    _check(drv.compile(small), small)
