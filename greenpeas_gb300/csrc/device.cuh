@@ -252,7 +252,11 @@ struct GroupLaunch {
   uint32_t n_circ;
   uint2 *cout;              // [n_circ] (first slot, first target) of each circuit's output
   uint32_t *err;
+  uint32_t *host_res;       // one circuit: [flags, groups, targets] in page-locked host memory, written by the
+                            // emission where emit_folds() (else the host copies them)
 };
+constexpr uint32_t kFoldBuckets = 32768;  // most buckets whose places the emission finds itself
+inline bool emit_folds(uint32_t nb) { return nb <= kFoldBuckets; }
 cudaError_t launch_group(const GroupLaunch &L, cudaStream_t s);
 
 // ---- noise-rate gradients (single circuit) ----------------------------------

@@ -515,6 +515,7 @@ struct gpc_driver {
   AllocCounter alloc_ctr;
   DevBuf arena{nullptr, 0, &alloc_ctr}, tgbuf{nullptr, 0, &alloc_ctr};
   HostBuf pin_in, pin_out;
+  HostBuf pin_res;  // a single circuit's [flags, groups, targets], written by its emission
   uint32_t tg_cap = 0;
   cudaEvent_t ev[5] = {};
   cudaEvent_t tune_ev[2] = {};  // the autotuner's timing of whole runs
@@ -633,6 +634,7 @@ struct gpc_driver {
     tgbuf.release();
     pin_in.release();
     pin_out.release();
+    pin_res.release();
     for (auto &e : ev)
       if (e) cudaEventDestroy(e);
     for (auto &e : tune_ev)
@@ -675,6 +677,7 @@ struct gpc_driver {
     for (auto &e : ev) CK(cudaEventCreate(&e));
     for (auto &e : tune_ev) CK(cudaEventCreate(&e));
     CK(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming));
+    pin_res.ensure(16);
   }
   // The first n auxiliary streams (made when a run first wants them: a single circuit uses one, a batch one
   // per walk class).
@@ -1480,6 +1483,7 @@ struct gpc_driver {
     gl.n_circ = ncirc();
     gl.cout = dptr<uint2>(L.cout);
     gl.err = dptr<uint32_t>(L.err);
+    gl.host_res = ncirc() == 1 ? static_cast<uint32_t *>(pin_res.p) : nullptr;
     return gl;
   }
 
@@ -1592,15 +1596,23 @@ struct gpc_driver {
   Finish finish(uint32_t *groups, uint32_t *targets) {
     bool did_full = false;
     for (int attempt = 0; attempt < 8; ++attempt) {
-      // one copy of [cout, flags, totals], which lie side by side (a rerun may have moved them)
+      // a single circuit's emission has written [flags, totals] for the host; else one copy of
+      // [cout, flags, totals], which lie side by side (a rerun may have moved them)
+      const bool direct = ncirc() == 1 && !used_global && L.nb && gpc::emit_folds(L.nb);
       const size_t bytes = L.totals + 8 - L.cout;
-      pin_out.ensure(bytes);
+      if (!direct) {
+        pin_out.ensure(bytes);
+        CK(cudaMemcpyAsync(pin_out.p, dptr<char>(L.cout), bytes, cudaMemcpyDeviceToHost, stream));
+      }
       const char *hc = static_cast<const char *>(pin_out.p);
-      CK(cudaMemcpyAsync(pin_out.p, dptr<char>(L.cout), bytes, cudaMemcpyDeviceToHost, stream));
       wait();
       uint32_t h[3];
-      memcpy(h, hc + (L.err - L.cout), 4);
-      memcpy(h + 1, hc + (L.totals - L.cout), 8);
+      if (direct) {
+        memcpy(h, pin_res.p, 12);
+      } else {
+        memcpy(h, hc + (L.err - L.cout), 4);
+        memcpy(h + 1, hc + (L.totals - L.cout), 8);
+      }
       const uint32_t err = h[0];
       if (err & gpc::DEV_ERR_TIMEOUT) throw gpc::Error(GPC_ERR_TIMEOUT, "a bounded device wait timed out");
       if (err & gpc::DEV_ERR_COLLISION)
@@ -1669,7 +1681,8 @@ struct gpc_driver {
       sizes.C = h[1];
       sizes.NT = h[2];
       sizes.first.resize(ncirc());
-      memcpy(sizes.first.data(), hc, (size_t)ncirc() * 8);
+      if (!direct) memcpy(sizes.first.data(), hc, (size_t)ncirc() * 8);
+      else sizes.first[0] = make_uint2(0, 0);
       sizes.known = true;
       return Finish::Ok;
     }

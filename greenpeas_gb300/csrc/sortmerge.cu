@@ -1086,7 +1086,6 @@ __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(MergeLaunch L) {
 // ---- merge of the compile pipeline ---------------------------------------
 
 constexpr uint32_t GW_WARPS = 8;  // buckets per group/emit block (one warp each)
-constexpr uint32_t kFoldBuckets = 32768;  // most buckets whose places the emission finds itself
 
 // Row of an item's later targets: its first mechanism.
 __device__ __forceinline__ const uint32_t *far_targets(const GroupLaunch &L, uint32_t m) {
@@ -1333,7 +1332,8 @@ __device__ __forceinline__ void emit_bucket(const GroupLaunch &L, uint32_t b, ui
 // and the aggregates before it in the tile: a few loads a thread for up to
 // kFoldBuckets buckets), which saves a small run the scan kernel; the block of
 // a circuit's first bucket writes the circuit's place, the last block the
-// totals.
+// totals (a single circuit's to page-locked host memory as well: the copy of
+// those 12 bytes that the host waited for cost 5 us of an 85-us run).
 template <bool FOLD>
 __global__ void __launch_bounds__(GW_WARPS * 32) emit_kernel(const __grid_constant__ GroupLaunch L) {
   const uint32_t tid = threadIdx.x, lane = tid & 31u, wi = tid >> 5;
@@ -1380,7 +1380,13 @@ __global__ void __launch_bounds__(GW_WARPS * 32) emit_kernel(const __grid_consta
       L.totals[0] = end.x;
       L.totals[1] = end.y;
       L.out_off[end.x] = end.y;  // the closing offset
-      if (end.y > L.tg_cap) atomicOr(L.err, DEV_FLAG_TG_OVF);
+      const uint32_t flag = end.y > L.tg_cap ? DEV_FLAG_TG_OVF : 0u;
+      if (flag) atomicOr(L.err, flag);
+      if (L.host_res) {  // (no kernel after this one sets a flag)
+        L.host_res[0] = *(volatile uint32_t *)L.err | flag;
+        L.host_res[1] = end.x;
+        L.host_res[2] = end.y;
+      }
     }
     for (uint32_t c = lane; c < L.n_circ; c += 32)
       if (L.cbbase[c] == b) L.cout[c] = out;
@@ -1590,7 +1596,7 @@ cudaError_t launch_group(const GroupLaunch &L, cudaStream_t s) {
 cudaError_t launch_scan_emit(const GroupLaunch &L, cudaStream_t s) {
   if (L.nb == 0) return cudaSuccess;
   const uint32_t blocks = (L.nb + GW_WARPS - 1) / GW_WARPS;
-  if (L.nb <= kFoldBuckets) {
+  if (emit_folds(L.nb)) {
     emit_kernel<true><<<blocks, GW_WARPS * 32, 0, s>>>(L);
   } else {
     group_scan_kernel<<<(L.nb + SCAN_TILE - 1) / SCAN_TILE, SCAN_THREADS, 0, s>>>(L);
