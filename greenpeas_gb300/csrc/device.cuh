@@ -28,8 +28,8 @@ struct CircuitDev {
   const uint32_t *ch_bytes;   // [n_chunks]
   const uint32_t *inj_lo;     // [w] first epoch injecting into word j (0xFFFFFFFF: none)
   const uint32_t *inj_hi;     // [w] last epoch injecting into word j
-  ulonglong2 *snap;           // [w][npoints] (X row, Z row) at each point
-  uint2 *band;                // [w] point range written by the walk of word j
+  ulonglong2 *snap;           // [w][npoints] (X row, Z row) at each point; stored where either is non-zero (nzm)
+  uint2 *band;                // [w] point range covered by the walk of word j
   unsigned long long *nzm;    // [npoints][mw] (zeroed) bit j: word j's rows at the point are non-zero
   const uint64_t *rec;        // [R] noise records
   const double *rec_p;        // [R]
@@ -323,7 +323,6 @@ cudaError_t launch_gather_hi(const ulonglong2 *key, const uint32_t *perm, uint64
 
 struct MergeLaunch {
   const CircuitDev *c_dev;  // single circuit
-  uint32_t w;
   const uint32_t *perm;     // sorted mechanism ids
   const uint64_t *sortkey;  // sorted keys (for the mixed-run check)
   uint64_t sort_mask;       // key bits the sort compared (0: skip the mixed-run check)

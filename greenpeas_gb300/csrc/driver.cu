@@ -1552,7 +1552,6 @@ struct gpc_driver {
   void launch_merge_now() {
     gpc::MergeLaunch ml{};
     ml.c_dev = dptr<CircuitDev>(L.cdev);
-    ml.w = tapes[0].w;
     ml.perm = sorted.perm;
     ml.sortkey = sorted.key;
     ml.sort_mask = sorted.mask;
@@ -1834,8 +1833,12 @@ struct gpc_driver {
       const Tape &T = tapes[i];
       std::vector<uint2> band(T.w);
       CK(cudaMemcpy(band.data(), dptr<char>(L.c[i].band), (size_t)T.w * 8, cudaMemcpyDeviceToHost));
+      // the snapshots stored: one per set mask bit
+      std::vector<uint64_t> nzm((size_t)T.npoints * ((T.w + 63) / 64));
+      CK(cudaMemcpy(nzm.data(), dptr<char>(L.c[i].nzm), nzm.size() * 8, cudaMemcpyDeviceToHost));
+      for (uint64_t x : nzm) pts += (double)__builtin_popcountll(x);
       // one walk CTA per group of circuit-words: it reads the tape of its
-      // epochs once and writes each word's snapshots
+      // epochs once
       const uint32_t W = circ_words.size() > i ? circ_words[i] : 1u;
       for (uint32_t j0 = 0; j0 < T.w; j0 += W) {
         const uint32_t nw = std::min(W, T.w - j0);
@@ -1847,14 +1850,12 @@ struct gpc_driver {
         uint32_t e1 = (uint32_t)(std::lower_bound(T.ep_ptoff.begin(), T.ep_ptoff.end(), band[j0].y) - T.ep_ptoff.begin());
         if (e1 > T.n_epochs) e1 = T.n_epochs;
         const uint64_t a = T.ep_opoff[e0], b = e1 < T.n_epochs ? T.ep_opoff[e1] : T.ops.size();
-        const double p = (double)(band[j0].y - band[j0].x) * nw;
-        walk += (double)(b - a) * 8 + 16.0 * p;
-        pts += p;
+        walk += (double)(b - a) * 8;
       }
       R += (double)T.rec.size();
     }
     const double M = L.M, groups = tot[0], targets = tot[1], nb = L.nb;
-    out[0] = walk;
+    out[0] = walk + 16.0 * pts;
     if (global_plan()) {
       // records, snapshot words read, key, descriptor and probability written
       out[1] = R * 20 + 16.0 * pts + M * 32;

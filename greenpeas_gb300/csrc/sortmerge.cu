@@ -43,17 +43,6 @@ __device__ __forceinline__ uint64_t pauli_sel(ulonglong2 s, uint32_t P) {
   return (s.x & (0ull - (uint64_t)(P & 1u))) ^ (s.y & (0ull - (uint64_t)((P >> 1) & 1u)));
 }
 
-// Word j of mechanism descriptor d (band-aware).
-__device__ __forceinline__ uint64_t symptom_word(const CircuitDev &C, uint64_t d, uint32_t j, uint2 b) {
-  const uint32_t pa = (uint32_t)(d & 0x3FFFFFFFu), Pa = (uint32_t)((d >> 30) & 3u);
-  const uint32_t pb = (uint32_t)((d >> 32) & 0x3FFFFFFFu), Pb = (uint32_t)(d >> 62);
-  const ulonglong2 *sj = C.snap + (size_t)j * C.npoints;
-  uint64_t v = 0;
-  if (Pa && pa - b.x < b.y - b.x) v ^= pauli_sel(sj[pa], Pa);
-  if (Pb && pb - b.x < b.y - b.x) v ^= pauli_sel(sj[pb], Pb);
-  return v;
-}
-
 __device__ __forceinline__ uint64_t mk_desc(uint32_t pa, uint32_t Pa, uint32_t pb, uint32_t Pb) {
   return (uint64_t)(pa & 0x3FFFFFFFu) | ((uint64_t)(Pa & 3u) << 30) | ((uint64_t)(pb & 0x3FFFFFFFu) << 32) |
          ((uint64_t)(Pb & 3u) << 62);
@@ -846,16 +835,27 @@ __device__ __forceinline__ void warp_lookback(unsigned long long *status, uint32
   *pre_t = et;
 }
 
-// Mask word i of the words where mechanism d's symptom can be non-zero: the
-// union of its points' non-zero masks (a word whose mask bit is clear has a
-// zero snapshot at that point, so it adds nothing to the symptom).
-__device__ __forceinline__ uint64_t symptom_mask(const CircuitDev &C, uint64_t d, uint32_t i) {
+// A mechanism's points, and mask word i of the words where each of them has a snapshot (a word whose bit is
+// clear has none stored: its rows were zero there).
+struct SymptomMask {
+  uint64_t a = 0, b = 0;  // of the first and the second point
+};
+__device__ __forceinline__ SymptomMask symptom_mask(const CircuitDev &C, uint64_t d, uint32_t i) {
   const uint32_t pa = (uint32_t)(d & 0x3FFFFFFFu), Pa = (uint32_t)((d >> 30) & 3u);
   const uint32_t pb = (uint32_t)((d >> 32) & 0x3FFFFFFFu), Pb = (uint32_t)(d >> 62);
-  uint64_t b = 0;
-  if (Pa) b |= __ldg(C.nzm + (size_t)pa * C.mw + i);
-  if (Pb) b |= __ldg(C.nzm + (size_t)pb * C.mw + i);
-  return b;
+  SymptomMask m;
+  if (Pa) m.a = __ldg(C.nzm + (size_t)pa * C.mw + i);
+  if (Pb) m.b = __ldg(C.nzm + (size_t)pb * C.mw + i);
+  return m;
+}
+
+// Word j of mechanism descriptor d (bit j % 64 of the mask words m).
+__device__ __forceinline__ uint64_t symptom_word(const CircuitDev &C, uint64_t d, uint32_t j, const SymptomMask &m) {
+  const ulonglong2 *sj = C.snap + (size_t)j * C.npoints;
+  uint64_t v = 0;
+  if ((m.a >> (j & 63u)) & 1ull) v = pauli_sel(sj[d & 0x3FFFFFFFu], (uint32_t)((d >> 30) & 3u));
+  if ((m.b >> (j & 63u)) & 1ull) v ^= pauli_sel(sj[(d >> 32) & 0x3FFFFFFFu], (uint32_t)(d >> 62));
+  return v;
 }
 
 // One thread per sorted position; one warp folds the tile's runs.  FP64 runs at 2 lanes a cycle and SM,
@@ -863,14 +863,13 @@ __device__ __forceinline__ uint64_t symptom_mask(const CircuitDev &C, uint64_t d
 // scan over the lanes, a tile of 256 costs 13 warp-wide merges (every warp scanning its 32 positions: 40,
 // and the carries as many again).  A run still open at its tile's end is read on by the block,
 // MERGE_THREADS positions at a time, and folded by the same warp; the tile's counts are published before
-// that and its predecessors' read after, 128 a step.  118k mechanisms in runs of 300: 26 -> 17.5 us
+// that and its predecessors' read after, 128 a step.  118k mechanisms in runs of 300: 26 -> 15.6 us
 // (one thread following its run alone: 503).  What is left is a chain of ~10 dependent loads (4.5k
 // cycles to the keys and symptoms, 4k in the open run, 3k in the look-back).  The tree is deterministic
 // and differs from a left-to-right fold by a few ulps.
 __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(MergeLaunch L) {
   constexpr uint32_t NW = MERGE_THREADS / 32;
   const CircuitDev C = *L.c_dev;
-  extern __shared__ uint2 sband[];  // [w]
   __shared__ uint32_t s_tile;
   __shared__ uint32_t wsum_c[MERGE_THREADS / 32], wsum_t[MERGE_THREADS / 32];
   __shared__ uint32_t s_pre_c, s_pre_t;
@@ -880,8 +879,6 @@ __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(MergeLaunch L) {
   __shared__ uint32_t s_head[NW];               // where runs start, a bit per position
   __shared__ ulonglong2 s_key;                  // the key of the run open at the tile's end
   __shared__ uint32_t s_open;                   // its first position in the tile (MERGE_THREADS: none follows)
-  const uint32_t w = L.w;
-  for (uint32_t j = threadIdx.x; j < w; j += blockDim.x) sband[j] = C.band[j];
   if (threadIdx.x == 0) s_tile = atomicAdd(L.tile_ctr, 1u);
   __syncthreads();
   const uint32_t tile = s_tile;
@@ -914,22 +911,23 @@ __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(MergeLaunch L) {
     // One loop for both kinds of position, two words at a time: a head counts its targets, another one's
     // full symptom is compared with its predecessor's on the words either can be non-zero in.
     bool diff = false;
-    for (uint32_t mi = 0; mi < C.mw; ++mi)
-      for (uint64_t bits = symptom_mask(C, d, mi) | (newgroup ? 0ull : symptom_mask(C, dp, mi)); bits;) {
+    for (uint32_t mi = 0; mi < C.mw; ++mi) {
+      const SymptomMask ma = symptom_mask(C, d, mi), mb = newgroup ? SymptomMask{} : symptom_mask(C, dp, mi);
+      for (uint64_t bits = ma.a | ma.b | mb.a | mb.b; bits;) {
         const uint32_t j0 = mi * 64u + (uint32_t)(__ffsll((long long)bits) - 1);
         bits &= bits - 1;
-        const uint32_t j1 = bits ? mi * 64u + (uint32_t)(__ffsll((long long)bits) - 1) : w;
+        const bool two = bits != 0;
+        const uint32_t j1 = two ? mi * 64u + (uint32_t)(__ffsll((long long)bits) - 1) : j0;
         bits &= bits - 1;
-        const uint64_t a0 = j0 < w ? symptom_word(C, d, j0, sband[j0]) : 0ull;
-        const uint64_t a1 = j1 < w ? symptom_word(C, d, j1, sband[j1]) : 0ull;
+        const uint64_t a0 = symptom_word(C, d, j0, ma), a1 = two ? symptom_word(C, d, j1, ma) : 0ull;
         if (newgroup) {
           ntg += __popcll(a0) + __popcll(a1);
         } else {
-          const uint64_t b0 = j0 < w ? symptom_word(C, dp, j0, sband[j0]) : 0ull;
-          const uint64_t b1 = j1 < w ? symptom_word(C, dp, j1, sband[j1]) : 0ull;
+          const uint64_t b0 = symptom_word(C, dp, j0, mb), b1 = two ? symptom_word(C, dp, j1, mb) : 0ull;
           diff |= a0 != b0 || a1 != b1;
         }
       }
+    }
     const bool empty = (k.x | k.y) == 0;
     // (a non-empty symptom hashed to zero is a collision too)
     if (diff || (newgroup && empty && ntg)) atomicOr(L.err, DEV_ERR_COLLISION);
@@ -1071,15 +1069,17 @@ __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(MergeLaunch L) {
   if ((uint64_t)toff + ntg <= L.tg_cap) {
     const uint64_t d = __ldg(C.mdesc + m);
     uint32_t o = toff;
-    for (uint32_t mi = 0; mi < C.mw; ++mi)  // the masked words, ascending: the targets stay ascending
-      for (uint64_t bits = symptom_mask(C, d, mi); bits; bits &= bits - 1) {
+    for (uint32_t mi = 0; mi < C.mw; ++mi) {  // the masked words, ascending: the targets stay ascending
+      const SymptomMask mk = symptom_mask(C, d, mi);
+      for (uint64_t bits = mk.a | mk.b; bits; bits &= bits - 1) {
         const uint32_t j = mi * 64u + (uint32_t)(__ffsll((long long)bits) - 1);
-        uint64_t v = j < w ? symptom_word(C, d, j, sband[j]) : 0ull;
+        uint64_t v = symptom_word(C, d, j, mk);
         while (v) {
           L.out_tg[o++] = j * 64u + (uint32_t)(__ffsll((long long)v) - 1);
           v &= v - 1;
         }
       }
+    }
   }
 }
 
@@ -1655,7 +1655,7 @@ cudaError_t launch_gather_hi(const ulonglong2 *key, const uint32_t *perm, uint64
 cudaError_t launch_merge(const MergeLaunch &L, cudaStream_t s) {
   if (L.n == 0) return cudaSuccess;
   const uint32_t tiles = merge_tiles(L.n);
-  merge_kernel<<<tiles, MERGE_THREADS, (size_t)L.w * sizeof(uint2), s>>>(L);
+  merge_kernel<<<tiles, MERGE_THREADS, 0, s>>>(L);
   return cudaGetLastError();
 }
 
