@@ -41,15 +41,15 @@ METRIC = "DEM compiles/s (plain method, one circuit per compile)"
 UNIT = "DEM/s"
 WORKLOAD = "bb_144_12_12_r12_uniform_p1e-3"
 PEAKS_FILE = ROOT / "MEASURED_PEAKS.json"
-# kernels of one run of the pipeline on one circuit: key-block table, walk, keys,
-# warp grouping, large-bucket grouping, scan, emit (the segmented walk is two launches)
-KERNELS_PER_RUN = 7
+# kernels of one run of the pipeline on one circuit: key-warp table, walk, keys,
+# grouping, emission (the segmented walk is two launches)
+KERNELS_PER_RUN = 5
 # DRAM bytes (read + write) of the walk on the headline workload, from ncu captures (cold cache:
 # the tape is read once from DRAM, the word walks re-read it from L2): the plain walk launch
 # (profiles/headline_bb12_kernels.txt) and the two launches of the segmented walk
 # (profiles/headline_bb12_segmented_walk.txt).
 WALK_DRAM_BYTES_PLAIN = 1_245_440
-WALK_DRAM_BYTES_PER_RUN = 1_147_904 + 1_919_488
+WALK_DRAM_BYTES_PER_RUN = 1_104_640 + 1_873_152
 
 
 def workload_text() -> str:
@@ -799,7 +799,7 @@ def main() -> None:
                      "note": "latency-bound: word walks cut into time segments walked side by side",
                      "pipeline": pipeline},
         "fallbacks": r["fallbacks"],
-        # key-block table, walk launch(es), keys, warp grouping, large-bucket grouping, scan, emit
+        # key-warp table, walk launch(es), keys, grouping, emission
         "gpu_launches": (KERNELS_PER_RUN - 1 + walk_launches) * args.steps,
         "clocks": clocks.summary(),
     }

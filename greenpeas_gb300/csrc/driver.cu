@@ -1277,13 +1277,14 @@ struct gpc_driver {
   // segments long.  A short segment means short walks and more compose steps
   // (about 0.5 us each); a large circuit's segment CTAs fill the GPU (one per
   // SM from ~600 slots on), so it is bound by their number and wants fewer.
-  // Measured on GB300 (walk stage with its event, whole / 32 / 64 / 96 units,
-  // us): [[144,12,12]] r12 77 / 28.5 / 30.8 / 39, surface d = 11 77 / 26 / 33 /
-  // 45, [[288,12,18]] 129 / 59 / 65 / 57, d = 17 - / 57 / 53 / 59, d = 21 192 /
-  // 104 / 98 / 100, d = 25 291 / 166 / 143 / 133; surface d = 3 walks 17 epochs
-  // and stays whole (its longest walk costs 123 units).  From 1,024 slots on
-  // (two a thread) 96 / 128 / 160 units: d = 23 116 / 110 / 109, d = 25 135 /
-  // 121 / 131, d = 27 172 / 172 / 182, d = 29 215 / 198 / 209.
+  // Measured on GB300 (walk stage with its event, us), whole / 32 / 64 / 96
+  // units: [[144,12,12]] r12 77 / 28.5 / 30.8 / 39, surface d = 11 77 / 26 / 33 /
+  // 45, [[288,12,18]] 129 / 59 / 47 / 47; 64 / 96 / 128: d = 17 53 / 59 / 57,
+  // d = 19 56 / 61 / 55 (153 whole), d = 21 77 / 76 / 76 (190 whole); surface
+  // d = 3 walks 17 epochs and stays whole (its longest walk costs 123 units).
+  // From 1,024 slots on (two a thread) 96 / 128 / 160 units: d = 23 116 / 110 /
+  // 109, d = 25 135 / 121 / 131 (286 whole), d = 27 172 / 172 / 182, d = 29 215 /
+  // 198 / 209.
   static uint32_t seg_target(uint32_t qpad) { return qpad < 1024u ? 32u * (1u + qpad / 512u) : 128u; }
   static constexpr uint32_t kSegMinSpan = 4;
   // A detector word's rows vanish some epochs after its last measurement

@@ -459,7 +459,10 @@ __global__ void __launch_bounds__(WalkBound<QPT>::value) walk_queue_kernel(const
 // Chunks of whole epochs and a ring of step buffers in shared memory, filled
 // by bulk copies, needed 243 KB for the 896 slots of a d = 21 surface memory,
 // which therefore walked whole.  Walk stage before -> now: surface d = 25 (1,280
-// slots) 291 -> 133 us, d = 21 192 -> 98, [[144,12,12]] 34.7 -> 28.5.
+// slots) 291 -> 121 us, d = 21 192 -> 79, [[144,12,12]] 34.7 -> 28.5.  Blocks of
+// 48 registers, two an SM, spill in the op loop (d = 25: 190 us); letting a warp
+// skip the rows of slots that are all zero costs a vote a row on the same chain
+// (140 us, and the plain walk of a batch 1,041 -> 1,197).
 constexpr int kAhead = 4;
 constexpr uint32_t kNoState = 0xFFFFFFFFu;
 enum : int { MODE_FIRST = 0, MODE_AFF = 1, MODE_XFER = 2, MODE_REST = 3 };
