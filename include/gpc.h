@@ -315,9 +315,9 @@ gpc_status gpc_walk_segments(gpc_driver *driver, uint32_t *segments, uint32_t *i
                              uint32_t *items_rest);
 
 /* Algorithmic bytes moved by each stage of the last run, counted from its
- * sizes: [0] walk (tape read + snapshots written), [1] key (records + snapshot
- * reads + keys, descriptors, target lists and bucket slots written), [2]
- * bucket grouping (slots read, lists compared, group records written), [3]
+ * sizes: [0] walk (tape read + snapshots stored, the non-zero ones), [1] key
+ * (records + snapshot reads + bucket slots written; on the global path keys and
+ * descriptors), [2] bucket grouping (slots read, group records written), [3]
  * scan + emit (group records and head lists read, DEM written). */
 gpc_status gpc_last_traffic(gpc_driver *driver, double *bytes4);
 
