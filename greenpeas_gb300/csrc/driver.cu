@@ -515,6 +515,7 @@ struct gpc_driver {
   AllocCounter alloc_ctr;
   DevBuf arena{nullptr, 0, &alloc_ctr}, tgbuf{nullptr, 0, &alloc_ctr};
   HostBuf pin_in, pin_out;
+  HostBuf pin_tab;  // gradients: the rates of the last forward and each source's split probabilities and slopes
   HostBuf pin_res;  // a single circuit's [flags, groups, targets], written by its emission
   uint32_t tg_cap = 0;
   cudaEvent_t ev[5] = {};
@@ -585,7 +586,7 @@ struct gpc_driver {
   }
   // noise-rate gradients: record probabilities come from a device noise tensor
   bool param = false;
-  const double *noise_dev = nullptr;
+  bool rates_known = false;  // pin_tab holds the prepared template's rates
   uint32_t param_groups = 0;
   cudaEvent_t caller_ev = nullptr, done_ev = nullptr;
   cudaGraph_t graph = nullptr;  // captured kernel sequence of run() for one launch configuration
@@ -634,6 +635,7 @@ struct gpc_driver {
     tgbuf.release();
     pin_in.release();
     pin_out.release();
+    pin_tab.release();
     pin_res.release();
     for (auto &e : ev)
       if (e) cudaEventDestroy(e);
@@ -1096,6 +1098,7 @@ struct gpc_driver {
     if (texts) {
       if (param_mode && n != 1) throw gpc::Error(GPC_ERR_INVALID, "noise-rate gradients take one circuit");
       param = param_mode;
+      rates_known = false;
     }
     prepared = false;
     ran = false;
@@ -1634,7 +1637,7 @@ struct gpc_driver {
           lists_off = true;
         }
         prepare(nullptr, nullptr, 0);
-        if (param && noise_dev) launch_param_rec_now();
+        if (param && rates_known) launch_param_rec_now();
         run();
         continue;
       }
@@ -1716,8 +1719,13 @@ struct gpc_driver {
   // ---- noise-rate gradients (one circuit) --------------------------------
   uint32_t n_src() const { return tapes.empty() ? 0 : tapes[0].n_ticks * gpc::SRC_CLASSES; }
 
+  // Record probabilities of the noise tensor's rates.  The split tables lie past the target lists in the
+  // arena, so they move when the lists are widened and prepare() does not write them: every call brings
+  // them along, from the page-locked copy that param_forward fills and nothing else uses.
   void launch_param_rec_now() {
     const Tape &T = tapes[0];
+    const size_t ns = n_src();
+    CK(cudaMemcpyAsync(dptr<char>(L.ptab), static_cast<double *>(pin_tab.p) + ns, ns * 6 * 8, cudaMemcpyHostToDevice, stream));
     gpc::ParamLaunch pl{};
     pl.rec = dptr<uint64_t>(L.c[0].rec);
     pl.rec_src = dptr<uint32_t>(L.c[0].rec_src);
@@ -1745,7 +1753,7 @@ struct gpc_driver {
     if (!noise) throw gpc::Error(GPC_ERR_INVALID, "noise tensor is null");
     CK(cudaSetDevice(device));
     wait_caller(caller);
-    noise_dev = noise;
+    rates_known = false;
     // The rates come to the host (n_ticks x 4 doubles): each source's split
     // probability and slope per channel kind are evaluated with the same
     // host formulas as the text path, so a template run with a rate tensor
@@ -1754,8 +1762,8 @@ struct gpc_driver {
     // root moves q by ~1e-12 relative at p ~ 1e-3, so the root must come from
     // the same pow.)
     const uint32_t ns = n_src();
-    pin_out.ensure((size_t)ns * 8 * 7);
-    double *h = static_cast<double *>(pin_out.p);
+    pin_tab.ensure((size_t)ns * 8 * 7);
+    double *h = static_cast<double *>(pin_tab.p);
     CK(cudaMemcpyAsync(h, noise, (size_t)ns * 8, cudaMemcpyDeviceToHost, stream));
     wait();
     double *qt = h + ns, *st = h + 4 * (size_t)ns;
@@ -1776,7 +1784,7 @@ struct gpc_driver {
       qt[3 * e + 2] = ok2 ? gpc::split_dep2(p) : 0.0;
       st[3 * e + 2] = ok2 && x2 > 0 ? std::pow(x2, 0.125) / (15.0 * x2) : 0.0;
     }
-    CK(cudaMemcpyAsync(dptr<char>(L.ptab), qt, (size_t)ns * 6 * 8, cudaMemcpyHostToDevice, stream));
+    rates_known = true;
     launch_param_rec_now();
     run();
     uint32_t C = 0, NT = 0;
