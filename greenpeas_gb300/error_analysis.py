@@ -159,7 +159,6 @@ class Driver:
         is lowered whole on all host threads."""
         L = _native.lib()
         self._h = ctypes.c_void_p()
-        self._views = None
         self.correlation_level = CorrelationLevel(correlation_level)
         self.device = device
         opts = _native.Options()
@@ -285,36 +284,12 @@ class Driver:
         n, end = ctypes.c_uint32(), ctypes.c_uint32()
         _native.check(L.gpc_device_dem(self._h, int(circuit), ctypes.byref(pp), ctypes.byref(po), ctypes.byref(pt),
                                        ctypes.byref(n), ctypes.byref(end)))
-        n, end = n.value, end.value
-        views = self._device_views(int(circuit), pp.value, po.value, pt.value, n, end)
-        return tuple(t[(addr - base) // size:(addr - base) // size + count] for (base, size, t), addr, count in
-                     zip(views, (pp.value, po.value, pt.value), (n, n + 1, end)))
-
-    def _device_views(self, circuit, pp, po, pt, n, end):
-        """(address, item size, tensor) over the run's whole probability, offset and target buffers.
-
-        Wrapping a device address costs ~10 us in torch and a slice ~1 us, so the buffers are wrapped
-        once and a batch's circuits slice them; they are wrapped again when the wanted range is not inside
-        (the driver's buffers moved or grew)."""
-        want = ((pp, n * 8), (po, (n + 1) * 4), (pt, end * 4))
-        views = self._views
-        if views is not None and all(base <= a and a + b <= base + t.numel() * size
-                                     for (base, size, t), (a, b) in zip(views, want)):
-            return views
         import torch
-        if circuit:  # the run's arrays start at its first circuit's
-            p0, o0, t0 = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p()
-            c = ctypes.c_uint32()
-            _native.check(_native.lib().gpc_device_dem(self._h, 0, ctypes.byref(p0), ctypes.byref(o0), ctypes.byref(t0),
-                                                       ctypes.byref(c), ctypes.byref(c)))
-            pp, po, pt = p0.value, o0.value, t0.value
-        raw = self.last_sizes()["raw"]  # capacity of the outputs; the target buffer holds 16 per mechanism at least
-
         dev = torch.device("cuda", self.device)
-        self._views = tuple((a, size, torch.as_tensor(_DeviceView(a, count, typestr), device=dev)) for a, count, size, typestr in
-                            ((pp, raw, 8, "<f8"), (po, raw + 1, 4, "<i4"),
-                             (pt, max(end, min(16 * raw, 0xFFFFFFF0)), 4, "<i4")))
-        return self._views
+        n, end = n.value, end.value
+        # (a tensor of its own for each array, made in the caller's mode: nothing is shared between calls or circuits)
+        return tuple(torch.as_tensor(_DeviceView(a.value, count, typestr), device=dev)
+                     for a, count, typestr in ((pp, n, "<f8"), (po, n + 1, "<i4"), (pt, end, "<i4")))
 
     # device-resident stages
     def prepare(self, circuit=None) -> None:
