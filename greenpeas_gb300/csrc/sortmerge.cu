@@ -112,6 +112,7 @@ constexpr uint32_t kKeyEntries = 64;   // entries a warp holds at once
 constexpr uint32_t kKeyValues = 128;   // distinct values
 constexpr uint32_t kKeyTargets = 160;  // targets of the records' unions (up to 32 a record)
 constexpr uint32_t kKeyItems = 256;
+constexpr uint32_t kKeyRecords = 128;  // records of a warp (one mechanism each at least: key_chunk)
 
 // Components present (bit s) and their place in the component list, by record type (kComp).
 __constant__ uint16_t kPresent[6] = {0, 0x0006, 0x000E, 0x0536, 0x177E, 0xFFFE};
@@ -133,6 +134,7 @@ struct KeyWarp {
   uint64_t place[32];        // kPlace of the record's type
   uint16_t present[32];      // the record's components (bit s)
   uint8_t e0[32], e1[32];
+  uint32_t late[kKeyRecords / 32];  // records left for key_late_records
 };
 
 // Probability that an odd number of `c` independent events of probability q happens.
@@ -170,12 +172,6 @@ __device__ __forceinline__ uint32_t coset_heads(uint32_t present, uint32_t zero,
   return heads;
 }
 
-// An item's name when the gradients need its record: the record and the place
-// of its first component (in the same order as the first mechanisms).
-__device__ __forceinline__ uint32_t item_id(uint32_t r, uint32_t type, uint32_t s) {
-  return r << 4 | ((uint32_t)(kPlace[type] >> (4u * s)) & 15u);
-}
-
 // Files an item in its bucket: one 64-byte slot as two 32-byte stores.  The
 // bucket's counter counts items in its low half and mechanisms in its high
 // half: a bucket overflows by its mechanisms, whatever is merged beforehand.
@@ -199,64 +195,128 @@ __device__ __forceinline__ void file_item(const KeyLaunch &L, uint32_t bbase, ui
                "r"(l[2]), "r"(l[3]), "r"(l[4]), "r"(l[5]), "r"(l[6]), "r"(l[7]));
 }
 
-// One record that holds more words, values or targets than the warp's arrays:
-// lane s follows selection s through the record's words, first to find the
-// selections without a symptom, then for the items' keys and targets.
-__device__ __noinline__ uint32_t key_record_direct(const KeyLaunch &L, const CircuitDev &C, uint32_t r, uint32_t *stage) {
-  const uint32_t lane = threadIdx.x & 31u;
+// ---- records of long symptoms
+//
+// Where a record holds more words, values or targets than the warp's arrays, or
+// so few records fit them that most lanes would idle, the warp leaves the
+// records for its end (the calls below in the loop itself would cost every
+// record their registers) and then follows their components through the words,
+// as many records of a type at a time as have components for the 32 lanes.
+// Bound by the instructions of the words' hashes and lists, and for few
+// mechanisms by the chain of the words' loads.  A memory of 400 qubits measured
+// 100 times without resets, every measurement a detector (460k mechanisms,
+// symptoms of up to 100 targets): one record at a time 6,390 us, side by side
+// 350; a thread per mechanism, which is slower for short symptoms, 222.
+
+// Components of a record, the lanes it takes in key_records_direct.
+__device__ __forceinline__ uint32_t components(uint32_t type) {
+  return type == REC_PAULI ? 1u : (uint32_t)__popc((uint32_t)kPresent[type]);
+}
+// Selections that are no component of the type (nibble l: lane l's; 0: none), a second one for some lanes.
+__constant__ uint64_t kSpare[6][2] = {{0, 0}, {0x3, 0}, {0, 0}, {0xCB9763, 0xFED}, {0xFEDB7, 0}, {0, 0}};
+
+// `n` records of one type side by side.  The components of one symptom are
+// merged as in key_items_kernel, which wants the selections without a symptom:
+// SPARE, the type's components are not all of them (correlation levels 0 and
+// 1), and each lane looks out for up to two more.
+template <bool SPARE>
+__device__ __forceinline__ uint32_t key_records_direct(const KeyLaunch &L, const CircuitDev &C, uint32_t r0, uint32_t n,
+                                                       uint32_t type, uint32_t *stage) {
+  const uint32_t lane = threadIdx.x & 31u, width = components(type);
+  const uint32_t k = lane / width, l0 = k * width, place = lane - l0;
+  const bool in = k < n;
+  const uint32_t r = r0 + (in ? k : 0u);
   const uint64_t d = __ldg(C.rec + r);
-  const uint32_t pa = (uint32_t)(d & 0x0FFFFFFFu), pb = (uint32_t)((d >> 28) & 0x0FFFFFFFu);
-  const uint32_t type = (uint32_t)((d >> 56) & 15u);
-  const uint32_t present = type == REC_PAULI ? 1u << ((uint32_t)(d >> 60) & 15u) : kPresent[type];
-  const bool has_a = (present & 0xEEEEu) != 0, has_b = (present & 0xFFF0u) != 0;
-  const uint32_t np = C.npoints, mw = C.mw, s = lane & 15u, inl = L.narrow ? 16u : 8u, tcap = C.tcap;
-  const unsigned long long *ma = C.nzm + (size_t)pa * mw, *mb = C.nzm + (size_t)pb * mw;
-  auto for_words = [&](auto &&f) {
-    for (uint32_t i = 0; i < mw; ++i) {
-      const uint64_t ba = has_a ? __ldg(ma + i) : 0ull, bb = has_b ? __ldg(mb + i) : 0ull;
-      for (uint64_t bits = ba | bb; bits; bits &= bits - 1) {
-        const uint32_t bit = (uint32_t)(__ffsll((long long)bits) - 1), j = i * 64u + bit;
-        const ulonglong2 *sj = C.snap + (size_t)j * np;
-        uint64_t v = 0;
-        if ((ba >> bit) & 1ull) v = pauli_sel(sj[pa], s & 3u);
-        if ((bb >> bit) & 1ull) v ^= pauli_sel(sj[pb], s >> 2);
-        if (v) f(j, v);
+  const uint32_t s = type == REC_PAULI ? (uint32_t)(d >> 60) & 15u : kComp[type][place];
+  const uint32_t s1 = SPARE ? (uint32_t)(kSpare[type][0] >> (4u * place)) & 15u : 0u;
+  const uint32_t s2 = SPARE ? (uint32_t)(kSpare[type][1] >> (4u * place)) & 15u : 0u;
+  const bool has_a = in && ((s | s1 | s2) & 3u), has_b = in && ((s | s1 | s2) >> 2);
+  const uint32_t np = C.npoints, mw = C.mw, tcap = C.tcap;
+  const bool narrow = L.narrow;
+  const uint32_t m = C.mbase + __ldg(C.rec_moff + r) + place;
+  uint32_t *const far = L.tl + (size_t)m * L.tstride - (narrow ? 16u : 8u);  // (the row holds the targets past the slot's)
+  // the item's first targets, [word][lane]
+  __syncwarp();
+  for (uint32_t i = 0; i < 8; ++i) stage[i * 32u + lane] = 0;
+  uint64_t hx = 0, hy = 0, any1 = 0, any2 = 0;
+  uint32_t cnt = 0;
+  auto word = [&](uint32_t j, uint64_t v) {
+    const ulonglong2 h = word_hash(j, v);
+    hx ^= h.x;
+    hy ^= h.y;
+    for (; v; v &= v - 1, ++cnt) {
+      const uint32_t t = j * 64u + (uint32_t)(__ffsll((long long)v) - 1);
+      if (cnt >= (narrow ? 16u : 8u)) {
+        if (cnt < tcap) far[cnt] = t;
+      } else if (narrow) {
+        reinterpret_cast<uint16_t *>(stage)[((cnt >> 1) * 32u + lane) * 2u + (cnt & 1u)] = (uint16_t)t;
+      } else {
+        stage[cnt * 32u + lane] = t;
       }
     }
   };
-  uint64_t any = 0;
-  for_words([&](uint32_t, uint64_t v) { any |= v; });
-  const uint32_t zero = __ballot_sync(0xFFFFFFFFu, any == 0) & 0xFFFFu;
-  const uint32_t join = joining(type, zero), heads = coset_heads(present, zero, join);
-  const bool item = lane < 16u && ((heads >> s) & 1u);
-  const uint32_t m = C.mbase + __ldg(C.rec_moff + r) + (uint32_t)(kPlace[type] >> (4u * s) & 15u);
-  uint64_t hx = 0, hy = 0;
-  uint32_t cnt = 0;
-  uint32_t *mine = stage + lane * 8u;  // 32 bytes: the item's first targets
-  if (item) {
-    uint32_t *far = L.tl + (size_t)m * L.tstride;
-    for (uint32_t i = 0; i < 8; ++i) mine[i] = 0;
-    for_words([&](uint32_t j, uint64_t v) {
-      const ulonglong2 h = word_hash(j, v);
-      hx ^= h.x;
-      hy ^= h.y;
-      for (uint64_t x = v; x; x &= x - 1, ++cnt) {
-        const uint32_t t = j * 64u + (uint32_t)(__ffsll((long long)x) - 1);
-        if (cnt >= inl) {
-          if (cnt < tcap) far[cnt - inl] = t;
-        } else if (L.narrow) {
-          reinterpret_cast<uint16_t *>(mine)[cnt] = (uint16_t)t;
-        } else {
-          mine[cnt] = t;
-        }
+  const uint32_t pa = (uint32_t)(d & 0x0FFFFFFFu), pb = (uint32_t)((d >> 28) & 0x0FFFFFFFu);
+  const unsigned long long *ma = C.nzm + (size_t)pa * mw, *mb = C.nzm + (size_t)pb * mw;
+  const ulonglong2 *const snap_a = C.snap + pa, *const snap_b = C.snap + pb;
+  for (uint32_t i = 0; i < mw; ++i) {
+    const uint64_t ba = has_a ? __ldg(ma + i) : 0ull, bb = has_b ? __ldg(mb + i) : 0ull;
+    for (uint64_t bits = ba | bb; bits;) {  // (two words' rows on the way at once; four targets a store: no gain)
+      const uint32_t b0 = (uint32_t)(__ffsll((long long)bits) - 1);
+      bits &= bits - 1;
+      const uint32_t b1 = bits ? (uint32_t)(__ffsll((long long)bits) - 1) : 64u;
+      bits &= bits - 1;
+      const size_t j0 = (size_t)(i * 64u + b0) * np, j1 = (size_t)(i * 64u + b1) * np;
+      ulonglong2 xa = make_ulonglong2(0, 0), xb = xa, ya = xa, yb = xa;
+      if ((ba >> b0) & 1ull) xa = snap_a[j0];
+      if ((bb >> b0) & 1ull) xb = snap_b[j0];
+      if (b1 < 64u && ((ba >> b1) & 1ull)) ya = snap_a[j1];
+      if (b1 < 64u && ((bb >> b1) & 1ull)) yb = snap_b[j1];
+      if constexpr (SPARE) {
+        any1 |= pauli_sel(xa, s1) ^ pauli_sel(xb, s1 >> 2) | pauli_sel(ya, s1) ^ pauli_sel(yb, s1 >> 2);
+        any2 |= pauli_sel(xa, s2) ^ pauli_sel(xb, s2 >> 2) | pauli_sel(ya, s2) ^ pauli_sel(yb, s2 >> 2);
       }
-    });
-    uint32_t l[8];
-    for (uint32_t i = 0; i < 8; ++i) l[i] = mine[i];
-    const uint32_t mult = (uint32_t)__popc(xor_bits16(join, s) & present);
-    file_item(L, C.bbase, C.bbits, C.tcap, hx, hy, L.keep ? item_id(r, type, s) : m, cnt, mult, repeat_merge(__ldg(C.rec_p + r), mult), l);
+      const uint64_t v0 = pauli_sel(xa, s) ^ pauli_sel(xb, s >> 2), v1 = pauli_sel(ya, s) ^ pauli_sel(yb, s >> 2);
+      if (v0) word(i * 64u + b0, v0);
+      if (v1) word(i * 64u + b1, v1);
+    }
   }
+  const uint32_t group = (uint32_t)(((1ull << width) - 1ull) << l0);  // the record's lanes (those past the last record's: one too)
+  __syncwarp();
+  const uint32_t zero = 1u | __reduce_or_sync(group, (cnt ? 0u : 1u << s) | (any1 ? 0u : 1u << s1) | (any2 ? 0u : 1u << s2));
+  const uint32_t present = type == REC_PAULI ? 1u << s : kPresent[type], join = joining(type, zero);
+  if (!in || !((coset_heads(present, zero, join) >> s) & 1u)) return 0;
+  uint32_t l[8];
+#pragma unroll
+  for (uint32_t i = 0; i < 8; ++i) l[i] = stage[i * 32u + lane];
+  const uint32_t mult = (uint32_t)__popc(xor_bits16(join, s) & present);
+  file_item(L, C.bbase, C.bbits, tcap, hx, hy, L.keep ? r << 4 | place : m, cnt, mult, repeat_merge(__ldg(C.rec_p + r), mult), l);
   return cnt;
+}
+
+// The records that a warp postponed: bits of `late`, from its first record on.
+__device__ __noinline__ uint32_t key_late_records(const KeyLaunch &L, const CircuitDev &C, uint32_t first, KeyWarp &S) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t listed = 0;
+  for (uint32_t p = 0; p < kKeyRecords;) {
+    // bits p .. p + 31
+    const uint32_t hi = p / 32u + 1u < kKeyRecords / 32u ? S.late[p / 32u + 1u] : 0u;
+    const uint32_t bits = __funnelshift_r(S.late[p / 32u], hi, p & 31u);
+    if (bits == 0) {
+      p += 32;
+      continue;
+    }
+    p += (uint32_t)__ffs((int)bits) - 1u;
+    const uint32_t run = bits >> (__ffs((int)bits) - 1);  // from its first record on
+    const uint32_t type = (run >> lane) & 1u ? (uint32_t)(__ldg(C.rec + first + p + lane) >> 56) & 15u : 16u;
+    const uint32_t type0 = __shfl_sync(0xFFFFFFFFu, type, 0);
+    const uint32_t other = __ballot_sync(0xFFFFFFFFu, type != type0);
+    const uint32_t n = min(other ? (uint32_t)__ffs((int)other) - 1u : 32u, 32u / components(type0));
+    uint32_t *const stage = reinterpret_cast<uint32_t *>(S.h);
+    listed += kSpare[type0][0] ? key_records_direct<true>(L, C, first + p, n, type0, stage)
+                               : key_records_direct<false>(L, C, first + p, n, type0, stage);
+    p += n;
+  }
+  return listed;
 }
 
 __global__ void __launch_bounds__(kKeyWarps * 32, 4) key_items_kernel(const __grid_constant__ KeyLaunch L) {
@@ -272,8 +332,24 @@ __global__ void __launch_bounds__(kKeyWarps * 32, 4) key_items_kernel(const __gr
   const ulonglong2 *const snap = C.snap;
   constexpr uint32_t ALL = 0xFFFFFFFFu;
   uint32_t listed = 0;  // targets written by this lane's items
+  if (lane < kKeyRecords / 32) S.late[lane] = 0;
+  // How many of the next records key_records_direct would take at a time: those of the first one's type.
+  auto side_by_side = [&](uint64_t d, uint32_t nrec) -> uint32_t {
+    const uint32_t type = (uint32_t)(d >> 56) & 15u, type0 = __shfl_sync(ALL, type, 0);
+    const uint32_t other = __ballot_sync(ALL, lane >= nrec || type != type0);
+    return min(other ? (uint32_t)__ffs((int)other) - 1u : 32u, 32u / components(type0));
+  };
+  // Leaves n records (32 at most) to key_late_records, from the warp's record r on.
+  auto postpone = [&](uint32_t r, uint32_t n) {
+    const uint64_t bits = (uint64_t)(0xFFFFFFFFu >> (32u - n)) << (r & 31u);
+    if (lane == 0) {
+      S.late[r / 32u] |= (uint32_t)bits;
+      if (bits >> 32) S.late[r / 32u + 1u] |= (uint32_t)(bits >> 32);
+    }
+  };
   // the records from r0 on, as many at a time as fit the warp's arrays
-  for (uint32_t r0 = L.first[w], r1 = r_end ? r_end : C.R; r0 < r1;) {
+  const uint32_t first = L.first[w];
+  for (uint32_t r0 = first, r1 = r_end ? r_end : C.R; r0 < r1;) {
     const uint32_t nrec = min(r1 - r0, 32u);
     uint64_t d = 0;
     uint32_t words = 0, present = 0;
@@ -307,6 +383,15 @@ __global__ void __launch_bounds__(kKeyWarps * 32, 4) key_items_kernel(const __gr
       if (lane >= (uint32_t)o) inc += x;
     }
     uint32_t take = (uint32_t)__popc(__ballot_sync(ALL, lane < nrec && inc <= kKeyEntries));
+    // (twice as many: records of a few words, as the bicycle codes', are better off here)
+    if (take < nrec) {
+      const uint32_t beside = side_by_side(d, nrec);
+      if (2u * take < beside) {
+        postpone(r0 - first, beside);
+        r0 += beside;
+        continue;
+      }
+    }
     uint32_t over = take;  // first record that does not fit the arrays below
     const uint32_t E = take ? __shfl_sync(ALL, inc, take - 1u) : 0u;
     if (lane < take) {
@@ -420,12 +505,13 @@ __global__ void __launch_bounds__(kKeyWarps * 32, 4) key_items_kernel(const __gr
       TG += __shfl_sync(ALL, it, 31);
     }
     over = __reduce_min_sync(ALL, over);
-    if (over == 0) {  // a record that does not fit alone
-      listed += key_record_direct(L, C, r0, reinterpret_cast<uint32_t *>(S.h));
-      ++r0;
-      continue;
-    }
     if (over < take) {  // only the records before it (theirs is all in place)
+      const uint32_t beside = side_by_side(d, nrec);
+      if (2u * over < beside) {
+        postpone(r0 - first, beside);
+        r0 += beside;
+        continue;
+      }
       take = over;
       H = S.vstart[over];
     }
@@ -516,10 +602,11 @@ __global__ void __launch_bounds__(kKeyWarps * 32, 4) key_items_kernel(const __gr
     }
     r0 += take;
   }
+  __syncwarp();
+  if (__any_sync(ALL, lane < kKeyRecords / 32 && S.late[lane])) listed += key_late_records(L, C, L.first[w], S);
   const uint32_t tot = __reduce_add_sync(ALL, listed);
   if (lane == 0 && tot) red_add(L.list_total, tot);
 }
-
 
 // ---- records of mechanisms (global path, gradients; one circuit) --------------
 
