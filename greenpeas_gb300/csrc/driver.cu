@@ -1584,7 +1584,7 @@ struct gpc_driver {
   // How often a run left the fast path (gpc_fallback_counts): [0] batches
   // compiled circuit by circuit, [1] runs through the global sort (a bucket
   // overflowed), [2] reruns with wider target lists (a long symptom), [3]
-  // full 128-bit re-sorts, [4] target-buffer regrowths.
+  // re-sorts on more key bits (64, then 128), [4] target-buffer regrowths.
   std::atomic<uint64_t> fallbacks[5] = {};
 
   // Result sizes of the last run, read once it has finished: device_dem answers every circuit of a
@@ -1652,6 +1652,7 @@ struct gpc_driver {
         continue;
       }
       if (used_global && (err & gpc::DEV_FLAG_MIXED) && sorted.on == SortKey::Auto && sort_auto && sorted.bits < 64) {
+        ++fallbacks[3];
         mixed = true;
         CK(cudaMemsetAsync(dptr<char>(L.err), 0, 4, stream));
         run_global(SortKey::Half);

@@ -293,9 +293,9 @@ gpc_status gpc_walk_form(gpc_driver *driver, int32_t *launches, int32_t *persist
  * counts5[0] batches compiled circuit by circuit instead (a circuit needed
  * one of the fallbacks below), [1] runs merged through the global radix sort
  * (a symptom repeated more often than a bucket's 256 slots), [2] reruns with
- * wider target lists (a symptom longer than the list stride), [3] full
- * 128-bit re-sorts on the global path, [4] reruns of scan + emit after the
- * target buffer grew. */
+ * wider target lists (a symptom longer than the list stride), [3] re-sorts
+ * on more key bits on the global path (64 bits, then all 128), [4] reruns of
+ * scan + emit after the target buffer grew. */
 gpc_status gpc_fallback_counts(gpc_driver *driver, uint64_t *counts5);
 
 /* Device allocations and frees of this driver's own buffers since its
