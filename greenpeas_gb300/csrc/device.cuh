@@ -10,7 +10,7 @@ namespace gpc {
 enum : uint32_t {
   DEV_ERR_TIMEOUT = 1u,    // a bounded wait (mbarrier or look-back) gave up
   DEV_ERR_COLLISION = 2u,  // equal 128-bit keys, different symptoms
-  DEV_FLAG_MIXED = 4u,     // equal sort keys, different 128-bit keys: re-sort on 128 bits
+  DEV_FLAG_MIXED = 4u,     // equal sort keys, different 128-bit keys: re-sort on 64 bits, then on all 128
   DEV_FLAG_TG_OVF = 8u,    // target buffer too small: grow and re-run the merge
   DEV_FLAG_BIG_BUCKET = 16u,  // a bucket exceeds the in-CTA capacity: use the global sort
   DEV_FLAG_LONG = 32u,        // a symptom has more targets than the target-list stride: widen it
@@ -51,9 +51,7 @@ __device__ __forceinline__ void red_add(uint32_t *p, uint32_t v) {
   asm volatile("red.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-constexpr uint32_t kMaxCircuitsStaged = 2048;  // batch tables staged in shared memory up to this size
-
-// Index of the circuit holding item x: the last c with base[c] <= x (base has n+1 entries).
+// Index of the circuit holding item x: the last c with base[c] <= x (base[0 .. n - 1]).
 __device__ __forceinline__ uint32_t find_circuit(const uint32_t *base, uint32_t n, uint32_t x) {
   uint32_t lo = 0, hi = n;
   while (hi - lo > 1) {
@@ -275,9 +273,9 @@ struct ParamLaunch {
 cudaError_t launch_param_rec(const ParamLaunch &L, cudaStream_t s);
 
 // Adjoint of the merge and of the channel splits:
-//  group:  one warp per bucket, a lane per group: dL/dq_m = dL/dp_g *
-//          prod_{j in g, j != m} (1 - 2 q_j) from prefix and suffix products
-//          along the group's run in the saved permutation;
+//  group:  one warp per bucket, a lane per sorted position: dL/dq_m = dL/dp_g *
+//          prod_{j in g, j != m} (1 - 2 q_j) from prefix and suffix product
+//          scans along the group's run in the saved permutation;
 //  source: dL/dnoise[e] = sum over the records of source e of (the sum of the
 //          record's mechanisms' dL/dq) * dq/dp, the split's slope at the
 //          source's rate (stab[src][kind], filled by the host).

@@ -31,8 +31,6 @@
 namespace gpc {
 namespace {
 
-constexpr unsigned long long kSpinLimitNs = 200ull * 1000 * 1000;  // 200 ms
-
 __device__ __forceinline__ unsigned long long globaltimer() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

@@ -500,7 +500,11 @@ __device__ __forceinline__ void sts_words(uint32_t a, const uint64_t (&v)[W]) {
 
 // Walks epochs [e0, e_end) from rows X, Z (W words per slot): FIRST and REST
 // store snapshots of word j, AFF does not, XFER leaves measurement bits out
-// too and stops once its rows vanish.  Published row r (X of slot r, or Z of
+// too.  All but XFER stop once their rows vanish past the word's last
+// measurement; a vote an epoch gives a transfer walk nothing even where every
+// column vanishes (a line of 60 qubits all reset each round: walk stage 24.5 us
+// with and without it) and costs where CTAs fill the GPU (d = 25, 60 rounds: 317
+// -> 330).  Published row r (X of slot r, or Z of
 // slot r - qpad) of buffer b is words [r * W, r * W + W) at pub + b * 2 qpad W
 // words; the first epoch publishes into buffer `seq` & 1.  Returns the epoch
 // the walk stopped at.
