@@ -58,6 +58,11 @@ class Options(ctypes.Structure):
                 ("test_fail_alloc", ctypes.c_int32), ("heap_results", ctypes.c_int32), ("incremental", ctypes.c_int32)]
 
 
+class DeviceDem(ctypes.Structure):
+    _fields_ = [("probs", ctypes.c_void_p), ("offsets", ctypes.c_void_p), ("targets", ctypes.c_void_p),
+                ("num_errors", ctypes.c_uint32), ("targets_end", ctypes.c_uint32)]
+
+
 class LowerStats(ctypes.Structure):
     _fields_ = [("incremental", ctypes.c_uint32), ("segments", ctypes.c_uint32), ("reused", ctypes.c_uint32),
                 ("reserved", ctypes.c_uint32), ("parsed_bytes", ctypes.c_uint64)]
@@ -150,7 +155,7 @@ def lib() -> ctypes.CDLL:
     L.gpc_lowerer_free.argtypes = [vp]
     L.gpc_lowerer_free.restype = None
     L.gpc_tape_last_error.restype = ctypes.c_char_p
-    L.gpc_device_dem.argtypes = [vp, i32, ctypes.POINTER(vp), ctypes.POINTER(vp), ctypes.POINTER(vp), u32p, u32p]
+    L.gpc_device_dem.argtypes = [vp, i32, vp, vp, vp, vp, vp]  # addresses of a DeviceDem's fields
     L.gpc_server_create.argtypes = [ctypes.POINTER(ServerOptions), ctypes.POINTER(vp)]
     L.gpc_server_submit.argtypes = [vp, vp, sz, u64p]
     L.gpc_server_wait.argtypes = [vp, ctypes.c_uint64, ctypes.c_double, ctypes.POINTER(vp),

@@ -279,17 +279,16 @@ class Driver:
         write them): probs[E] float64, offsets[E + 1] int32 positions in
         targets (the run's whole target array, so offsets need not start at
         0)."""
-        L = _native.lib()
-        pp, po, pt = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p()
-        n, end = ctypes.c_uint32(), ctypes.c_uint32()
-        _native.check(L.gpc_device_dem(self._h, int(circuit), ctypes.byref(pp), ctypes.byref(po), ctypes.byref(pt),
-                                       ctypes.byref(n), ctypes.byref(end)))
+        # (a batch calls this for every circuit: one record for the five results and no generator, 9.6 -> 7.7 us)
+        d = _native.DeviceDem()
+        at = ctypes.addressof(d)
+        _native.check(_native.lib().gpc_device_dem(self._h, int(circuit), at, at + 8, at + 16, at + 24, at + 28))
         import torch
-        dev = torch.device("cuda", self.device)
-        n, end = n.value, end.value
+        dev, n = torch.device("cuda", self.device), d.num_errors
         # (a tensor of its own for each array, made in the caller's mode: nothing is shared between calls or circuits)
-        return tuple(torch.as_tensor(_DeviceView(a.value, count, typestr), device=dev)
-                     for a, count, typestr in ((pp, n, "<f8"), (po, n + 1, "<i4"), (pt, end, "<i4")))
+        return (torch.as_tensor(_DeviceView(d.probs, n, "<f8"), device=dev),
+                torch.as_tensor(_DeviceView(d.offsets, n + 1, "<i4"), device=dev),
+                torch.as_tensor(_DeviceView(d.targets, d.targets_end, "<i4"), device=dev))
 
     # device-resident stages
     def prepare(self, circuit=None) -> None:
