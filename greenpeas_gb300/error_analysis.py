@@ -156,7 +156,8 @@ class Driver:
         """``incremental``: in batches, lower each circuit against the previous one of its lowering
         thread (branches of one circuit re-parse only the statements that differ and reschedule only
         the time segments those change; see ``Lowerer``).  The DEMs are the same.  A single circuit
-        is lowered whole on all host threads."""
+        is lowered whole on all host threads.
+        ``key_split`` is accepted (0 or -1) and has no effect."""
         L = _native.lib()
         self._h = ctypes.c_void_p()
         self.correlation_level = CorrelationLevel(correlation_level)
